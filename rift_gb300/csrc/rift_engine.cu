@@ -61,7 +61,7 @@ struct rift_handle {
     int nx = 0, ny = 0, nBX = 0, nBY = 0, gridSize = 0, pitch = 0, rows = 0;
     int numSMs = 0, gridStage = 0, gridSpeed = 0, gridTrack = 0, gridDt = 0, gridMarch = 0;
     int gridUpdate = 0;  // k_update1: resident CTAs over half-strip items
-    int gridMarch1 = 0;  // k_march<1>: its own occupancy (fewer registers than k_march<2>)
+    bool marchPrefetch = false;  // the step's working set is larger than L2
     int nSX = 0, nSY = 0;
     int marchMin = 0;  // active strips from which the march kernels run
     int gridGrow = 0;      // CTAs of the grow kernel of the graph path
@@ -76,7 +76,8 @@ struct rift_handle {
     int* strips = nullptr;
     uint8_t* stripFlag = nullptr;
     int marchRows = STRIP_TY;  // tile rows per march work item (1, 2 or 4)
-    CUtensorMap tmAm{}, tmBm{}, tmEm{};  // 120 x 4-row boxes of the march kernels
+    bool marchAuto = true;     // ... not set by the caller: rows fitted to the grid
+    CUtensorMap tmAm{}, tmBm{}, tmEm{};  // 64 x 2-row boxes of the march
     U1Maps tmU1{};                           // 116 x 7-row boxes of k_update1
     float* tmU1Rain[2] = {nullptr, nullptr};  // rain maps the boxes were encoded for
     cudaStream_t stream = nullptr;
@@ -330,29 +331,21 @@ uint32_t marchFix(const rift_handle* h) {
     return 0u;
 }
 
-template <int STAGE, int STY>
-void launchMarchRows(const rift_handle* h, const CUtensorMap& tmIn, const Params& P, cudaStream_t s,
-                     int grid) {
-    switch (marchFix(h)) {
-        case FIX_RAIN: k_march<STAGE, FIX_RAIN, STY><<<grid, MT, 0, s>>>(tmIn, h->tmEm, P); break;
-        case FIX_INFIL_SRC:
-            k_march<STAGE, FIX_INFIL_SRC, STY><<<grid, MT, 0, s>>>(tmIn, h->tmEm, P);
-            break;
-        case FIX_RAINMAP_DRAIN:
-            k_march<STAGE, FIX_RAINMAP_DRAIN, STY><<<grid, MT, 0, s>>>(tmIn, h->tmEm, P);
-            break;
-        default: k_march<STAGE, 0, STY><<<grid, MT, 0, s>>>(tmIn, h->tmEm, P);
-    }
-}
-
 // The march pass of STAGE with the handle's work-item height.
 template <int STAGE>
 void launchMarch(const rift_handle* h, const CUtensorMap& tmIn, const Params& P, cudaStream_t s,
                  int grid) {
-    switch (h->marchRows) {
-        case 1: launchMarchRows<STAGE, 1>(h, tmIn, P, s, grid); break;
-        case 4: launchMarchRows<STAGE, 4>(h, tmIn, P, s, grid); break;
-        default: launchMarchRows<STAGE, 2>(h, tmIn, P, s, grid);
+    const CUtensorMap& tmE = h->tmEm;
+    const int rows = h->marchAuto ? marchItemRows(h->nx, h->ny, grid * MW) : h->marchRows * TH, pf = h->marchPrefetch ? 1 : 0;
+    if (STAGE == 1) {  // no cell update in stage 1: one instantiation
+        k_march<1><<<grid, MT, 0, s>>>(tmIn, tmE, P, rows, pf);
+        return;
+    }
+    switch (marchFix(h)) {
+        case FIX_RAIN: k_march<2, FIX_RAIN><<<grid, MT, 0, s>>>(tmIn, tmE, P, rows, pf); break;
+        case FIX_INFIL_SRC: k_march<2, FIX_INFIL_SRC><<<grid, MT, 0, s>>>(tmIn, tmE, P, rows, pf); break;
+        case FIX_RAINMAP_DRAIN: k_march<2, FIX_RAINMAP_DRAIN><<<grid, MT, 0, s>>>(tmIn, tmE, P, rows, pf); break;
+        default: k_march<2><<<grid, MT, 0, s>>>(tmIn, tmE, P, rows, pf);
     }
 }
 
@@ -402,7 +395,7 @@ void enqueueStep(rift_handle* h) {
     // per-tile and march variants of each pass; the device keeps one of them
     // (useMarch) and the other returns at once
     k_speed_dt<<<h->gridSpeed, NT, 0, s>>>(h->tmA, h->tmE, P);
-    launchMarch<1>(h, h->tmAm, P, s, h->gridMarch1);  // fluxes, speeds, dt
+    launchMarch<1>(h, h->tmAm, P, s, h->gridMarch);  // fluxes, speeds, dt
     k_stage<1><<<h->gridStage, NT, 0, s>>>(h->tmA, h->tmE, P);
     launchUpdate1(h, P, s);
     if (!h->has(RIFT_F_EULER)) {
@@ -704,9 +697,9 @@ int rift_create(const rift_grid_desc* g, rift_handle** out) {
     CUDA_TRY(h, cudaMalloc(&h->volPartial, 2 * 1024 * sizeof(double)));
     if ((r = encodeMap(h, &h->tmA, h->A, 3)) || (r = encodeMap(h, &h->tmB, h->B, 3)) ||
         (r = encodeMap(h, &h->tmE, h->E, 4)) ||
-        (r = encodeMap(h, &h->tmAm, h->A, 3, MBOXW, MRC)) ||
-        (r = encodeMap(h, &h->tmBm, h->B, 3, MBOXW, MRC)) ||
-        (r = encodeMap(h, &h->tmEm, h->E, 4, MBOXW, MRC)))
+        (r = encodeMap(h, &h->tmAm, h->A, 3, MBOX, MCR)) ||
+        (r = encodeMap(h, &h->tmBm, h->B, 3, MBOX, MCR)) ||
+        (r = encodeMap(h, &h->tmEm, h->E, 4, MBOX, MCR)))
         return r;
     if ((r = encodeMap(h, &h->tmU1.a, h->A, 3, UBOXW, URC)) ||
         (r = encodeMap(h, &h->tmU1.d, h->D, 3, UBOXW, URC)) ||
@@ -732,11 +725,11 @@ int rift_create(const rift_grid_desc* g, rift_handle** out) {
     if (occ < 1) occ = 1;
     h->gridStage = std::max(1, std::min(G, h->numSMs * occ));
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_march<2>, MT, 0);
-    if (occ < 1) occ = 1;
-    h->gridMarch = std::max(1, std::min(NS, h->numSMs * occ));
-    int occ1 = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ1, k_march<1>, MT, 0);
-    h->gridMarch1 = std::max(1, std::min(NS, h->numSMs * std::max(occ1, 1)));
+    occ = std::max(1, std::min(occ, MARCH_CTAS));
+    h->gridMarch = h->numSMs * occ;
+    int l2 = 0;
+    cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
+    h->marchPrefetch = h->plane() * 4 * 20 > (size_t)l2;  // the 20 planes a step moves
     int occU = 1;
     // the gridded-rain instantiation stages two more planes (3 CTAs per SM, 4 without)
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occU, k_update1<FIX_RAINMAP_DRAIN>, MT,
@@ -1627,7 +1620,7 @@ int rift_bench_run(rift_handle* h, int32_t nsteps, double* ms_total, double* act
         k_grow<<<h->gridGrow, NT, 0, s>>>(P);
         k_speed_dt<<<h->gridSpeed, NT, 0, s>>>(h->tmA, h->tmE, P);
         CUDA_TRY(h, cudaEventRecord(e0, s));
-        launchMarch<1>(h, h->tmAm, P, s, h->gridMarch1);
+        launchMarch<1>(h, h->tmAm, P, s, h->gridMarch);
         k_stage<1><<<h->gridStage, NT, 0, s>>>(h->tmA, h->tmE, P);
         launchUpdate1(h, P, s);
         if (!h->has(RIFT_F_EULER)) {
@@ -1657,6 +1650,7 @@ int rift_set_march_rows(rift_handle* h, int32_t tile_rows) {
     if (tile_rows != 1 && tile_rows != 2 && tile_rows != 4)
         return fail(h, RIFT_ERR_ARG, "march work items are 1, 2 or 4 tile rows high");
     h->marchRows = tile_rows;
+    h->marchAuto = false;
     destroyGraph(h);
     return RIFT_OK;
 }
@@ -1724,6 +1718,7 @@ int rift_autotune(rift_handle* h, int32_t probe_steps, int32_t* choice, double* 
         return RIFT_OK;
     };
     const int keepPersist = h->persistMax, keepMarch = h->marchMin, keepRows = h->marchRows;
+    const bool keepAuto = h->marchAuto;
     // candidates: persistent loop; per-step graph with the tile kernels; with
     // the march kernels on work items of 2, 1 and 4 tile rows
     constexpr int NC = RIFT_AUTOTUNE_CANDIDATES;
@@ -1742,6 +1737,7 @@ int rift_autotune(rift_handle* h, int32_t probe_steps, int32_t* choice, double* 
         h->persistMax = persistOf[c];
         h->marchMin = marchOf[c];
         h->marchRows = rowsOf[c];
+        h->marchAuto = c < 2 ? keepAuto : c == 2;  // 2: the default, rows fitted to the grid
         destroyGraph(h);
         *h->hst = saved;
         h->hst->t_stop = INFINITY;
@@ -1771,6 +1767,7 @@ int rift_autotune(rift_handle* h, int32_t probe_steps, int32_t* choice, double* 
     h->persistMax = rc ? keepPersist : (pick == 0 ? INT32_MAX : 0);
     h->marchMin = rc ? keepMarch : marchOf[pick];
     h->marchRows = rc ? keepRows : rowsOf[pick];
+    h->marchAuto = rc || pick < 2 ? keepAuto : pick == 2;
     destroyGraph(h);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);

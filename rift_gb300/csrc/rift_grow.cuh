@@ -127,11 +127,10 @@ __device__ void growAppend(const Params& P, unsigned* staleDst = nullptr) {
         }
         if (t.f[0]) cells += (unsigned long long)t.cells;
         if (t.b >= 0) {
-            if (t.v && t.cells == 0) {
+            if (t.v) {  // the march folds an active tile's speeds into a cleared entry
                 P.mx[t.b] = 0.f;
                 P.my[t.b] = 0.f;
-            }
-            if (!t.v) {  // a tile not active this step: its stale speeds count for dt (A5)
+            } else {  // a tile not active this step: its stale speeds count for dt (A5)
                 smx = fmaxf(smx, t.mxb);
                 smy = fmaxf(smy, t.myb);
             }

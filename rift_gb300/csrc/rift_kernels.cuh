@@ -873,36 +873,45 @@ __global__ void __launch_bounds__(NT) k_speed_dt(const __grid_constant__ CUtenso
 // (ApplyBoundariesX_k: clamped at epsilon; ApplyBoundariesY_k: not).
 // The ghost's reference elevation is that of the interior cell it copies,
 // so its depth is the critical depth itself.
-__device__ __forceinline__ void writeGhosts(const Params& P, float* U, int j, int i, float h,
-                                            float hu, float hv) {
-    auto put = [&](int jj, int ii, float gh) {
-        U[cidx(P, 0, jj, ii)] = gh;
-        U[cidx(P, 1, jj, ii)] = hu;
-        U[cidx(P, 2, jj, ii)] = hv;
-    };
+__device__ __forceinline__ void putGhost(const Params& P, float* U, int j, int i, float h, float hu,
+                                         float hv) {
+    U[cidx(P, 0, j, i)] = h;
+    U[cidx(P, 1, j, i)] = hu;
+    U[cidx(P, 2, j, i)] = hv;
+}
+__device__ __forceinline__ void writeGhostCols(const Params& P, float* U, int j, int i, float h,
+                                               float hu, float hv) {
     if (i == 2 || i == P.nx - 3) {
         float HL = criticalDepth(hu, h);
         HL = (HL > kEps) ? HL : 0.f;
         if (i == 2) {
-            put(j, 0, HL);
-            put(j, 1, HL);
+            putGhost(P, U, j, 0, HL, hu, hv);
+            putGhost(P, U, j, 1, HL, hu, hv);
         }
         if (i == P.nx - 3) {
-            put(j, P.nx - 2, HL);
-            put(j, P.nx - 1, HL);
+            putGhost(P, U, j, P.nx - 2, HL, hu, hv);
+            putGhost(P, U, j, P.nx - 1, HL, hu, hv);
         }
     }
+}
+__device__ __forceinline__ void writeGhostRows(const Params& P, float* U, int j, int i, float h,
+                                               float hu, float hv) {
     if (j == 2 || j == P.ny - 3) {
         float HB = criticalDepth(hv, h);
         if (j == 2) {
-            put(0, i, HB);
-            put(1, i, HB);
+            putGhost(P, U, 0, i, HB, hu, hv);
+            putGhost(P, U, 1, i, HB, hu, hv);
         }
         if (j == P.ny - 3) {
-            put(P.ny - 2, i, HB);
-            put(P.ny - 1, i, HB);
+            putGhost(P, U, P.ny - 2, i, HB, hu, hv);
+            putGhost(P, U, P.ny - 1, i, HB, hu, hv);
         }
     }
+}
+__device__ __forceinline__ void writeGhosts(const Params& P, float* U, int j, int i, float h,
+                                            float hu, float hv) {
+    writeGhostCols(P, U, j, i, h, hu, hv);
+    writeGhostRows(P, U, j, i, h, hu, hv);
 }
 
 // Step-wide constants of a stage kernel.
@@ -1095,13 +1104,14 @@ __device__ __forceinline__ void rk1Core(const Params& P, const StageConsts& C, s
     hN = (hN > kEps) ? hN : 0.f;
 }
 
-// edge: the work item holds a cell next to the ghost band (i or j at 2 or
-// at n - 3); false skips the ghost tests for the items inside.
+// The stage's result at the cell (hN, huN, hvN; the caller stores them) and
+// its wet vote; F and the output maps are written here.
 // L (check_volume runs, else null): the cell's ledger terms are added to it.
 template <int STAGE, bool PREF = false, uint32_t FIX = 0>
-__device__ __forceinline__ bool cellFinish(const Params& P, const StageConsts& C, int j, int i,
+__device__ __forceinline__ bool cellResult(const Params& P, const StageConsts& C, int j, int i,
                                            const CellSrc& src, float hC, float hu0, float hv0,
-                                           const float* pre, bool edge, Led* L = nullptr) {
+                                           const float* pre, Led* L, float& hN, float& huN,
+                                           float& hvN) {
     const uint32_t fl = cellFlags<FIX>(C.fl);
     const bool euler = FIX ? (FIX & F_EULER) != 0 : C.euler;
     const size_t c = cidx(P, 0, j, i);
@@ -1110,7 +1120,6 @@ __device__ __forceinline__ bool cellFinish(const Params& P, const StageConsts& C
     const float rainG = src.rainG;
     const bool srcCell = src.srcCell;
     const float dtNew = C.dtNew;
-    float hN, huN, hvN;
     bool wetCell = false;
     if (STAGE == 1) {
         // Integrate_1_k (grid.cu:856-922)
@@ -1162,6 +1171,19 @@ __device__ __forceinline__ bool cellFinish(const Params& P, const StageConsts& C
         L->v[LED_DRAIN] += C.wRate * src.drained;
         L->v[LED_INFIL] += C.wRate * dF;
     }
+    return wetCell;
+}
+
+// cellResult with its stores.  edge: the work item holds a cell next to the
+// ghost band (i or j at 2 or at n - 3); false skips the ghost tests for the
+// items inside.
+template <int STAGE, bool PREF = false, uint32_t FIX = 0>
+__device__ __forceinline__ bool cellFinish(const Params& P, const StageConsts& C, int j, int i,
+                                           const CellSrc& src, float hC, float hu0, float hv0,
+                                           const float* pre, bool edge, Led* L = nullptr) {
+    float hN, huN, hvN;
+    const bool wetCell =
+        cellResult<STAGE, PREF, FIX>(P, C, j, i, src, hC, hu0, hv0, pre, L, hN, huN, hvN);
     C.Uout[cidx(P, 0, j, i)] = hN;
     C.Uout[cidx(P, 1, j, i)] = huN;
     C.Uout[cidx(P, 2, j, i)] = hvN;

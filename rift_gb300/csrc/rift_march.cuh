@@ -1,389 +1,442 @@
-// rift_march.cuh -- the two fused RK stages as a column march over strips.
+// rift_march.cuh -- the two flux passes of a step as a column march by warps.
 //
-// Work item: a strip of 7 x 2 reference tiles (112 x 28 cells).  A CTA of
-// four warps walks the strip row by row.  Lane l of warp w holds column
-// 28w + l - 2 of the strip; lanes 2..29 own their column, lanes 0, 1, 30, 31
-// supply the x halo (the warps overlap by four columns).  Per output row:
+// Work item: 60 columns x `itemRows` rows of the grid, walked row by row by
+// one warp with no CTA barrier.  Lane l holds the two
+// columns 60 s + 2l and 60 s + 2l + 1 of segment s as a pair, so the
+// arithmetic runs on the packed FP32 instructions (rift_pair.cuh); lanes 1..30
+// own their columns, lanes 0 and 31 supply the x halo (4 of 64 columns).
+// Per row:
 //   - the y reconstruction of the row above and the flux through the row's
-//     north face come from registers rolled down the column (no recompute,
-//     no shared memory);
-//   - the x reconstruction takes its neighbours by warp shuffle, the flux
-//     through the east face takes the east neighbour's west-face values by
-//     shuffle, and the west-face flux is the west neighbour's east-face flux;
-//   - the cell update (sources, friction, RK stage, outputs, ghost cells) is
-//     the same arithmetic as grid.cu's Integrate kernels.
-// Rows arrive in shared memory through TMA: 4-row chunks of the 120-column
-// block of (h, hu, hv) and of the four face-elevation offsets, a 2-slot ring
-// refilled as the march moves up (one barrier per chunk).
+//     north face come from registers rolled down the columns;
+//   - the differences to the east are formed once per face: the west ones are
+//     the neighbour's, one shuffle each, and the west-face flux is the
+//     neighbour's east-face flux (13 shuffles for two cells);
+//   - the cell update is the same arithmetic as grid.cu's Integrate kernels.
+// Rows arrive through TMA in chunks of two rows of 64 columns, a ring of
+// three chunks per warp: two hold the three rows a step of the march reads,
+// the third is in flight during two rows.  The cell's own values (stage 2:
+// U^n, maps, infiltration) are loaded one row ahead; on grids
+// larger than L2 one prefetch instruction per row asks for them MPF rows
+// ahead (lane q takes one 128-byte line).
 // A cell is updated only when its reference tile is active, so results and
 // tile flags are those of the per-tile schedule of the reference.
 //
 // Stage 1 needs dt, and dt needs the speeds of stage 1's own fluxes (the
 // first ComputeFluxes of the step).  So the stage-1 march computes the
-// fluxes, the tile speeds and dt (last CTA), and stores each cell's flux
+// fluxes, the speed maxima and dt (last CTA), and stores each cell's flux
 // divergence with the bed-slope source folded in (3 words); k_update1
-// (rift_update1.cuh) then
-// applies the rest of Integrate_1_k.  The step does one flux pass per stage
-// and no separate speed pass.
+// (rift_update1.cuh) then applies the rest of Integrate_1_k.  The step does
+// one flux pass per stage and no separate speed pass.
+//
+// What bounds it: on 4096^2 cells of urban rain the passes issue 201 and 292
+// lane instructions per cell (397 and 505 with one column per lane, a CTA of
+// four warps in step and scalar arithmetic) and take 153 and 222 us (219 and
+// 294); they issue on 60% of cycles, the packed instructions' FMA pipe is 60%
+// busy, DRAM moves at 4.6 and 5.0 TB/s.  A lone warp needs 0.56 us per row.
 #pragma once
 #include "rift_kernels.cuh"
+#include "rift_pair.cuh"
 
 namespace rift {
 
-constexpr int MW = 4;                              // warps per CTA
-constexpr int MT = MW * 32;                        // threads per CTA
-constexpr int MOWN = 28;                           // owned columns per warp
-constexpr int MCOLS = STRIP_TX * TW;               // 112 columns per strip
-constexpr int MBOXW = 120;                         // staged columns [112 sx - 4, 112 sx + 116)
-constexpr int MRC = 4;                             // rows per staged chunk
-constexpr int MNSLOT = 2;                          // chunk ring depth
-constexpr int MHR = STRIP_TY * TH;                 // 28 output rows per strip
-constexpr int MNROWS = MHR + 4;                    // 32 staged rows (2-row halo each side)
-constexpr int MNCHUNK = (MNROWS + MRC - 1) / MRC;  // 8 chunks
-static_assert(MW * MOWN == MCOLS, "strip width");
-static_assert(MNROWS % MRC == 0, "whole chunks");
+constexpr int MW = 4;                  // warps per CTA
+constexpr int MT = MW * 32;            // threads per CTA
+constexpr int MCOLS = STRIP_TX * TW;   // columns of the grow's strips (112)
+constexpr int MSEG = 60;               // columns a warp owns
+constexpr int MBOX = 64;               // columns a warp stages
+constexpr int MCR = 2;                 // rows per staged chunk
+constexpr int MNS = 3;                 // chunks in a warp's ring
+constexpr int MPF = 5;                 // rows ahead of the L2 prefetch of the centre values
 constexpr unsigned FULL = 0xffffffffu;
 
-struct __align__(128) MarchSlot {
-    float s[3][MRC][MBOXW];  // h, hu, hv     (5760 B)
-    float e[4][MRC][MBOXW];  // eW, eE, eS, eN (7680 B)
-};
-static_assert(sizeof(MarchSlot) % 128 == 0, "TMA destination alignment");
-static_assert(offsetof(MarchSlot, e) % 128 == 0, "TMA destination alignment");
-constexpr uint32_t MBYTES_S = 3 * MRC * MBOXW * 4;
-constexpr uint32_t MBYTES_E = 4 * MRC * MBOXW * 4;
-
-// Work items of the march are 112 columns wide and STY reference tile rows
-// high (STY = 1, 2 or 4: 14, 28 or 56 cells), chosen per handle
-// (rift_set_march_rows, the autotuner).  The grow lists strips of 7 x 2
-// tiles; an item of one tile row is half such a strip, one of four rows a
-// pair of vertically adjacent strips.
-constexpr int STY_MAX = 4;
-
-struct __align__(128) MarchSmem {
-    MarchSlot slot[MNSLOT];
-    uint64_t bar[MNSLOT];
-    unsigned tmx[STRIP_TX * STY_MAX];
-    unsigned tmy[STRIP_TX * STY_MAX];
-    int twet[STRIP_TX * STY_MAX];
-    int tact[STRIP_TX * STY_MAX];
-};
-
-// Does strip (sx, sy) of the grow's 7 x 2 strips hold an active tile?
-__device__ __forceinline__ bool stripHasActive(const Params& P, int sx, int sy) {
-    for (int q = 0; q < STRIP_TX * STRIP_TY; q++) {
-        const int bx = STRIP_TX * sx + q % STRIP_TX, by = STRIP_TY * sy + q / STRIP_TX;
-        if (bx < P.nBX && by < P.nBY && P.prevAct[by * P.nBX + bx] && bx * TW + 2 <= P.nx - 3 &&
-            by * TH + 2 <= P.ny - 3)
-            return true;
-    }
-    return false;
+__device__ __forceinline__ P2 ld2(const float* p) {
+    return P2{*reinterpret_cast<const unsigned long long*>(p)};
+}
+__device__ __forceinline__ void st2(float* p, P2 a) {
+    *reinterpret_cast<unsigned long long*>(p) = a.v;
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
-// Work item `item` of an STY-row march: its strip column and first tile row;
-// false when the item is covered by another one (STY = 4: the upper strip of
-// a pair whose lower strip is listed).  Items: 2 x the listed strips for
-// STY = 1, the listed strips otherwise.
-template <int STY>
-__device__ __forceinline__ bool marchItem(const Params& P, int item, int& sx, int& by0) {
-    if (STY == 1) {
-        const int st = P.strips[item >> 1];
-        sx = st % P.nSX;
-        by0 = STRIP_TY * (st / P.nSX) + (item & 1);
-        return true;
+// A warp's ring of staged rows: chunks of two rows of 64 columns of h, hu, hv
+// (one TMA copy) and of the four face offsets (another).
+struct __align__(128) MarchSlot {
+    float s[3][MCR][MBOX];
+    float e[4][MCR][MBOX];
+};
+static_assert(sizeof(MarchSlot) % 128 == 0 && offsetof(MarchSlot, e) % 128 == 0,
+              "TMA destination alignment");
+struct __align__(128) MarchRing {
+    MarchSlot slot[MNS];
+    uint64_t bar[MNS];
+};
+// Plane p (0..2 h, hu, hv, 3..6 eW, eE, eS, eN) of a staged row at this
+// lane's columns; r points at plane 0 of the row.
+__device__ __forceinline__ P2 row2(const float* r, int p) { return ld2(r + p * MCR * MBOX); }
+
+struct Cell2 {  // state of this lane's two columns in one row
+    P2 h, u, v;
+};
+__device__ __forceinline__ Cell2 loadCell2(const float* r) {
+    return Cell2{row2(r, 0), row2(r, 1), row2(r, 2)};
+}
+
+struct Diff2 {  // differences of surface and momenta across the faces of two columns
+    P2 w, u, v;
+};
+// from row a to the row b above it (their staged rows ra, rb)
+__device__ __forceinline__ Diff2 diffY(const Cell2& a, const float* ra, const Cell2& b, const float* rb) {
+    return Diff2{add2(sub2(row2(ra, 6), row2(rb, 5)), sub2(b.h, a.h)), sub2(b.u, a.u), sub2(b.v, a.v)};
+}
+__device__ __forceinline__ void constructY2(const Cell2& c, const float* r, const Diff2& dP,
+                                            const Diff2& dM, Face2& P, Face2& M) {
+    construct2(c.h, c.u, c.v, limit2(dP.w, dM.w), limit2(dP.u, dM.u), limit2(dP.v, dM.v), row2(r, 5),
+               row2(r, 6), P, M);
+}
+// x reconstruction of a row and the fluxes through the east faces of both
+// columns; fx: the difference of each column's east and west fluxes, fW0, fE0
+// the mass fluxes through both.  The differences mix neighbours of a pair, so
+// they stay scalar (packing them would cost a move each).
+__device__ __forceinline__ void rowFluxX(const Cell2& c, P2 eW, P2 eE, float kappa, P2 fx[3], P2& fW0,
+                                         P2& fE0, P2& spd) {
+    auto down = [](float a) { return __shfl_down_sync(FULL, a, 1); };
+    auto up = [](float a) { return __shfl_up_sync(FULL, a, 1); };
+    // limited differences of both columns from d0 (across the face between
+    // them) and d1 (across the east face of the second)
+    auto limit = [&](float d0, float d1) { return pack2(limit1(d0, up(d1)), limit1(d1, d0)); };
+    const P2 tw = limit((lo(eE) - hi(eW)) + (hi(c.h) - lo(c.h)),
+                        (hi(eE) - down(lo(eW))) + (down(lo(c.h)) - hi(c.h)));
+    const P2 tu = limit(hi(c.u) - lo(c.u), down(lo(c.u)) - hi(c.u));
+    const P2 tv = limit(hi(c.v) - lo(c.v), down(lo(c.v)) - hi(c.v));
+    Face2 Pf, Mf;
+    construct2(c.h, c.u, c.v, tw, tu, tv, eW, eE, Pf, Mf);
+    auto east = [&](P2 a) { return pack2(hi(a), down(lo(a))); };
+    const Face2 R{east(Mf.h), east(Mf.u), east(Mf.v)};
+    P2 f[3];
+    faceFlux2<0>(Pf, R, kappa, f, spd);
+    float w[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        w[q] = up(hi(f[q]));
+        fx[q] = pack2(lo(f[q]) - w[q], hi(f[q]) - lo(f[q]));
     }
-    const int st = P.strips[item];
-    sx = st % P.nSX;
-    const int sy = st / P.nSX;
-    if (STY == 2) {
-        by0 = STRIP_TY * sy;
-        return true;
+    fW0 = pack2(w[0], lo(f[0]));
+    fE0 = f[0];
+}
+
+// Rows per item: every warp gets the same number of items, as few rows as
+// that allows (an item also loads 4 halo rows and reconstructs about 3 rows'
+// worth before its first).  4096^2 cells on 2432 warps: 59 rows in two rounds.
+inline int marchItemRows(int nx, int ny, int warps) {
+    const long long segs = (nx - 4 + MSEG - 1) / MSEG;
+    int best = 2;
+    double cost = 1e300;
+    for (int r = 2; r <= 64; r++) {
+        const long long items = segs * ((ny - 4 + r - 1) / r);
+        const double c = (double)((items + warps - 1) / warps) * (r + 3.0);
+        if (c < cost) {
+            cost = c;
+            best = r;
+        }
     }
-    if (sy & 1) {  // pairs (2p, 2p + 1): the upper one alone only without its partner
-        if (stripHasActive(P, sx, sy - 1)) return false;
-        by0 = STRIP_TY * (sy - 1);
-    } else {
-        by0 = STRIP_TY * sy;
+    return best;
+}
+
+// Segments of 60 columns across the interior.
+__host__ __device__ constexpr int marchSegs(int nx) { return (nx - 4 + MSEG - 1) / MSEG; }
+
+// Rows [j0, j1) of segment seg by one warp.  on(by, bx): is the tile active?
+// (called by all lanes; false for lanes that own no interior column).
+// STAGE 1: reads U^n (A) -> flux divergence + bed source (D), the speed
+//          maxima of active cells (tmx, tmy); Euler mode: tile speeds.  RK2:
+//          clears the tiles' wet flags for stage 2.
+// STAGE 2: reads U* (B) and U^n (A) at the cell -> writes U^{n+1} (A),
+//          F^{n+1} (FA), outputs, tile wet flags and tile speeds (mx, my were
+//          cleared since stage 1's flux pass).
+template <int STAGE, uint32_t FIX, class On>
+__device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C, const CUtensorMap* tmIn,
+                                          const CUtensorMap* tmE, MarchRing& S, uint32_t& par, int seg,
+                                          int j0, int j1, On on, bool led, Led& L, float& tmx,
+                                          float& tmy, bool pf) {
+    constexpr bool RAINPRE = STAGE == 2 && (FIX & F_RAIN_G) != 0;
+    constexpr bool INFPRE = STAGE == 2 && (FIX & F_INFIL) != 0;
+    const int lane = threadIdx.x & 31;
+    const int i = MSEG * seg + 2 * lane;            // this lane's columns i, i + 1
+    const unsigned ic = (unsigned)min(i, P.pitch - 2);
+    const bool own = lane >= 1 && lane <= 30;
+    const bool inX = own && i <= P.nx - 3, inY = own && i + 1 <= P.nx - 3;
+    const int bx = inX ? (i - 2) / TW : -1;         // both columns lie in one tile
+    const unsigned group = __match_any_sync(FULL, bx);
+    const bool leader = inX && lane == __ffs(group) - 1;
+    const bool edge = seg == 0 || MSEG * (seg + 1) + 1 >= P.nx - 3 || j0 == 2 || j1 - 1 >= P.ny - 3;
+    const float kappa = C.kappa;
+    const unsigned pitch = (unsigned)P.pitch;
+    const size_t pl = (size_t)P.planeSize;
+    const uint32_t fl = cellFlags<FIX>(C.fl);
+    const bool euler = FIX ? (FIX & F_EULER) != 0 : C.euler;
+    const P2 nidx = both(-P.inv_dx), nidy = both(-P.inv_dy), idx = both(P.inv_dx), idy = both(P.inv_dy);
+
+    // the line of plane lane / 4 this lane prefetches (3 lines hold the 64 columns)
+    const float* pfB = nullptr;
+    if (STAGE == 2 && pf && (lane & 3) < 3) {
+        const int p = lane >> 2;
+        const unsigned pc = (unsigned)min(MSEG * seg + 32 * (lane & 3), P.pitch - 1);
+        if (p < 3) pfB = P.A + p * pl + pc;
+        if (RAINPRE && p >= 3 && p < 5 && P.mapMode[0] >= p - 2)
+            pfB = (p == 3 ? P.map0[0] : P.map1[0]) + pc;
+    }
+    // staged row r is grid row j0 - 2 + r; chunk c holds rows 2c and 2c + 1
+    const int nch = (j1 - j0 + 4 + MCR - 1) / MCR;
+    auto issue = [&](int c, int sl) {
+        fence_proxy_async();
+        mbar_expect_tx(&S.bar[sl], (uint32_t)sizeof(MarchSlot));
+        tma_load_3d(&S.slot[sl].s[0][0][0], tmIn, &S.bar[sl], MSEG * seg, j0 - 2 + MCR * c, 0);
+        tma_load_3d(&S.slot[sl].e[0][0][0], tmE, &S.bar[sl], MSEG * seg, j0 - 2 + MCR * c, 0);
+    };
+    // wait for the chunk in slot sl; false after the spin limit, once the
+    // copies in flight have landed or given up too
+    auto acquire = [&](int sl) {
+        const bool ok = __all_sync(FULL, mbar_wait_bounded(&S.bar[sl], (par >> sl) & 1u));
+        if (!ok)
+            for (int q = 0; q < MNS; q++) mbar_wait_bounded(&S.bar[q], (par >> q) & 1u);
+        par ^= 1u << sl;
+        return ok;
+    };
+    __syncwarp();  // the previous item no longer reads the ring
+    if (lane == 0)
+        for (int c = 0; c < MNS && c < nch; c++) issue(c, c);
+    if (!acquire(0) || !acquire(1)) return false;
+    // rows j, j + 1, j + 2 of the current output row
+    const float* rc = &S.slot[1].s[0][0][2 * lane];
+    const float* rn = rc + MBOX;
+    const float* rl = &S.slot[2].s[0][0][2 * lane];
+    Cell2 cur = loadCell2(rc), nxt = loadCell2(rn);
+    Face2 yP;      // the row's reconstruction at its north face
+    P2 fS[3];      // flux through its south face
+    Diff2 dN;      // differences to the row above
+    {
+        const float* r0 = &S.slot[0].s[0][0][2 * lane];
+        const float* r1 = r0 + MBOX;
+        const Cell2 m2 = loadCell2(r0), m1 = loadCell2(r1);
+        const Diff2 d0 = diffY(m2, r0, m1, r1), d1 = diffY(m1, r1, cur, rc);
+        dN = diffY(cur, rc, nxt, rn);
+        Face2 a, b, M;
+        constructY2(m1, r1, d1, d0, a, b);
+        constructY2(cur, rc, dN, d1, yP, M);
+        P2 s;
+        faceFlux2<1>(a, M, kappa, fS, s);
+    }
+    // the row's centre values (stage 2: U^n; rain maps or F, K, F^n when the
+    // instantiation reads them ahead), one row ahead of their use
+    P2 pre[6], nextPre[6];
+    auto loadCentre = [&](P2 (&d)[6], int jj) {
+        const unsigned c = (unsigned)jj * pitch + ic;
+        d[0] = ld2(P.A + c);
+        d[1] = ld2(P.A + pl + c);
+        d[2] = ld2(P.A + 2 * pl + c);
+        if (RAINPRE) {
+            d[3] = P.mapMode[0] != 0 ? ld2(P.map0[0] + c) : both(0.f);
+            d[4] = P.mapMode[0] == 2 ? ld2(P.map1[0] + c) : both(0.f);
+        } else if (INFPRE) {
+            d[3] = ld2(C.Fin + c);
+            d[4] = ld2(P.K + c);
+            d[5] = ld2(P.FA + c);
+        }
+    };
+#pragma unroll
+    for (int q = 0; q < 6; q++) pre[q] = nextPre[q] = both(0.f);
+    if (STAGE == 2) loadCentre(pre, j0);
+
+    int sl = 1;  // slot of the chunk that holds row j + 1
+    int by = (j0 - 2) / TH, rt = (j0 - 2) % TH;  // tile row, row in it
+    bool act = on(by, bx);
+    float ax = 0.f, ay = 0.f;
+    bool wet = false;
+    if (STAGE == 1 && !euler && leader && act) P.wet[by * P.nBX + bx] = 0;
+    constexpr int UNROLL = STAGE == 1 ? 2 : 1;
+#pragma unroll UNROLL
+    for (int j = j0; j < j1; j++) {
+        if (((j - j0) & 1) == 0) {
+            // row j + 2 opens chunk k + 1 (k holds row j); rows below j are
+            // done: their slot takes chunk k - 1 + MNS
+            const int k = (j - j0) / 2 + 1;
+            __syncwarp();
+            sl = sl == MNS - 1 ? 0 : sl + 1;  // slot of chunk k + 1
+            if (lane == 0 && k - 1 + MNS < nch) issue(k - 1 + MNS, sl < 2 ? sl + MNS - 2 : sl - 2);
+            if (!acquire(sl)) return false;
+            rl = &S.slot[sl].s[0][0][2 * lane];
+        }
+        if (STAGE == 2) loadCentre(nextPre, j + 1);
+        if (STAGE == 2 && pfB) prefetch_l2(pfB + (size_t)((unsigned)min(j + MPF, P.rows - 1) * pitch));
+        const P2 eW = row2(rc, 3), eE = row2(rc, 4);
+        P2 fN[3], sy, fx[3], fW0, fE0, sx;
+        rowFluxX(cur, eW, eE, kappa, fx, fW0, fE0, sx);
+        // y: reconstruction of row j + 1, flux through the north face of row j
+        const Cell2 ld = loadCell2(rl);
+        const Diff2 dNN = diffY(nxt, rn, ld, rl);
+        Face2 yn, yM;
+        constructY2(nxt, rn, dNN, dN, yn, yM);
+        faceFlux2<1>(yP, yM, kappa, fN, sy);
+        // divergence, with the bed-slope source in the momenta
+        P2 d[3];
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+            d[q] = fma2(fx[q], nidx, mul2(sub2(fN[q], fS[q]), nidy));
+        const P2 gh = mul2(both(-kG), cur.h);
+        d[1] = fma2(gh, mul2(sub2(eE, eW), idx), d[1]);
+        d[2] = fma2(gh, mul2(sub2(row2(rc, 6), row2(rc, 5)), idy), d[2]);
+        if (act) {
+            ax = max3(ax, lo(sx), inY ? hi(sx) : 0.f);
+            ay = max3(ay, lo(sy), inY ? hi(sy) : 0.f);
+            const unsigned c = (unsigned)j * pitch + (unsigned)i;
+            if (led && edge) {
+                float r = edgeInflow(P, j, i, lo(fW0), lo(fE0), lo(fS[0]), lo(fN[0]));
+                if (inY) r += edgeInflow(P, j, i + 1, hi(fW0), hi(fE0), hi(fS[0]), hi(fN[0]));
+                L.v[LED_BOUND] += STAGE == 1 ? r : C.wRate * r;
+            }
+            if (STAGE == 1) {
+                st2(P.D + c, d[0]);
+                st2(P.D + pl + c, d[1]);
+                st2(P.D + 2 * pl + c, d[2]);
+            } else {
+                const int tile = by * P.nBX + bx;
+                float r[2][3];
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    if (k == 1 && !inY) break;
+                    auto at = [&](P2 a) { return k == 0 ? lo(a) : hi(a); };
+                    const float hC = at(cur.h), u0 = at(cur.u), v0 = at(cur.v);
+                    const float pk[8] = {at(pre[0]), at(pre[1]), at(pre[2]), at(pre[3]),
+                                         at(pre[4]), at(pre[5]), at(pre[3]), at(pre[4])};
+                    const CellSrc s = cellSources<2, INFPRE, false, FIX, RAINPRE>(
+                        P, C, tile, j, i + k, at(d[0]), at(d[1]), at(d[2]), hC, u0, v0, 0.f, 0.f,
+                        0.f, 0.f, pk);
+                    wet |= cellResult<2, INFPRE, FIX>(P, C, j, i + k, s, hC, u0, v0, pk,
+                                                      led ? &L : nullptr, r[k][0], r[k][1], r[k][2]);
+                }
+#pragma unroll
+                for (int q = 0; q < 3; q++) {
+                    if (inY)
+                        st2(P.A + q * pl + c, pack2(r[0][q], r[1][q]));
+                    else
+                        P.A[q * pl + c] = r[0][q];
+                }
+                if (j == 2 || j == P.ny - 3) {
+                    writeGhostRows(P, P.A, j, i, r[0][0], r[0][1], r[0][2]);
+                    if (inY) writeGhostRows(P, P.A, j, i + 1, r[1][0], r[1][1], r[1][2]);
+                }
+            }
+        }
+        if (++rt == TH || j + 1 == j1) {  // the item's last row of a tile row (warp-uniform)
+            if (STAGE == 1) {
+                tmx = fmaxf(tmx, ax);
+                tmy = fmaxf(tmy, ay);
+            }
+            if (STAGE == 2 || euler) {  // speeds are non-negative: their bits order like the values
+                const unsigned mx = __reduce_max_sync(group, __float_as_uint(ax));
+                const unsigned my = __reduce_max_sync(group, __float_as_uint(ay));
+                const unsigned any = __reduce_or_sync(group, wet ? 1u : 0u);
+                if (leader && act) {
+                    const int tile = by * P.nBX + bx;
+                    atomicMax(reinterpret_cast<unsigned*>(P.mx) + tile, mx);
+                    atomicMax(reinterpret_cast<unsigned*>(P.my) + tile, my);
+                    if (STAGE == 2 && (any || !(fl & F_TILE_ACC))) P.wet[tile] = 1;
+                }
+            }
+            rt = 0;
+            ax = ay = 0.f;
+            wet = false;
+            if (j + 1 < j1) {
+                by++;
+                act = on(by, bx);
+                if (STAGE == 1 && !euler && leader && act) P.wet[by * P.nBX + bx] = 0;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 3; q++) fS[q] = fN[q];
+#pragma unroll
+        for (int q = 0; q < 6; q++) pre[q] = nextPre[q];
+        yP = yn;
+        dN = dNN;
+        cur = nxt;
+        nxt = ld;
+        rc = rn;
+        rn = rl;
+        rl += MBOX;
+    }
+    if (STAGE == 2) {
+        // ghost columns, a row per lane (the cube root is long: once per 32
+        // rows instead of once per row)
+        __syncwarp();
+        for (int side = 0; side < 2; side++) {
+            const int gi = side ? P.nx - 3 : 2;
+            if (gi < MSEG * seg + 2 || gi >= MSEG * (seg + 1) + 2) continue;
+            for (int j = j0 + lane; j < j1; j += 32) {
+                if (!on((j - 2) / TH, (gi - 2) / TW)) continue;
+                const unsigned c = (unsigned)j * pitch + (unsigned)gi;
+                writeGhostCols(P, P.A, j, gi, P.A[c], P.A[pl + c], P.A[2 * pl + c]);
+            }
+        }
     }
     return true;
 }
 
-template <int STY>
-__host__ __device__ constexpr int marchItems(int nStrips) {
-    return STY == 1 ? 2 * nStrips : nStrips;
+// Maximum of a warp's speeds in every lane.
+__device__ __forceinline__ float warpMax(float v) {
+    return __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(v)));
 }
 
-struct Row {  // one staged row at this lane's column
-    float h, u, v, eW, eE, eS, eN;
-};
+// Resident CTAs per SM the march is compiled for: 128 registers a thread.
+// (4096^2 urban rain, stage 1 / stage 2: 153 / 222 us at 4, 177 / 233 us at 3
+// with 168 registers; at 5 the 96 registers spill and both run slower than the
+// kernel of one column per lane this one replaced.)  Two rows per loop
+// iteration in stage 1 (167 us with one), one in stage 2 (243 us with two).
+constexpr int MARCH_CTAS = 4;
 
-__device__ __forceinline__ Row loadRow(const MarchSlot& S, int r, int col) {
-    Row x;
-    x.h = S.s[0][r][col];
-    x.u = S.s[1][r][col];
-    x.v = S.s[2][r][col];
-    x.eW = S.e[0][r][col];
-    x.eE = S.e[1][r][col];
-    x.eS = S.e[2][r][col];
-    x.eN = S.e[3][r][col];
-    return x;
-}
-
-// y reconstruction of row c between rows m (below) and p (above)
-__device__ __forceinline__ Rec constructY(const Row& m, const Row& c, const Row& p) {
-    return construct(c.h, c.u, c.v, p.h, p.u, p.v, m.h, m.u, m.v, c.eS, c.eN, c.eN - p.eS,
-                     m.eN - c.eS);
-}
-
-__device__ __forceinline__ void issueChunk(MarchSmem& S, int slot, const CUtensorMap* tmIn,
-                                           const CUtensorMap* tmE, int xs, int ys) {
-    fence_proxy_async();
-    mbar_expect_tx(&S.bar[slot], MBYTES_S + MBYTES_E);
-    tma_load_3d(&S.slot[slot].s[0][0][0], tmIn, &S.bar[slot], xs, ys, 0);
-    tma_load_3d(&S.slot[slot].e[0][0][0], tmE, &S.bar[slot], xs, ys, 0);
-}
-
-// Error path of a timed-out ring wait on chunk c: wait, bounded, for the
-// chunks still in flight (c .. c+MNSLOT-1), so that no TMA write lands after
-// the CTA has left.  `par` holds the slots' parities before chunk c's wait.
-__device__ __forceinline__ void marchDrain(MarchSmem& S, uint32_t par, int c, int nchunk = MNCHUNK) {
-    for (int k = c; k < c + MNSLOT && k < nchunk; k++)
-        mbar_wait_bounded(&S.bar[k % MNSLOT], (par >> (k % MNSLOT)) & 1u);
-}
-
-// STAGE 1: reads U^n (A) -> flux divergence + bed source (D), tile speed
-//          maxima, dt and t (ComputeFluxes' speed output and
-//          ComputeTimestep), re-sync of U* on tiles that went inactive.
-// STAGE 2: reads U* (B) and U^n (A) at the cell -> writes U^{n+1} (A),
-//          F^{n+1} (FA), outputs, tile wet flags and tile speeds.
-// Resident CTAs per SM the march kernels are compiled for: the stage-1 flux
-// pass fits 8 (64 registers, 27 KB shared memory; measured 1% faster on the
-// 8192^2 step than 6), stage 2 needs its 80 registers at 6.
-#ifndef RIFT_MARCH1_MINB
-#define RIFT_MARCH1_MINB 8
-#endif
-#ifndef RIFT_MARCH2_MINB
-#define RIFT_MARCH2_MINB 6
-#endif
-
-template <int STAGE, uint32_t FIX = 0, int STY = STRIP_TY>
-__global__ void __launch_bounds__(MT, STAGE == 1 ? RIFT_MARCH1_MINB : RIFT_MARCH2_MINB)
-    k_march(const __grid_constant__ CUtensorMap tmIn,
-                                              const __grid_constant__ CUtensorMap tmE, Params P) {
-    __shared__ MarchSmem S;
+template <int STAGE, uint32_t FIX = 0>
+__global__ void __launch_bounds__(MT, MARCH_CTAS) k_march(const __grid_constant__ CUtensorMap tmIn,
+                                                                  const __grid_constant__ CUtensorMap tmE,
+                                                                  Params P, int itemRows, int pf) {
+    __shared__ MarchRing rings[MW];
     __shared__ bool last;
+    __shared__ float wmax[2][MW];
     if (P.st->stop || !useMarch(P)) return;
-    // rain maps read ahead with U^n when the instantiation has gridded rain
-    constexpr bool RAINPRE = STAGE == 2 && (FIX & F_RAIN_G) != 0;
-    constexpr int HR = STY * TH;                      // output rows per item
-    constexpr int NCHUNK = (HR + 4 + MRC - 1) / MRC;  // staged chunks (2-row halo each side)
-    constexpr int NT_ = STRIP_TX * STY;                // tiles per item
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nItems = marchItems<STY>(P.st->nStrips);
-    const StageConsts C = blockConsts<STAGE>(P);
-    float tmxAll = 0.f, tmyAll = 0.f;
+    __shared__ __align__(8) unsigned char cbuf[sizeof(StageConsts)];
+    StageConsts& C = *reinterpret_cast<StageConsts*>(cbuf);
+    MarchRing& S = rings[warp];
     if (tid == 0) {
+        C = stageConsts<STAGE>(P);
         prefetch_tmap(&tmIn);
         prefetch_tmap(&tmE);
-        for (int k = 0; k < MNSLOT; k++) mbar_init(&S.bar[k], 1);
+    }
+    if (lane == 0) {
+        for (int k = 0; k < MNS; k++) mbar_init(&S.bar[k], 1);
         fence_mbar_init();
     }
     __syncthreads();
-    uint32_t par = 0u;                          // wait parity, one bit per ring slot
-    const int lc = MOWN * warp + lane - 2;      // column relative to the strip's first interior column
-    const int col = lc + 6;                     // staged column
-    const bool owned = lane >= 2 && lane <= 29;
-    const int tcol = owned ? lc / TW : 0;       // tile column inside the strip
-    const float kappa = C.kappa;
-    // check_volume ledger: stage 1 sums the edge inflow rates (dt is not
-    // known yet), stage 2 the weighted terms of its cells
+    uint32_t par = 0u;
     const bool led = (cellFlags<FIX>(C.fl) & F_CHECKVOL) != 0;
     Led L;
     ledZero(L);
-
-    for (int item = blockIdx.x; item < nItems; item += gridDim.x) {
-        int sx, by0;
-        if (!marchItem<STY>(P, item, sx, by0)) continue;  // item-uniform
-        const int X0 = MCOLS * sx + 2, Y0 = TH * by0 + 2;
-        // item-uniform: does the item reach the first or last interior row/column?
-        const bool edgeStrip =
-            X0 == 2 || Y0 == 2 || X0 + MCOLS - 1 >= P.nx - 3 || Y0 + HR - 1 >= P.ny - 3;
-        const int xs = MCOLS * sx - 4, ys = Y0 - 2;
-        const int i = X0 + lc;
-        __syncthreads();  // the previous item no longer reads the ring or the tile tables
-        if (tid < NT_) {
-            const int bx = STRIP_TX * sx + tid % STRIP_TX, by = by0 + tid / STRIP_TX;
-            int a = 0;
-            if (bx < P.nBX && by < P.nBY)
-                a = P.prevAct[by * P.nBX + bx] && (bx * TW + 2 <= P.nx - 3) &&
-                    (by * TH + 2 <= P.ny - 3);
-            S.tact[tid] = a;
-            S.tmx[tid] = 0u;
-            S.tmy[tid] = 0u;
-            S.twet[tid] = 0;
-        }
-        if (tid == 0)
-            for (int c = 0; c < MNSLOT; c++) issueChunk(S, c, &tmIn, &tmE, xs, ys + c * MRC);
-        bool ok = mbar_wait_bounded(&S.bar[0], par & 1u);
-        if (!__syncthreads_and(ok)) {
-            marchDrain(S, par, 0, NCHUNK);
-            if (tid == 0) atomicOr(&P.st->error, ERR_TMA_TIMEOUT);
-            return;
-        }
-        par ^= 1u;
-        // prologue: staged rows 0..3; y reconstruction of rows 1 and 2 and the
-        // flux through the south face of row 2 (the first output row)
-        const Row r0 = loadRow(S.slot[0], 0, col);
-        const Row r1 = loadRow(S.slot[0], 1, col);
-        Row cur = loadRow(S.slot[0], 2, col);
-        Row nxt = loadRow(S.slot[0], 3, col);
-        float fS0, fS1, fS2, yPh, yPu, yPv;
-        {
-            const Rec y1 = constructY(r0, r1, cur);
-            const Rec y2 = constructY(r1, cur, nxt);
-            float f[3];
-            faceFlux<1>(y1.hP, y1.uP, y1.vP, y2.hM, y2.uM, y2.vM, kappa, f);
-            fS0 = f[0];
-            fS1 = f[1];
-            fS2 = f[2];
-            yPh = y2.hP;
-            yPu = y2.uP;
-            yPv = y2.vP;
-        }
-        // centre values of the first output row (stage 2: U^n, and the rain
-        // maps when the instantiation reads them ahead), loaded ahead of use
-        const bool colIn = owned && i <= P.nx - 3;
-        // row jj's centre values into d (U^n; the rain maps, or an L1 hint)
-        auto loadCentre = [&](float (&d)[8], int jj) {
-            const size_t cn = cidx(P, 0, jj, i);
-            d[0] = P.A[cn];
-            d[1] = P.A[cn + P.planeSize];
-            d[2] = P.A[cn + 2 * (size_t)P.planeSize];
-            if (RAINPRE)
-                loadRainMaps(P, cn, d + 6);
-            else
-                prefetchMaps(P, cellFlags<FIX>(C.fl), cn);
-        };
-        float pre[8], nextPre[8];
-#pragma unroll
-        for (int q = 0; q < 8; q++) pre[q] = nextPre[q] = 0.f;
-        if (STAGE == 2 && colIn && Y0 <= P.ny - 3) loadCentre(pre, Y0);
-        float accMx = 0.f, accMy = 0.f;
-        bool accWet = false;
-        // two rows per iteration: the compiler interleaves their independent
-        // work (7% faster than one row at the same 80 registers)
-#pragma unroll 2
-        for (int R = 2; R <= HR + 1; R++) {
-            const int lead = R + 2;
-            if (lead % MRC == 0) {  // entering chunk c: refill the slot chunk c-1 used
-                const int c = lead / MRC;
-                __syncthreads();
-                if (tid == 0 && c - 1 + MNSLOT < NCHUNK)
-                    issueChunk(S, (c - 1) % MNSLOT, &tmIn, &tmE, xs, ys + (c - 1 + MNSLOT) * MRC);
-                const int sl = c % MNSLOT;
-                bool ok2 = mbar_wait_bounded(&S.bar[sl], (par >> sl) & 1u);
-                if (!__syncthreads_and(ok2)) {
-                    marchDrain(S, par, c, NCHUNK);
-                    if (tid == 0) atomicOr(&P.st->error, ERR_TMA_TIMEOUT);
-                    return;
-                }
-                par ^= (1u << sl);
-            }
-            const Row ld = loadRow(S.slot[(lead / MRC) % MNSLOT], lead % MRC, col);
-            const int j = Y0 + R - 2;
-            // centre values of the next output row, in flight during this one
-            if (STAGE == 2 && colIn && j + 1 <= P.ny - 3) loadCentre(nextPre, j + 1);
-            const int tslot = ((R - 2) / TH) * STRIP_TX + tcol;
-            const bool cellOn = colIn && S.tact[tslot] && j <= P.ny - 3;
-            float spx, spy;
-            {
-                // y: reconstruction of row R+1, flux through the north face of row R
-                const Rec yn = constructY(cur, nxt, ld);
-                float fN[3];
-                spy = faceFlux<1>(yPh, yPu, yPv, yn.hM, yn.uM, yn.vM, kappa, fN);
-                // x: reconstruction of row R, neighbours by shuffle
-                const float hm = __shfl_up_sync(FULL, cur.h, 1), hp = __shfl_down_sync(FULL, cur.h, 1);
-                const float um = __shfl_up_sync(FULL, cur.u, 1), up = __shfl_down_sync(FULL, cur.u, 1);
-                const float vm = __shfl_up_sync(FULL, cur.v, 1), vp = __shfl_down_sync(FULL, cur.v, 1);
-                const float eEm = __shfl_up_sync(FULL, cur.eE, 1);
-                const float eWp = __shfl_down_sync(FULL, cur.eW, 1);
-                const Rec xr = construct(cur.h, cur.u, cur.v, hp, up, vp, hm, um, vm, cur.eW,
-                                         cur.eE, cur.eE - eWp, eEm - cur.eW);
-                const float rh = __shfl_down_sync(FULL, xr.hM, 1);
-                const float ru = __shfl_down_sync(FULL, xr.uM, 1);
-                const float rv = __shfl_down_sync(FULL, xr.vM, 1);
-                float fE[3];
-                spx = faceFlux<0>(xr.hP, xr.uP, xr.vP, rh, ru, rv, kappa, fE);
-                const float fW0 = __shfl_up_sync(FULL, fE[0], 1);
-                const float fW1 = __shfl_up_sync(FULL, fE[1], 1);
-                const float fW2 = __shfl_up_sync(FULL, fE[2], 1);
-                if (cellOn) {
-                    if (led && edgeStrip) {
-                        const float r = edgeInflow(P, j, i, fW0, fE[0], fS0, fN[0]);
-                        L.v[LED_BOUND] += STAGE == 1 ? r : C.wRate * r;
-                    }
-                    const float dh = -(fE[0] - fW0) * P.inv_dx - (fN[0] - fS0) * P.inv_dy;
-                    const float dhu = -(fE[1] - fW1) * P.inv_dx - (fN[1] - fS1) * P.inv_dy;
-                    const float dhv = -(fE[2] - fW2) * P.inv_dx - (fN[2] - fS2) * P.inv_dy;
-                    if (STAGE == 1) {
-                        // divergence + bed-slope source (dt-free) for k_update1
-                        const size_t c = cidx(P, 0, j, i);
-                        P.D[c] = dh;
-                        P.D[c + P.planeSize] = dhu + bedSourceX(P, cur.h, cur.eW, cur.eE);
-                        P.D[c + 2 * (size_t)P.planeSize] = dhv + bedSourceY(P, cur.h, cur.eS, cur.eN);
-                    } else {
-                        const int tile = (by0 + (R - 2) / TH) * P.nBX + STRIP_TX * sx + tcol;
-                        accWet |= cellUpdate<STAGE, false, true, FIX, RAINPRE>(P, C, tile, j, i, dh, dhu, dhv, cur.h, cur.u,
-                                                    cur.v, cur.eW, cur.eE, cur.eS, cur.eN, pre,
-                                                    edgeStrip, led ? &L : nullptr);
-                    }
-                }
-                fS0 = fN[0];
-                fS1 = fN[1];
-                fS2 = fN[2];
-                yPh = yn.hP;
-                yPu = yn.uP;
-                yPv = yn.vP;
-            }
-            if (cellOn) {
-                accMx = fmaxf(accMx, spx);
-                accMy = fmaxf(accMy, spy);
-            }
-            if ((R - 2) % TH == TH - 1) {  // last row of a tile row: fold into the tile
-                if (owned) {
-                    atomicMax(&S.tmx[tslot], __float_as_uint(accMx));
-                    atomicMax(&S.tmy[tslot], __float_as_uint(accMy));
-                    if (STAGE == 2 && accWet) atomicOr(&S.twet[tslot], 1);
-                }
-                accMx = 0.f;
-                accMy = 0.f;
-                accWet = false;
-            }
-            pre[0] = nextPre[0];
-            pre[1] = nextPre[1];
-            pre[2] = nextPre[2];
-            pre[6] = nextPre[6];
-            pre[7] = nextPre[7];
-
-            cur = nxt;
-            nxt = ld;
-        }
-        __syncthreads();
-        if (tid < NT_ && S.tact[tid]) {
-            const int bx = STRIP_TX * sx + tid % STRIP_TX, by = by0 + tid / STRIP_TX;
-            const int b = by * P.nBX + bx;
-            if (STAGE == 2) P.wet[b] = (uint8_t)((!(C.fl & F_TILE_ACC)) || S.twet[tid]);
-            P.mx[b] = __uint_as_float(S.tmx[tid]);
-            P.my[b] = __uint_as_float(S.tmy[tid]);
-        }
-        if (STAGE == 1) {  // thread 0 keeps this CTA's maximum of new tile speeds
-            __syncthreads();
-            if (tid == 0)
-                for (int k = 0; k < NT_; k++)
-                    if (S.tact[k]) {
-                        tmxAll = fmaxf(tmxAll, __uint_as_float(S.tmx[k]));
-                        tmyAll = fmaxf(tmyAll, __uint_as_float(S.tmy[k]));
-                    }
+    float tmx = 0.f, tmy = 0.f;
+    const int nSeg = marchSegs(P.nx), nGroup = (P.ny - 4 + itemRows - 1) / itemRows;
+    auto on = [&](int by, int bx) { return bx >= 0 && P.prevAct[by * P.nBX + bx] != 0; };
+    for (int item = blockIdx.x * MW + warp; item < nSeg * nGroup; item += gridDim.x * MW) {
+        const int seg = item % nSeg, j0 = 2 + itemRows * (item / nSeg);
+        const int j1 = min(j0 + itemRows, P.ny - 2);
+        // does the item hold an active tile? (lane q tests tile row q of its rows)
+        const int bx0 = MSEG * seg / TW, bx1 = min(MSEG * seg + MSEG - 1, P.nx - 5) / TW;
+        const int by0 = (j0 - 2) / TH, by1 = (j1 - 3) / TH;
+        const int nb = bx1 - bx0 + 1;
+        bool any = false;
+        for (int q = lane; q < nb * (by1 - by0 + 1); q += 32)
+            any |= on(by0 + q / nb, bx0 + q % nb);
+        if (!__any_sync(FULL, any)) continue;
+        if (!marchRows<STAGE, FIX>(P, C, &tmIn, &tmE, S, par, seg, j0, j1, on, led, L, tmx, tmy, pf != 0)) {
+            if (lane == 0) atomicOr(&P.st->error, ERR_TMA_TIMEOUT);
+            break;
         }
     }
     if (led) {
@@ -397,8 +450,19 @@ __global__ void __launch_bounds__(MT, STAGE == 1 ? RIFT_MARCH1_MINB : RIFT_MARCH
         }
     }
     if (STAGE == 1) {
+        tmx = warpMax(tmx);
+        tmy = warpMax(tmy);
+        if (lane == 0) {
+            wmax[0][warp] = tmx;
+            wmax[1][warp] = tmy;
+        }
         __syncthreads();
-        finishDt(P, tmxAll, tmyAll, &last);
+        if (tid == 0)
+            for (int w = 0; w < MW; w++) {
+                tmx = fmaxf(tmx, wmax[0][w]);
+                tmy = fmaxf(tmy, wmax[1][w]);
+            }
+        finishDt(P, tmx, tmy, &last);
         resyncDeactivated(P);
     }
 }
