@@ -238,17 +238,18 @@ int rift_set_schedule(rift_handle* h, int32_t march_min_strips);
 /* Persistent step loop (no reference counterpart): while at most
  * max_active_tiles tiles are active, rift_run / rift_step run their steps
  * in one cooperative launch whose phases are separated by grid barriers,
- * with the per-tile arithmetic of the per-step kernels.  -1 restores the
- * default (the march threshold in tiles), 0 turns it off.
+ * with the arithmetic of the per-step kernels (one tile per CTA, or the
+ * march's items once the tiles outnumber the CTAs).  -1 restores the default
+ * (10240, with infiltration 40960), 0 turns it off.
  * RIFT_ERR_UNSUPPORTED when the device has no cooperative launch. */
 int rift_set_persistent(rift_handle* h, int32_t max_active_tiles);
 
-/* Height of the column march's work items (no reference counterpart): 1, 2
- * (default) or 4 reference tile rows, i.e. CTA items of 112 x 14, 112 x 28
- * or 112 x 56 cells.  Each item stages its rows with a 2-row halo, so taller
- * items stage fewer rows twice and shorter ones balance a ragged active set
- * better.  The activity tiles stay 16 x 14: every height gives the same
- * results. */
+/* Height of the column march's work items (no reference counterpart): 60
+ * columns x 1, 2 or 4 reference tile rows.  Until it is set the height is
+ * fitted to the grid (and rift_get_march_rows gives 2).  Each item loads a
+ * 2-row halo, so taller items load fewer rows twice and shorter ones balance
+ * a ragged active set better.  The activity tiles stay 16 x 14: every height
+ * gives the same results. */
 int rift_set_march_rows(rift_handle* h, int32_t tile_rows);
 int rift_get_march_rows(rift_handle* h, int32_t* tile_rows);
 
@@ -256,8 +257,8 @@ int rift_get_march_rows(rift_handle* h, int32_t* tile_rows);
  * counterpart): from the current state, runs probe_steps steps on each
  * candidate -- 0 the persistent loop, 1 the per-step graph with the per-tile
  * kernels (one 16 x 14 tile per CTA of 256 threads), 2, 3, 4 the graph with
- * the column-march kernels on items of 2, 1 and 4 tile rows (128 threads per
- * 7-tile-wide item) -- timing each with CUDA events, restores the state
+ * the column-march kernels on items of the default height, 1 and 4 tile rows
+ * -- timing each with CUDA events, restores the state
  * exactly, and keeps the fastest (as rift_set_persistent / rift_set_schedule
  * / rift_set_march_rows would set it).  choice: the candidate's index;
  * ms_per_step[RIFT_AUTOTUNE_CANDIDATES] (may be NULL): the measured times

@@ -30,6 +30,7 @@
 #include "rift_march.cuh"
 #include "rift_update1.cuh"
 #include "rift_persist.cuh"
+#include "rift_flow.cuh"
 #include "rift_ensemble.cuh"
 
 using namespace rift;
@@ -69,6 +70,8 @@ struct rift_handle {
     int persistMax = 0;    // it runs while the active tiles are at most this many
     GridBar* gbar = nullptr;
     int* owner = nullptr;  // [gridSize] tile table of the persistent loop
+    int *items = nullptr, *itemStamp = nullptr;  // [segments x tile rows] item list of k_flow
+    bool flowOk = false;      // k_flow fits one CTA per SM
     int* tileFlag = nullptr;  // [gridSize] stage-1 completion of the persistent loop
     long long persistSteps = 0, graphSteps = 0;  // steps run by each path (diagnostics)
     long long launches = 0;  // kernels launched by the run paths (graph replays count their kernels)
@@ -280,6 +283,8 @@ Params makeParams(rift_handle* h) {
     P.gbar = h->gbar;
     P.owner = h->owner;
     P.tileFlag = h->tileFlag;
+    P.items = h->items;
+    P.itemStamp = h->itemStamp;
     P.mx = h->mx;
     P.my = h->my;
     P.srcIdx = h->srcIdx;
@@ -327,7 +332,7 @@ void destroyGraph(rift_handle* h) {
 uint32_t marchFix(const rift_handle* h) {
     const uint32_t f = h->g.flags & CELL_FLAGS;
     if (((f & F_POINT) != 0) != (h->nsrc > 0)) return 0u;
-    if (f == FIX_RAIN || f == FIX_INFIL_SRC || f == FIX_RAINMAP_DRAIN) return f;
+    if (f == FIX_RAIN || f == FIX_RAIN_INFIL || f == FIX_INFIL_SRC || f == FIX_RAINMAP_DRAIN) return f;
     return 0u;
 }
 
@@ -343,6 +348,7 @@ void launchMarch(const rift_handle* h, const CUtensorMap& tmIn, const Params& P,
     }
     switch (marchFix(h)) {
         case FIX_RAIN: k_march<2, FIX_RAIN><<<grid, MT, 0, s>>>(tmIn, tmE, P, rows, pf); break;
+        case FIX_RAIN_INFIL: k_march<2, FIX_RAIN_INFIL><<<grid, MT, 0, s>>>(tmIn, tmE, P, rows, pf); break;
         case FIX_INFIL_SRC: k_march<2, FIX_INFIL_SRC><<<grid, MT, 0, s>>>(tmIn, tmE, P, rows, pf); break;
         case FIX_RAINMAP_DRAIN: k_march<2, FIX_RAINMAP_DRAIN><<<grid, MT, 0, s>>>(tmIn, tmE, P, rows, pf); break;
         default: k_march<2><<<grid, MT, 0, s>>>(tmIn, tmE, P, rows, pf);
@@ -355,6 +361,16 @@ const void* persistKernel(const rift_handle* h) {
         case FIX_RAIN: return (const void*)k_persist<FIX_RAIN>;
         case FIX_INFIL_SRC: return (const void*)k_persist<FIX_INFIL_SRC>;
         default: return (const void*)k_persist<>;
+    }
+}
+
+const void* flowKernel(const rift_handle* h) {
+    switch (marchFix(h)) {
+        case FIX_RAIN: return (const void*)k_flow<FIX_RAIN>;
+        case FIX_RAIN_INFIL: return (const void*)k_flow<FIX_RAIN_INFIL>;
+        case FIX_INFIL_SRC: return (const void*)k_flow<FIX_INFIL_SRC>;
+        case FIX_RAINMAP_DRAIN: return (const void*)k_flow<FIX_RAINMAP_DRAIN>;
+        default: return (const void*)k_flow<>;
     }
 }
 
@@ -574,6 +590,16 @@ void parallelRows(int ny, size_t cells, F fn) {
     for (auto& x : th) x.join();
 }
 
+// Active tiles up to which the persistent loops run the steps.  k_flow against
+// the step graph, us per step: uniform rain 72 / 82 at 7,708 tiles, 96 / 96 at
+// 10,152, 137 / 122 at 14,577 (beyond L2 the graph's staged update wins); with
+// infiltration, which that update does not stage, 107 / 140 at 10,152 and
+// 362 / 411 at 40,420.
+int defaultPersistMax(const rift_handle* h) {
+    if (h->gridPersist <= 0) return 0;
+    return h->has(RIFT_F_INFILTRATION) ? 40960 : 10240;
+}
+
 bool tileInGrid(const rift_handle* h, int b) {
     int i0 = (b % h->nBX) * TW + 2, j0 = (b / h->nBX) * TH + 2;
     return i0 < h->nx && j0 < h->ny;
@@ -757,9 +783,22 @@ int rift_create(const rift_grid_desc* g, rift_handle** out) {
         CUDA_TRY(h, cudaMalloc(&h->gbar, sizeof(GridBar)));
         CUDA_TRY(h, cudaMalloc(&h->owner, (size_t)G * 4));
         CUDA_TRY(h, cudaMalloc(&h->tileFlag, (size_t)G * 4));
+        const size_t nItem = (size_t)segCount(h->nx) * h->nBY;
+        CUDA_TRY(h, cudaMalloc(&h->items, nItem * 4));
+        CUDA_TRY(h, cudaMalloc(&h->itemStamp, nItem * 4));
+        CUDA_TRY(h, cudaMemset(h->itemStamp, 0, nItem * 4));
+        h->flowOk = true;
+        for (const void* fn : {(const void*)k_flow<>, (const void*)k_flow<FIX_RAIN>,
+                               (const void*)k_flow<FIX_RAIN_INFIL>, (const void*)k_flow<FIX_INFIL_SRC>,
+                               (const void*)k_flow<FIX_RAINMAP_DRAIN>}) {
+            int o = 0;
+            CUDA_TRY(h, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, FLOW_SMEM));
+            CUDA_TRY(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, FLOW_T, FLOW_SMEM));
+            h->flowOk = h->flowOk && o >= 1;
+        }
     }
     h->gridGrow = std::max(1, std::min(NS, h->numSMs * 4));
-    h->persistMax = h->gridPersist > 0 ? h->marchMin * STRIP_TX * STRIP_TY : 0;
+    h->persistMax = defaultPersistMax(h);
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     return RIFT_OK;
 }
@@ -1005,8 +1044,7 @@ int rift_set_persistent(rift_handle* h, int32_t max_active_tiles) {
         return max_active_tiles > 0 ? fail(h, RIFT_ERR_UNSUPPORTED, "no cooperative launch")
                                     : RIFT_OK;
     }
-    h->persistMax = max_active_tiles >= 0 ? max_active_tiles
-                                          : h->marchMin * STRIP_TX * STRIP_TY;
+    h->persistMax = max_active_tiles >= 0 ? max_active_tiles : defaultPersistMax(h);
     destroyGraph(h);  // the step graph holds the bound
     return RIFT_OK;
 }
@@ -1052,13 +1090,36 @@ int persistGrid(const rift_handle* h) {
     return std::max(1, std::min(h->gridPersist, h->numSMs * perSM));
 }
 
-int launchPersist(rift_handle* h, int nsteps) {
-    CUDA_TRY(h, cudaMemsetAsync(h->gbar, 0, GRIDBAR_CLEAR, h->stream));
+// The active set does not fit one tile per CTA of k_persist: k_flow's warps
+// take it (RK2 only).  Against the per-tile phases of k_persist, us per step:
+// 400^2 rain and infiltration, 754 tiles, 38 -> 22; 512^2 rain, 1221 tiles,
+// 34 -> 24; a 2048^2 channel flood, 651 tiles, 34 -> 27; 1024^2 rain, 4810
+// tiles, 86 -> 49.
+bool useFlow(const rift_handle* h) {
+    return h->flowOk && !h->has(RIFT_F_EULER) && h->hst->nActive > h->gridPersist;
+}
+
+// One cooperative launch of the chosen loop (also under capture).
+cudaError_t enqueuePersist(rift_handle* h, int nsteps) {
+    cudaError_t e = cudaMemsetAsync(h->gbar, 0, GRIDBAR_CLEAR, h->stream);
+    if (e != cudaSuccess) return e;
     Params P = makeParams(h);
-    const int grid = persistGrid(h);
+    if (useFlow(h)) {
+        int rows = marchItemRows(h->nx, h->ny, h->numSMs * FLOW_WARPS);
+        int minTiles = h->gridPersist * 3 / 4;  // (hysteresis between the two loops)
+        void* args[] = {(void*)&h->tmAm, (void*)&h->tmBm, (void*)&h->tmEm, (void*)&P, (void*)&nsteps,
+                        (void*)&rows, (void*)&minTiles};
+        return cudaLaunchCooperativeKernel(flowKernel(h), dim3(h->numSMs), dim3(FLOW_T), args, FLOW_SMEM,
+                                           h->stream);
+    }
+    if (h->flowOk && !h->has(RIFT_F_EULER)) P.persistMax = std::min(P.persistMax, h->gridPersist);
     void* args[] = {(void*)&h->tmA, (void*)&h->tmB, (void*)&h->tmE, (void*)&P, (void*)&nsteps};
-    CUDA_TRY(h, cudaLaunchCooperativeKernel(persistKernel(h), dim3(grid), dim3(NT), args, 0,
-                                            h->stream));
+    return cudaLaunchCooperativeKernel(persistKernel(h), dim3(persistGrid(h)), dim3(NT), args, 0,
+                                       h->stream);
+}
+
+int launchPersist(rift_handle* h, int nsteps) {
+    CUDA_TRY(h, enqueuePersist(h, nsteps));
     h->launches += 1;
     return RIFT_OK;
 }
@@ -1085,6 +1146,7 @@ int runSteps(rift_handle* h, int nsteps, bool* mirrorCurrent) {
             h->persistSteps += ran;
             left -= ran;
             if (!h->hst->persistExit) break;  // all steps done, or t_stop reached
+            if (left > 0 && h->hst->nActive <= h->persistMax) continue;  // the other loop's turn
         }
         if (left <= 0) break;
         const int chunk = std::min(left, kGraphChunk);
@@ -1114,7 +1176,7 @@ namespace {
 bool stepGraph(rift_handle* h, int& rc) {
     rc = RIFT_OK;
     if (h->stepGraphBroken) return false;
-    const int grid = persistGrid(h);
+    const int grid = useFlow(h) ? -1 : persistGrid(h);  // -1: k_flow
     int slot = -1;
     for (int k = 0; k < rift_handle::STEP_CACHE; k++)
         if (h->stepExec[k] && h->stepGrid[k] == grid) slot = k;
@@ -1123,9 +1185,6 @@ bool stepGraph(rift_handle* h, int& rc) {
         h->stepNext = (h->stepNext + 1) % rift_handle::STEP_CACHE;
         if (h->stepExec[slot]) cudaGraphExecDestroy(h->stepExec[slot]);
         h->stepExec[slot] = nullptr;
-        Params P = makeParams(h);
-        int one = 1;
-        void* args[] = {(void*)&h->tmA, (void*)&h->tmB, (void*)&h->tmE, (void*)&P, (void*)&one};
         cudaGraph_t g = nullptr;
         if (cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             h->stepGraphBroken = true;
@@ -1133,8 +1192,7 @@ bool stepGraph(rift_handle* h, int& rc) {
             return false;
         }
         cudaMemcpyAsync(h->st, h->hst, sizeof(DevState), cudaMemcpyHostToDevice, h->stream);
-        cudaMemsetAsync(h->gbar, 0, GRIDBAR_CLEAR, h->stream);
-        cudaLaunchCooperativeKernel(persistKernel(h), dim3(grid), dim3(NT), args, 0, h->stream);
+        enqueuePersist(h, 1);
         cudaMemcpyAsync(h->hst, h->st, sizeof(DevState), cudaMemcpyDeviceToHost, h->stream);
         cudaError_t e = cudaStreamEndCapture(h->stream, &g);
         if (e != cudaSuccess || !g ||
@@ -1989,7 +2047,7 @@ void rift_destroy(rift_handle* h) {
     for (int k = 0; k < 3; k++)
         for (int q = 0; q < 2; q++)
             if (h->maps[k][q]) cudaFree(h->maps[k][q]);
-    for (void* p : {(void*)h->gbar, (void*)h->owner, (void*)h->tileFlag,
+    for (void* p : {(void*)h->gbar, (void*)h->owner, (void*)h->tileFlag, (void*)h->items, (void*)h->itemStamp,
                     (void*)h->strips, (void*)h->stripFlag, (void*)h->wet, (void*)h->prevAct,
                     (void*)h->act, (void*)h->deact,
                     (void*)h->inact, (void*)h->srcIdx, (void*)h->srcTileStart,

@@ -22,6 +22,10 @@ namespace rift {
 
 constexpr int GROW_LISTS = 4;            // scheduled active, deactivated, inactive, strips
 constexpr int STRIPS_PER_ROUND = NT / 16;
+constexpr int SEG = 60;                  // columns of a march item
+
+// Segments of 60 columns across the interior.
+__host__ __device__ constexpr int segCount(int nx) { return (nx - 4 + SEG - 1) / SEG; }
 
 // active(t) of tile b: wet itself or a wet 4-neighbour; tile 0 always.
 // The five flags are loaded together (no short-circuit: a dry tile would
@@ -102,8 +106,11 @@ __device__ __forceinline__ GrowItem growItem(const Params& P, int base, int s1) 
 // publishes the list sizes and clears the counters for the next step;
 // without, the caller reads the counters after a grid barrier and publishes
 // them later (publishGrow).
-template <bool PUBLISH = true>
-__device__ void growAppend(const Params& P, unsigned* staleDst = nullptr) {
+// With ITEMS the (60-column segment, tile row) pairs that hold a scheduled tile
+// are listed too (P.items, *itemCnt): the first tile to set a pair's stamp
+// appends it; the caller clears the listed pairs' stamps after its barrier.
+template <bool PUBLISH = true, bool ITEMS = false>
+__device__ void growAppend(const Params& P, unsigned* staleDst = nullptr, int* itemCnt = nullptr) {
     DevState* s = P.st;
     const int tid = threadIdx.x, lane = tid & 31;
     int s0, s1;
@@ -126,6 +133,13 @@ __device__ void growAppend(const Params& P, unsigned* staleDst = nullptr) {
             if (t.f[q]) lists[q][bq + __popc(bal[q] & below)] = q == 3 ? t.strip : t.b;
         }
         if (t.f[0]) cells += (unsigned long long)t.cells;
+        if (ITEMS && t.f[0]) {
+            const int nSeg = segCount(P.nx), bx = t.b % P.nBX, by = t.b / P.nBX;
+            const int s1 = min(TW * bx + TW - 1, P.nx - 5) / SEG;
+            for (int s = TW * bx / SEG; s <= s1; s++)
+                if (atomicExch(&P.itemStamp[by * nSeg + s], 1) == 0)
+                    P.items[atomicAdd(itemCnt, 1)] = by * nSeg + s;
+        }
         if (t.b >= 0) {
             if (t.v) {  // the march folds an active tile's speeds into a cleared entry
                 P.mx[t.b] = 0.f;

@@ -58,10 +58,11 @@ constexpr uint32_t F_RAIN_U = 1u << 0, F_RAIN_G = 1u << 1, F_DRAIN_U = 1u << 2,
 constexpr uint32_t CELL_FLAGS = F_RAIN_U | F_RAIN_G | F_DRAIN_U | F_DRAIN_G | F_INFIL | F_SURGE |
                                 F_EULER | F_SAVE_MAX | F_SAVE_ARR | F_TILE_ACC | F_POINT |
                                 F_CHECKVOL;
-// the fixed sets with march instantiations: uniform rain; infiltration with
-// a point hydrograph; gridded rain with a uniform drain (all with tile
-// acceleration)
+// the fixed sets with instantiations: uniform rain, without and with
+// infiltration; infiltration with a point hydrograph; gridded rain with a
+// uniform drain (all with tile acceleration)
 constexpr uint32_t FIX_RAIN = F_RAIN_U | F_TILE_ACC;
+constexpr uint32_t FIX_RAIN_INFIL = F_RAIN_U | F_INFIL | F_TILE_ACC;
 constexpr uint32_t FIX_INFIL_SRC = F_INFIL | F_POINT | F_TILE_ACC;
 constexpr uint32_t FIX_RAINMAP_DRAIN = F_RAIN_G | F_DRAIN_U | F_TILE_ACC;
 
@@ -148,6 +149,8 @@ struct Params {
     int persistMax;    // the persistent step kernel runs while active tiles <= this
     struct GridBar* gbar;            // grid barrier of the persistent kernel
     int* owner;        // [gridSize] tile -> CTA of the persistent loop's tile table, or -1
+    int* items;        // k_flow: (segment, tile row) pairs holding an active tile
+    int* itemStamp;    // [segments x tile rows] k_flow: the pair is listed
     int* tileFlag;     // [gridSize] persistent loop: last step whose stage 1 the tile finished
     float* mx;
     float* my;
@@ -179,6 +182,9 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 }
 __device__ __forceinline__ void fence_mbar_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+__device__ __forceinline__ void fence_proxy_async_global() {
+    asm volatile("fence.proxy.async.global;" ::: "memory");
 }
 __device__ __forceinline__ void fence_proxy_async() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1008,6 +1014,12 @@ struct CellSrc {
     bool srcCell;        // the cell holds a point source
 };
 
+// `tile` for cellSources: -1 when the tile holds no point source.
+__device__ __forceinline__ int sourceTile(const Params& P, int tile) {
+    return P.nsrc > 0 && P.srcTileStart[tile + 1] > P.srcTileStart[tile] ? tile : -1;
+}
+
+// tile: the cell's tile, or -1 when it holds no point source.
 // BED: add the bed-slope source here (false: the caller's dhu, dhv hold it).
 // RAINPRE: the cell's rain-map entries were loaded ahead into pre[6], pre[7].
 template <int STAGE, bool PREF = false, bool BED = true, uint32_t FIX = 0, bool RAINPRE = false>
@@ -1041,7 +1053,7 @@ __device__ __forceinline__ CellSrc cellSources(const Params& P, const StageConst
         drained += d;
     }
     bool srcCell = false;
-    if ((FIX == 0 || (FIX & F_POINT)) && P.nsrc > 0) {
+    if ((FIX == 0 || (FIX & F_POINT)) && P.nsrc > 0 && tile >= 0) {
         const int flat = j * P.nx + i;
         for (int q = P.srcTileStart[tile]; q < P.srcTileStart[tile + 1]; q++) {
             int sidx = P.srcTileList[q];

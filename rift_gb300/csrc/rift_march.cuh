@@ -15,7 +15,7 @@
 // Rows arrive through TMA in chunks of two rows of 64 columns, a ring of
 // three chunks per warp: two hold the three rows a step of the march reads,
 // the third is in flight during two rows.  The cell's own values (stage 2:
-// U^n, maps, infiltration) are loaded one row ahead; on grids
+// U^n, maps, infiltration) are loaded at the start of its row; on grids
 // larger than L2 one prefetch instruction per row asks for them MPF rows
 // ahead (lane q takes one 128-byte line).
 // A cell is updated only when its reference tile is active, so results and
@@ -34,7 +34,7 @@
 // 294); they issue on 60% of cycles, the packed instructions' FMA pipe is 60%
 // busy, DRAM moves at 4.6 and 5.0 TB/s.  A lone warp needs 0.56 us per row.
 #pragma once
-#include "rift_kernels.cuh"
+#include "rift_grow.cuh"
 #include "rift_pair.cuh"
 
 namespace rift {
@@ -42,7 +42,7 @@ namespace rift {
 constexpr int MW = 4;                  // warps per CTA
 constexpr int MT = MW * 32;            // threads per CTA
 constexpr int MCOLS = STRIP_TX * TW;   // columns of the grow's strips (112)
-constexpr int MSEG = 60;               // columns a warp owns
+constexpr int MSEG = SEG;              // columns a warp owns
 constexpr int MBOX = 64;               // columns a warp stages
 constexpr int MCR = 2;                 // rows per staged chunk
 constexpr int MNS = 3;                 // chunks in a warp's ring
@@ -129,7 +129,7 @@ __device__ __forceinline__ void rowFluxX(const Cell2& c, P2 eW, P2 eE, float kap
 // that allows (an item also loads 4 halo rows and reconstructs about 3 rows'
 // worth before its first).  4096^2 cells on 2432 warps: 59 rows in two rounds.
 inline int marchItemRows(int nx, int ny, int warps) {
-    const long long segs = (nx - 4 + MSEG - 1) / MSEG;
+    const long long segs = segCount(nx);
     int best = 2;
     double cost = 1e300;
     for (int r = 2; r <= 64; r++) {
@@ -143,18 +143,40 @@ inline int marchItemRows(int nx, int ny, int warps) {
     return best;
 }
 
-// Segments of 60 columns across the interior.
-__host__ __device__ constexpr int marchSegs(int nx) { return (nx - 4 + MSEG - 1) / MSEG; }
+// Ghost columns of U beside rows [j0, j1) of segment seg, a row per lane (the
+// cube root is long: once per 32 rows instead of once per row).
+template <class On>
+__device__ __forceinline__ void ghostColumns(const Params& P, float* U, int seg, int j0, int j1, On on) {
+    const size_t pl = (size_t)P.planeSize;
+    __syncwarp();
+    for (int side = 0; side < 2; side++) {
+        const int gi = side ? P.nx - 3 : 2;
+        if (gi < MSEG * seg + 2 || gi >= MSEG * (seg + 1) + 2) continue;
+        for (int j = j0 + (int)(threadIdx.x & 31); j < j1; j += 32) {
+            if (!on((j - 2) / TH, (gi - 2) / TW)) continue;
+            const unsigned c = (unsigned)j * (unsigned)P.pitch + (unsigned)gi;
+            writeGhostCols(P, U, j, gi, U[c], U[pl + c], U[2 * pl + c]);
+        }
+    }
+}
+
+// Stage 2 (RK2) folds an active tile's wet flag and speeds into cleared
+// entries: cleared between the grow and stage 2, by every item that holds
+// rows of the tile.
+__device__ __forceinline__ void clearTile(const Params& P, int tile) {
+    P.wet[tile] = 0;
+    P.mx[tile] = 0.f;
+    P.my[tile] = 0.f;
+}
 
 // Rows [j0, j1) of segment seg by one warp.  on(by, bx): is the tile active?
 // (called by all lanes; false for lanes that own no interior column).
+// CLEAR (stage 1): see clearTile.
 // STAGE 1: reads U^n (A) -> flux divergence + bed source (D), the speed
-//          maxima of active cells (tmx, tmy); Euler mode: tile speeds.  RK2:
-//          clears the tiles' wet flags for stage 2.
+//          maxima of active cells (tmx, tmy); Euler mode: tile speeds.
 // STAGE 2: reads U* (B) and U^n (A) at the cell -> writes U^{n+1} (A),
-//          F^{n+1} (FA), outputs, tile wet flags and tile speeds (mx, my were
-//          cleared since stage 1's flux pass).
-template <int STAGE, uint32_t FIX, class On>
+//          F^{n+1} (FA), outputs, tile wet flags and tile speeds.
+template <int STAGE, uint32_t FIX, bool CLEAR, class On>
 __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C, const CUtensorMap* tmIn,
                                           const CUtensorMap* tmE, MarchRing& S, uint32_t& par, int seg,
                                           int j0, int j1, On on, bool led, Led& L, float& tmx,
@@ -204,8 +226,10 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
         return ok;
     };
     __syncwarp();  // the previous item no longer reads the ring
-    if (lane == 0)
+    if (lane == 0) {
+        fence_proxy_async_global();  // the copies see what was stored before the last barrier
         for (int c = 0; c < MNS && c < nch; c++) issue(c, c);
+    }
     if (!acquire(0) || !acquire(1)) return false;
     // rows j, j + 1, j + 2 of the current output row
     const float* rc = &S.slot[1].s[0][0][2 * lane];
@@ -228,8 +252,8 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
         faceFlux2<1>(a, M, kappa, fS, s);
     }
     // the row's centre values (stage 2: U^n; rain maps or F, K, F^n when the
-    // instantiation reads them ahead), one row ahead of their use
-    P2 pre[6], nextPre[6];
+    // instantiation reads them ahead)
+    P2 pre[6];
     auto loadCentre = [&](P2 (&d)[6], int jj) {
         const unsigned c = (unsigned)jj * pitch + ic;
         d[0] = ld2(P.A + c);
@@ -245,15 +269,15 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
         }
     };
 #pragma unroll
-    for (int q = 0; q < 6; q++) pre[q] = nextPre[q] = both(0.f);
-    if (STAGE == 2) loadCentre(pre, j0);
+    for (int q = 0; q < 6; q++) pre[q] = both(0.f);
 
     int sl = 1;  // slot of the chunk that holds row j + 1
     int by = (j0 - 2) / TH, rt = (j0 - 2) % TH;  // tile row, row in it
     bool act = on(by, bx);
+    int src = STAGE == 2 && act ? sourceTile(P, by * P.nBX + bx) : -1;
     float ax = 0.f, ay = 0.f;
     bool wet = false;
-    if (STAGE == 1 && !euler && leader && act) P.wet[by * P.nBX + bx] = 0;
+    if (CLEAR && !euler && leader && act) clearTile(P, by * P.nBX + bx);
     constexpr int UNROLL = STAGE == 1 ? 2 : 1;
 #pragma unroll UNROLL
     for (int j = j0; j < j1; j++) {
@@ -267,7 +291,8 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
             if (!acquire(sl)) return false;
             rl = &S.slot[sl].s[0][0][2 * lane];
         }
-        if (STAGE == 2) loadCentre(nextPre, j + 1);
+        if (STAGE == 2) loadCentre(pre, j);  // in flight during both directions' fluxes
+        if (STAGE == 2 && FIX == 0) prefetchMaps(P, fl, (unsigned)j * pitch + ic);
         if (STAGE == 2 && pfB) prefetch_l2(pfB + (size_t)((unsigned)min(j + MPF, P.rows - 1) * pitch));
         const P2 eW = row2(rc, 3), eE = row2(rc, 4);
         P2 fN[3], sy, fx[3], fW0, fE0, sx;
@@ -300,7 +325,6 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
                 st2(P.D + pl + c, d[1]);
                 st2(P.D + 2 * pl + c, d[2]);
             } else {
-                const int tile = by * P.nBX + bx;
                 float r[2][3];
 #pragma unroll
                 for (int k = 0; k < 2; k++) {
@@ -310,7 +334,7 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
                     const float pk[8] = {at(pre[0]), at(pre[1]), at(pre[2]), at(pre[3]),
                                          at(pre[4]), at(pre[5]), at(pre[3]), at(pre[4])};
                     const CellSrc s = cellSources<2, INFPRE, false, FIX, RAINPRE>(
-                        P, C, tile, j, i + k, at(d[0]), at(d[1]), at(d[2]), hC, u0, v0, 0.f, 0.f,
+                        P, C, src, j, i + k, at(d[0]), at(d[1]), at(d[2]), hC, u0, v0, 0.f, 0.f,
                         0.f, 0.f, pk);
                     wet |= cellResult<2, INFPRE, FIX>(P, C, j, i + k, s, hC, u0, v0, pk,
                                                       led ? &L : nullptr, r[k][0], r[k][1], r[k][2]);
@@ -350,13 +374,12 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
             if (j + 1 < j1) {
                 by++;
                 act = on(by, bx);
-                if (STAGE == 1 && !euler && leader && act) P.wet[by * P.nBX + bx] = 0;
+                src = STAGE == 2 && act ? sourceTile(P, by * P.nBX + bx) : -1;
+                if (CLEAR && !euler && leader && act) clearTile(P, by * P.nBX + bx);
             }
         }
 #pragma unroll
         for (int q = 0; q < 3; q++) fS[q] = fN[q];
-#pragma unroll
-        for (int q = 0; q < 6; q++) pre[q] = nextPre[q];
         yP = yn;
         dN = dNN;
         cur = nxt;
@@ -365,20 +388,7 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
         rn = rl;
         rl += MBOX;
     }
-    if (STAGE == 2) {
-        // ghost columns, a row per lane (the cube root is long: once per 32
-        // rows instead of once per row)
-        __syncwarp();
-        for (int side = 0; side < 2; side++) {
-            const int gi = side ? P.nx - 3 : 2;
-            if (gi < MSEG * seg + 2 || gi >= MSEG * (seg + 1) + 2) continue;
-            for (int j = j0 + lane; j < j1; j += 32) {
-                if (!on((j - 2) / TH, (gi - 2) / TW)) continue;
-                const unsigned c = (unsigned)j * pitch + (unsigned)gi;
-                writeGhostCols(P, P.A, j, gi, P.A[c], P.A[pl + c], P.A[2 * pl + c]);
-            }
-        }
-    }
+    if (STAGE == 2 && edge) ghostColumns(P, P.A, seg, j0, j1, on);
     return true;
 }
 
@@ -421,7 +431,7 @@ __global__ void __launch_bounds__(MT, MARCH_CTAS) k_march(const __grid_constant_
     Led L;
     ledZero(L);
     float tmx = 0.f, tmy = 0.f;
-    const int nSeg = marchSegs(P.nx), nGroup = (P.ny - 4 + itemRows - 1) / itemRows;
+    const int nSeg = segCount(P.nx), nGroup = (P.ny - 4 + itemRows - 1) / itemRows;
     auto on = [&](int by, int bx) { return bx >= 0 && P.prevAct[by * P.nBX + bx] != 0; };
     for (int item = blockIdx.x * MW + warp; item < nSeg * nGroup; item += gridDim.x * MW) {
         const int seg = item % nSeg, j0 = 2 + itemRows * (item / nSeg);
@@ -434,7 +444,7 @@ __global__ void __launch_bounds__(MT, MARCH_CTAS) k_march(const __grid_constant_
         for (int q = lane; q < nb * (by1 - by0 + 1); q += 32)
             any |= on(by0 + q / nb, bx0 + q % nb);
         if (!__any_sync(FULL, any)) continue;
-        if (!marchRows<STAGE, FIX>(P, C, &tmIn, &tmE, S, par, seg, j0, j1, on, led, L, tmx, tmy, pf != 0)) {
+        if (!marchRows<STAGE, FIX, STAGE == 1>(P, C, &tmIn, &tmE, S, par, seg, j0, j1, on, led, L, tmx, tmy, pf != 0)) {
             if (lane == 0) atomicOr(&P.st->error, ERR_TMA_TIMEOUT);
             break;
         }

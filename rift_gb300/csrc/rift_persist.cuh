@@ -50,6 +50,9 @@ struct GridBar {
     int ownedCnt[2];       // owned tiles found active
     int schedCnt[2];       // scheduled tiles found by the scan
     int freeTop;           // entries of freeStack
+    int itemCnt[2];        // k_flow, by step parity: listed items,
+    int changed[2];        //   the active set differs from the last step's,
+    unsigned guess[2][2];  //   speed maxima of a flux phase run on the last step's set
     float nextRates[6];    // the next step's source rates and series state (spare CTA)
     // (the tables below are written before they are read in every launch:
     // only the part above is cleared, GRIDBAR_CLEAR bytes)
@@ -70,9 +73,6 @@ __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
 }
 __device__ __forceinline__ void red_add_release_gpu(unsigned* p, unsigned v) {
     asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ void fence_proxy_async_global() {
-    asm volatile("fence.proxy.async.global;" ::: "memory");
 }
 
 // Grid-wide barrier.  Every CTA adds 1 to a monotonic counter with release
