@@ -269,8 +269,8 @@ int rift_autotune(rift_handle* h, int32_t probe_steps, int32_t* choice, double* 
 /* Ensembles (no reference counterpart; the reference runs one scenario per
  * process): members -- handles created, uploaded and initialised as usual,
  * on one device, of any sizes and options -- advance together in one
- * persistent cooperative kernel that walks device queues of (member, tile)
- * work items; each member keeps its own dt, t, sources and outputs, and its
+ * persistent cooperative kernel that walks a device queue over the members'
+ * rows; each member keeps its own dt, t, sources and outputs, and its
  * results are those of a run of its own.  rift_ensemble_run advances each
  * member until t >= t_stop or max_steps of its steps; t_out and steps_out
  * (n entries each, may be NULL) receive each member's final t and steps.
@@ -281,9 +281,7 @@ int rift_ensemble_run(rift_ensemble* e, double t_stop, int32_t max_steps, double
                       int32_t* steps_out);
 /* Members with at least min_cells interior cells (0, the default: none) are
  * not stepped by the persistent ensemble kernel: after it, each of them runs
- * on its own per-step graph, smallest first, with the whole GPU (the column
- * march on dense grids, about 2.5x the cell rate of the kernel's per-tile
- * code).  Their results are those of a run of their own, as every member's. */
+ * on its own, smallest first, with the whole GPU.  Their results are those of a run of their own, as every member's. */
 int rift_ensemble_set_solo_cells(rift_ensemble* e, int64_t min_cells);
 /* Per member (n entries): the device time, in seconds, from the start of the
  * last rift_ensemble_run's kernel to the end of the member's last step in it

@@ -11,6 +11,8 @@
 #pragma once
 #include <cstdint>
 
+#include "rift_pair.cuh"
+
 namespace rift {
 
 constexpr float kG = 9.80665f;         // grid.cu:28
@@ -20,55 +22,59 @@ constexpr float kTheta = 1.3f;         // grid.cu:30
 // Effective limiter of the reference (grid.cu:62-80).  Its signf reads the
 // low word of a double and is never negative, so minmod(a,b,c) evaluates to
 // +min(|a|,|b|,|c|) (times a factor within 1.5e-6 of 1) and the slope is
-//   0.5 * min(theta|d+|, 0.5|d+ + d-|, theta|d-|)  >= 0.
-// It is zero whenever one argument is zero, which min() already gives.
-// The outer factor 0.5 is folded into the three terms (0.65 = 1.3 / 2 and
-// 0.25 exactly, so each product is the same float as half the unfolded one).
-__device__ __forceinline__ float slope(float dp, float dm) {
-    constexpr float kHalfTheta = 0.5f * kTheta;
-    float a = kHalfTheta * fabsf(dp);
-    float b = 0.25f * fabsf(dp + dm);
-    float c = kHalfTheta * fabsf(dm);
-    return fminf(fminf(a, b), c);
+//   0.5 * min(theta|d+|, 0.5|d+ + d-|, theta|d-|)  >= 0
+// = kSlope * min(|d+|, kMid |d+ + d-|, |d-|), the minimum given here: the
+// factor goes into the fma that adds the slope.  It is zero whenever one
+// argument is zero, which min() already gives.
+constexpr float kSlope = 0.5f * kTheta;
+constexpr float kMid = 0.5f / kTheta;
+template <class V>
+__device__ __forceinline__ V limited(V dp, V dm) {
+    return minAbs3(dp, dm, vmul(splat<V>(kMid), vadd(dp, dm)));
 }
 
-// Reconstructed face values of one cell in one direction (Construct,
-// grid.cu:91-116), in depth form.  P = the face toward +x (+y), M = toward -x.
+// State at one face of a cell (of two cells: V = P2): depth, hu, hv.
+template <class V>
+struct Face {
+    V h, u, v;
+};
+
+// Reconstruction of one cell in one direction (Construct, grid.cu:91-116), in
+// depth form, from the limited differences tw, tu, tv of the surface and the
+// momenta: P at the face toward +x (+y), M toward -x.  eM/eP: the cell's - and
+// + face elevation offsets.
+// The wet/dry correction against the face elevations: wBar = 2w, so the face
+// depths add up to bar = 2h - eP - eM, and "if (hP < 0) hP = 0, hM = bar; if
+// (hM < 0) hM = 0, hP = bar" is min(max(hP, 0), bar) and max(min(hM, bar), 0).
+template <class V>
+__device__ __forceinline__ void construct(V h0, V u0, V v0, V tw, V tu, V tv, V eM, V eP, Face<V>& P,
+                                          Face<V>& M) {
+    const V k = splat<V>(kSlope), nk = splat<V>(-kSlope), zero = splat<V>(0.f);
+    const V hP = vsub(vfma(k, tw, h0), eP), hM = vsub(vfma(nk, tw, h0), eM);
+    const V bar = vsub(vadd(h0, h0), vadd(eP, eM));
+    P.h = vmin(vmax(hP, zero), bar);
+    M.h = vmax(vmin(hM, bar), zero);
+    P.u = vfma(k, tu, u0);
+    M.u = vfma(nk, tu, u0);
+    P.v = vfma(k, tv, v0);
+    M.v = vfma(nk, tv, v0);
+}
+
+// Reconstructed face values of one cell from its neighbours' states.
 struct Rec {
     float hP, uP, vP;  // depth, hu, hv at the + face
     float hM, uM, vM;  // at the - face
 };
 
 // h0/u0/v0: the cell; hp../hm..: its + and - neighbours in this direction;
-// eM/eP: the cell's - and + face elevation offsets; dP, dM: reference
-// elevation steps to the + and - neighbour.
+// dP, dM: reference elevation steps to the + and - neighbour.
 __device__ __forceinline__ Rec construct(float h0, float u0, float v0, float hp, float up, float vp,
                                          float hm, float um, float vm, float eM, float eP,
                                          float dP, float dM) {
-    float sw = slope(dP + (hp - h0), dM + (h0 - hm));
-    float su = slope(up - u0, u0 - um);
-    float sv = slope(vp - v0, v0 - vm);
-    Rec r;
-    float hP = (h0 + sw) - eP;
-    float hM = (h0 - sw) - eM;
-    // wet/dry correction against the face elevations; wBar = 2w, so the
-    // corrected depth on the other face is 2h - eP - eM.
-    float hBar = (h0 + h0) - (eP + eM);
-    if (hP < 0.f) {
-        hP = 0.f;
-        hM = hBar;
-    }
-    if (hM < 0.f) {
-        hP = hBar;
-        hM = 0.f;
-    }
-    r.hP = hP;
-    r.hM = hM;
-    r.uP = u0 + su;
-    r.uM = u0 - su;
-    r.vP = v0 + sv;
-    r.vM = v0 - sv;
-    return r;
+    Face<float> P, M;
+    construct(h0, u0, v0, limited(vadd(dP, vsub(hp, h0)), vadd(dM, vsub(h0, hm))),
+              limited(vsub(up, u0), vsub(u0, um)), limited(vsub(vp, v0), vsub(v0, vm)), eM, eP, P, M);
+    return Rec{P.h, P.u, P.v, M.h, M.u, M.v};
 }
 
 // Depth-only part of the reconstruction (speed pass): depth and the normal
@@ -79,90 +85,89 @@ struct RecN {
 
 __device__ __forceinline__ RecN constructN(float h0, float q0, float hp, float qp, float hm,
                                            float qm, float eM, float eP, float dP, float dM) {
-    float sw = slope(dP + (hp - h0), dM + (h0 - hm));
-    float sq = slope(qp - q0, q0 - qm);
-    float hP = (h0 + sw) - eP;
-    float hM = (h0 - sw) - eM;
-    float hBar = (h0 + h0) - (eP + eM);
-    if (hP < 0.f) {
-        hP = 0.f;
-        hM = hBar;
-    }
-    if (hM < 0.f) {
-        hP = hBar;
-        hM = 0.f;
-    }
-    RecN r;
-    r.hP = hP;
-    r.hM = hM;
-    r.qP = q0 + sq;
-    r.qM = q0 - sq;
-    return r;
+    Face<float> P, M;
+    construct(h0, q0, q0, limited(vadd(dP, vsub(hp, h0)), vadd(dM, vsub(h0, hm))),
+              limited(vsub(qp, q0), vsub(q0, qm)), 0.f, eM, eP, P, M);
+    return RecN{P.h, P.u, M.h, M.u};
 }
 
-// Desingularised velocity factor 2h / (h^2 + max(h^2, kappa)) (grid.cu:82-84).
-__device__ __forceinline__ float velFactor(float h, float kappa) {
-    float h2 = h * h;
-    return (2.f * h) / (h2 + fmaxf(h2, kappa));
+// Desingularised velocity factor 2h / (h^2 + max(h^2, kappa)) (grid.cu:82-84),
+// both halves of the fraction halved.
+template <class V>
+__device__ __forceinline__ V velFactor(V h, float kappa) {
+    const V h2 = vmul(h, h);
+    return vmul(h, vrcp(vmax(h2, vfma(splat<V>(0.5f), h2, splat<V>(0.5f * kappa)))));
 }
 
-// Local speed at a face (the mx / my of getHX / getHY, grid.cu:118-214),
-// from the upstream cell's + face (L) and the downstream cell's - face (R);
-// qn is the momentum normal to the face.
-__device__ __forceinline__ float faceSpeed(float hL, float qL, float hR, float qR, float kappa) {
-    float uL = qL * velFactor(hL, kappa);
-    float uR = qR * velFactor(hR, kappa);
-    float cL = sqrtf(kG * hL), cR = sqrtf(kG * hR);
-    float ap = fmaxf(fmaxf(uL + cL, uR + cR), 0.f);
-    float am = fminf(fminf(uL - cL, uR - cR), 0.f);
-    return fmaxf(ap, -am);
+// One side of a face: velocities (n normal, t tangential), the momenta formed
+// from them, the wave speeds n + c and c - n, and the flux F(U), zero where
+// the depth is not positive (formed from the depth clamped at 0).
+template <class V>
+struct Side {
+    V qn, qt, sp, sm, f0, fn, ft;
+};
+template <class V>
+__device__ __forceinline__ Side<V> faceSide(V h, V qn, V qt, float kappa) {
+    Side<V> s;
+    const V r = velFactor(h, kappa);
+    const V n = vmul(qn, r), t = vmul(qt, r);
+    s.qn = vmul(h, n);
+    s.qt = vmul(h, t);
+    const V c = vsqrt(vmul(splat<V>(kG), h));
+    s.sp = vadd(c, n);
+    s.sm = vsub(c, n);
+    const V hp = vmax(h, splat<V>(0.f));
+    s.f0 = vmul(hp, n);
+    s.fn = vfma(s.f0, n, vmul(vmul(splat<V>(0.5f * kG), hp), hp));
+    s.ft = vmul(s.f0, t);
+    return s;
 }
 
 // Central-upwind numerical flux through one face (getHX for DIR 0, getHY for
-// DIR 1; grid.cu:118-214, computeH grid.cu:86-89).  f[0] mass, f[1] x
-// momentum, f[2] y momentum.  Returns the local speed max(a+, -a-).
+// DIR 1; grid.cu:118-214, computeH grid.cu:86-89), from the upstream cell's +
+// face (L) and the downstream cell's - face (R).  f[0] mass, f[1] x momentum,
+// f[2] y momentum; returns the local speed max(a+, -a-).  a- enters as its
+// magnitude; at a dry face (a+ = a- = 0) every product is zero, so 1 / max(a+
+// - a-, tiny) takes the place of a branch.
+template <int DIR, class V>
+__device__ __forceinline__ V faceFlux(const Face<V>& L, const Face<V>& R, float kappa, V f[3]) {
+    const Side<V> a = faceSide(L.h, DIR == 0 ? L.u : L.v, DIR == 0 ? L.v : L.u, kappa);
+    const Side<V> b = faceSide(R.h, DIR == 0 ? R.u : R.v, DIR == 0 ? R.v : R.u, kappa);
+    const V ap = vmaxz(a.sp, b.sp), am = vmaxz(a.sm, b.sm);
+    const V r = vrcp(vmax(vadd(ap, am), splat<V>(1e-30f)));
+    const V k = vmul(vmul(ap, am), r);
+    f[0] = vfma(vfma(ap, a.f0, vmul(am, b.f0)), r, vmul(k, vsub(L.h, R.h)));
+    const V fn = vfma(vfma(ap, a.fn, vmul(am, b.fn)), r, vmul(k, vsub(a.qn, b.qn)));
+    const V ft = vfma(vfma(ap, a.ft, vmul(am, b.ft)), r, vmul(k, vsub(a.qt, b.qt)));
+    f[1] = DIR == 0 ? fn : ft;
+    f[2] = DIR == 0 ? ft : fn;
+    return vmax(ap, am);
+}
 template <int DIR>
 __device__ __forceinline__ float faceFlux(float hL, float huL, float hvL, float hR, float huR,
                                           float hvR, float kappa, float f[3]) {
-    float rL = velFactor(hL, kappa), rR = velFactor(hR, kappa);
-    float uL = huL * rL, vL = hvL * rL, uR = huR * rR, vR = hvR * rR;
-    // momenta recomputed from the desingularised velocities
-    float quL = hL * uL, qvL = hL * vL, quR = hR * uR, qvR = hR * vR;
-    float cL = sqrtf(kG * hL), cR = sqrtf(kG * hR);
-    float nL = DIR == 0 ? uL : vL;
-    float nR = DIR == 0 ? uR : vR;
-    float ap = fmaxf(fmaxf(nL + cL, nR + cR), 0.f);
-    float am = fminf(fminf(nL - cL, nR - cR), 0.f);
-    float pL = 0.5f * kG * hL * hL, pR = 0.5f * kG * hR * hR;
-    float FL0, FL1, FL2, FR0, FR1, FR2;
-    if (DIR == 0) {
-        FL0 = quL;
-        FL1 = quL * uL + pL;
-        FL2 = quL * vL;
-        FR0 = quR;
-        FR1 = quR * uR + pR;
-        FR2 = quR * vR;
-    } else {
-        FL0 = qvL;
-        FL1 = qvL * uL;
-        FL2 = qvL * vL + pL;
-        FR0 = qvR;
-        FR1 = qvR * uR;
-        FR2 = qvR * vR + pR;
-    }
-    if (!(hL > 0.f)) FL0 = FL1 = FL2 = 0.f;
-    if (!(hR > 0.f)) FR0 = FR1 = FR2 = 0.f;
-    float d = ap - am;
-    if (d > 0.f) {
-        float r = 1.f / d;
-        float k = ap * am * r;
-        f[0] = (ap * FL0 - am * FR0) * r + k * (hR - hL);
-        f[1] = (ap * FL1 - am * FR1) * r + k * (quR - quL);
-        f[2] = (ap * FL2 - am * FR2) * r + k * (qvR - qvL);
-    } else {
-        f[0] = f[1] = f[2] = 0.f;
-    }
-    return fmaxf(ap, -am);
+    return faceFlux<DIR>(Face<float>{hL, huL, hvL}, Face<float>{hR, huR, hvR}, kappa, f);
+}
+
+// Local speed at a face (the mx / my of getHX / getHY, grid.cu:118-214); qn is
+// the momentum normal to the face.
+__device__ __forceinline__ float faceSpeed(float hL, float qL, float hR, float qR, float kappa) {
+    float f[3];
+    return faceFlux<0>(Face<float>{hL, qL, 0.f}, Face<float>{hR, qR, 0.f}, kappa, f);
+}
+
+// Flux divergence from the differences of the fluxes through a cell's east and
+// west (fx) and north and south faces (fy).
+template <class V>
+__device__ __forceinline__ V divergence(V fx, V fy, float inv_dx, float inv_dy) {
+    return vfma(fx, splat<V>(-inv_dx), vmul(fy, splat<V>(-inv_dy)));
+}
+
+// d plus the bed-slope source of a momentum equation (grid.cu:701,751-752): eM
+// and eP are the cell's face offsets in the direction, inv its inverse width.
+template <class V>
+__device__ __forceinline__ V addBed(V d, V hC, V eM, V eP, float inv) {
+    return vfma(vmul(splat<V>(-kG), hC), vmul(vsub(eP, eM), splat<V>(inv)), d);
 }
 
 // Green-Ampt infiltration rate (grid.cu:791-805), clamped to [0, h/dt].

@@ -768,6 +768,10 @@ int rift_create(const rift_grid_desc* g, rift_handle** out) {
     h->gridSpeed = std::max(1, std::min(G, h->numSMs * occ));
     h->gridTrack = std::max(1, std::min(G, h->numSMs * 4));
     h->gridDt = std::max(1, std::min((G + 255) / 256, h->numSMs * 2));
+    const size_t nItem = (size_t)segCount(h->nx) * h->nBY;
+    CUDA_TRY(h, cudaMalloc(&h->items, nItem * 4));
+    CUDA_TRY(h, cudaMalloc(&h->itemStamp, nItem * 4));
+    CUDA_TRY(h, cudaMemset(h->itemStamp, 0, nItem * 4));
     // the cooperative step kernel: every CTA resident at once
     int coop = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
@@ -783,10 +787,6 @@ int rift_create(const rift_grid_desc* g, rift_handle** out) {
         CUDA_TRY(h, cudaMalloc(&h->gbar, sizeof(GridBar)));
         CUDA_TRY(h, cudaMalloc(&h->owner, (size_t)G * 4));
         CUDA_TRY(h, cudaMalloc(&h->tileFlag, (size_t)G * 4));
-        const size_t nItem = (size_t)segCount(h->nx) * h->nBY;
-        CUDA_TRY(h, cudaMalloc(&h->items, nItem * 4));
-        CUDA_TRY(h, cudaMalloc(&h->itemStamp, nItem * 4));
-        CUDA_TRY(h, cudaMemset(h->itemStamp, 0, nItem * 4));
         h->flowOk = true;
         for (const void* fn : {(const void*)k_flow<>, (const void*)k_flow<FIX_RAIN>,
                                (const void*)k_flow<FIX_RAIN_INFIL>, (const void*)k_flow<FIX_INFIL_SRC>,
@@ -1844,9 +1844,13 @@ struct rift_ensemble {
     int64_t soloCells = 0;          // members with at least this many interior cells run on their own
     long long launches = 0;         // ensemble kernels launched (members run on their own count theirs)
     cudaStream_t stream = nullptr;
-    Params* dP = nullptr;
-    CUtensorMap* dMaps = nullptr;
+    // one run's transfers: every member's tensor maps, parameters and device
+    // state, one pinned block and its device copy
+    EnsMember* hM = nullptr;
+    EnsMember* dM = nullptr;
     EnsDev* dE = nullptr;
+    EnsTimes* hT = nullptr;  // pinned: the members' end times
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int grid = 0;
     long long steps = 0;
     std::string err;
@@ -1890,13 +1894,17 @@ int rift_ensemble_create(rift_handle* const* members, int32_t n, rift_ensemble**
     int coop = 0, sms = 0, occ = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, members[0]->g.device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, members[0]->g.device);
-    ENS_TRY(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ensemble, NT, 0));
+    ENS_TRY(e, cudaFuncSetAttribute(k_ensemble, cudaFuncAttributeMaxDynamicSharedMemorySize, ENS_SMEM));
+    ENS_TRY(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ensemble, ENS_T, ENS_SMEM));
     if (!coop || occ < 1) return efail(e, RIFT_ERR_UNSUPPORTED, "no cooperative launch");
-    e->grid = sms * occ;
+    e->grid = sms;  // one CTA per SM
     ENS_TRY(e, cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
-    ENS_TRY(e, cudaMalloc(&e->dP, sizeof(Params) * n));
-    ENS_TRY(e, cudaMalloc(&e->dMaps, sizeof(CUtensorMap) * 3 * n));
+    ENS_TRY(e, cudaMalloc(&e->dM, sizeof(EnsMember) * n));
+    ENS_TRY(e, cudaMallocHost(&e->hM, sizeof(EnsMember) * n));
     ENS_TRY(e, cudaMalloc(&e->dE, sizeof(EnsDev)));
+    ENS_TRY(e, cudaMallocHost(&e->hT, sizeof(EnsTimes)));
+    ENS_TRY(e, cudaEventCreate(&e->ev0));
+    ENS_TRY(e, cudaEventCreate(&e->ev1));
     return RIFT_OK;
 }
 
@@ -1904,8 +1912,6 @@ int rift_ensemble_run(rift_ensemble* e, double t_stop, int32_t max_steps, double
                       int32_t* steps_out) {
     if (!e || max_steps < 0) return RIFT_ERR_ARG;
     const int n = (int)e->m.size();
-    std::vector<Params> P(n);
-    std::vector<CUtensorMap> maps(3 * (size_t)n);
     std::vector<int> live(n, 0);
     int nAlive = 0;
     for (int k = 0; k < n; k++) {
@@ -1914,44 +1920,46 @@ int rift_ensemble_run(rift_ensemble* e, double t_stop, int32_t max_steps, double
         // every entry point leaves the pinned mirror equal to the device state
         h->hst->t_stop = t_stop;
         h->hst->steps_done = 0;
-        ENS_TRY(e, cudaMemcpyAsync(h->st, h->hst, sizeof(DevState), cudaMemcpyHostToDevice, e->stream));
-        P[k] = makeParams(h);
-        maps[3 * k] = h->tmA;
-        maps[3 * k + 1] = h->tmB;
-        maps[3 * k + 2] = h->tmE;
+        EnsMember& M = e->hM[k];
+        M.maps[0] = h->tmAm;
+        M.maps[1] = h->tmBm;
+        M.maps[2] = h->tmEm;
+        M.P = makeParams(h);
+        M.st = *h->hst;
         live[k] = (h->hst->t < t_stop && max_steps > 0 && !isSolo(e, h)) ? 1 : 0;
+        M.live = live[k];
         nAlive += live[k];
     }
-    ENS_TRY(e, cudaMemcpyAsync(e->dP, P.data(), sizeof(Params) * n, cudaMemcpyHostToDevice, e->stream));
-    ENS_TRY(e, cudaMemcpyAsync(e->dMaps, maps.data(), sizeof(CUtensorMap) * 3 * n,
-                               cudaMemcpyHostToDevice, e->stream));
+    cudaEvent_t ev0 = e->ev0, ev1 = e->ev1;
     ENS_TRY(e, cudaMemsetAsync(e->dE, 0, sizeof(EnsDev), e->stream));
-    ENS_TRY(e, cudaMemcpyAsync(e->dE->live[0], live.data(), sizeof(int) * n, cudaMemcpyHostToDevice,
-                               e->stream));
-    ENS_TRY(e, cudaMemcpyAsync(&e->dE->nAlive[0], &nAlive, sizeof(int), cudaMemcpyHostToDevice,
-                               e->stream));
-    EnsArgs A{e->dP, e->dMaps, e->dE, n, max_steps};
+    ENS_TRY(e, cudaMemcpyAsync(e->dM, e->hM, sizeof(EnsMember) * n, cudaMemcpyHostToDevice, e->stream));
+    k_ens_begin<<<n, 128, 0, e->stream>>>(e->dM, e->dE);
+    EnsArgs A{e->dM, e->dE, n, max_steps};
     void* args[] = {(void*)&A};
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    ENS_TRY(e, cudaEventCreate(&ev0));
-    ENS_TRY(e, cudaEventCreate(&ev1));
     ENS_TRY(e, cudaEventRecord(ev0, e->stream));
     if (nAlive > 0) {
-        ENS_TRY(e, cudaLaunchCooperativeKernel((const void*)k_ensemble, dim3(e->grid), dim3(NT), args, 0,
-                                               e->stream));
+        ENS_TRY(e, cudaLaunchCooperativeKernel((const void*)k_ensemble, dim3(e->grid), dim3(ENS_T), args,
+                                               ENS_SMEM, e->stream));
         e->launches += 1;
     }
     ENS_TRY(e, cudaEventRecord(ev1, e->stream));
+    k_ens_end<<<n, 128, 0, e->stream>>>(e->dM);
+    ENS_TRY(e, cudaGetLastError());
+    ENS_TRY(e, cudaMemcpyAsync(e->hM, e->dM, sizeof(EnsMember) * n, cudaMemcpyDeviceToHost, e->stream));
+    ENS_TRY(e, cudaMemcpyAsync(e->hT, &e->dE->times, sizeof(EnsTimes), cudaMemcpyDeviceToHost, e->stream));
     ENS_TRY(e, cudaStreamSynchronize(e->stream));
-    {  // each member's completion on the device clock
-        std::vector<unsigned long long> done(n, 0ull);
-        unsigned long long t0 = 0ull;
-        ENS_TRY(e, cudaMemcpy(done.data(), e->dE->tDone, sizeof(unsigned long long) * n,
-                              cudaMemcpyDeviceToHost));
-        ENS_TRY(e, cudaMemcpy(&t0, &e->dE->t0, sizeof(t0), cudaMemcpyDeviceToHost));
-        e->memberSec.assign(n, 0.0);
-        for (int k = 0; k < n; k++)
-            if (live[k] && done[k] >= t0) e->memberSec[k] = 1e-9 * (double)(done[k] - t0);
+    int rc = RIFT_OK;
+    e->memberSec.assign(n, 0.0);
+    for (int k = 0; k < n; k++) {
+        rift_handle* h = e->m[k];
+        *h->hst = e->hM[k].st;
+        if (h->hst->error && !rc) {
+            rc = fail(h, RIFT_ERR_CUDA, deviceErrorText(h->hst->error));
+            e->err = "member " + std::to_string(k) + ": " + h->err;
+        }
+        // each member's completion on the device clock
+        if (live[k] && e->hT->tDone[k] >= e->hT->t0)
+            e->memberSec[k] = 1e-9 * (double)(e->hT->tDone[k] - e->hT->t0);
     }
     // The large members, one after another on their own per-step graphs (the
     // column march on dense grids), smallest first; each one's completion is
@@ -1972,11 +1980,7 @@ int rift_ensemble_run(rift_ensemble* e, double t_stop, int32_t max_steps, double
             int32_t dk = 0;
             ENS_TRY(e, cudaEventRecord(ev0, h->stream));
             int r = rift_run(h, max_steps, t_stop, &tk, &dtk, &dk);
-            if (r) {
-                cudaEventDestroy(ev0);
-                cudaEventDestroy(ev1);
-                return efail(e, r, "member " + std::to_string(k) + ": " + h->err);
-            }
+            if (r) return efail(e, r, "member " + std::to_string(k) + ": " + h->err);
             ENS_TRY(e, cudaEventRecord(ev1, h->stream));
             ENS_TRY(e, cudaEventSynchronize(ev1));
             float ms = 0.f;
@@ -1985,16 +1989,8 @@ int rift_ensemble_run(rift_ensemble* e, double t_stop, int32_t max_steps, double
             e->memberSec[k] = dk > 0 ? offset : 0.0;
         }
     }
-    cudaEventDestroy(ev0);
-    cudaEventDestroy(ev1);
-    int rc = RIFT_OK;
     for (int k = 0; k < n; k++) {
         rift_handle* h = e->m[k];
-        int r = pullState(h);
-        if (r && !rc) {
-            rc = r;
-            e->err = "member " + std::to_string(k) + ": " + h->err;
-        }
         if (t_out) t_out[k] = h->hst->t;
         if (steps_out) steps_out[k] = h->hst->steps_done;
         e->steps += h->hst->steps_done;
@@ -2028,9 +2024,12 @@ const char* rift_ensemble_last_error(rift_ensemble* e) { return e ? e->err.c_str
 void rift_ensemble_destroy(rift_ensemble* e) {
     if (!e) return;
     if (e->stream) cudaStreamSynchronize(e->stream);
-    if (e->dP) cudaFree(e->dP);
-    if (e->dMaps) cudaFree(e->dMaps);
+    if (e->dM) cudaFree(e->dM);
+    if (e->hM) cudaFreeHost(e->hM);
     if (e->dE) cudaFree(e->dE);
+    if (e->hT) cudaFreeHost(e->hT);
+    if (e->ev0) cudaEventDestroy(e->ev0);
+    if (e->ev1) cudaEventDestroy(e->ev1);
     if (e->stream) cudaStreamDestroy(e->stream);
     delete e;
 }

@@ -39,10 +39,10 @@ constexpr int FLOW_T = FLOW_WARPS * 32;
 constexpr uint32_t FLOW_SMEM = FLOW_WARPS * sizeof(MarchRing);
 
 // The rest of Integrate_1_k (grid.cu:856-922) on rows [j0, j1) of segment seg,
-// once dt is known: U* and F* from U^n and the stored divergence; clears the
-// tiles for stage 2.  One warp, the lanes and columns of marchRows; two rows
-// of loads in flight.
-template <uint32_t FIX, class On>
+// once dt is known: U* and F* from U^n and the stored divergence.  CLEAR: see
+// clearTile.  Euler mode: the tiles' wet flags (cleared before).  One warp, the
+// lanes and columns of marchRows; two rows of loads in flight.
+template <uint32_t FIX, bool CLEAR, class On>
 __device__ __forceinline__ void updateRows(const Params& P, const StageConsts& C, int seg, int j0,
                                            int j1, On on, bool led, Led& L) {
     constexpr bool RAINPRE = (FIX & F_RAIN_G) != 0;
@@ -55,6 +55,7 @@ __device__ __forceinline__ void updateRows(const Params& P, const StageConsts& C
     const unsigned pitch = (unsigned)P.pitch;
     const size_t pl = (size_t)P.planeSize;
     const bool edge = seg == 0 || MSEG * (seg + 1) + 1 >= P.nx - 3;
+    const bool euler = FIX ? (FIX & F_EULER) != 0 : C.euler;
     struct In {
         P2 a[3], d[3], n, x[2];
     };
@@ -76,6 +77,7 @@ __device__ __forceinline__ void updateRows(const Params& P, const StageConsts& C
     };
     auto cells = [&](const In& r, int tile, int j) {
         const unsigned c = (unsigned)j * pitch + (unsigned)i;
+        bool wet = false;
         float u[2][3];
 #pragma unroll
         for (int k = 0; k < 2; k++) {
@@ -85,8 +87,8 @@ __device__ __forceinline__ void updateRows(const Params& P, const StageConsts& C
             const CellSrc s = cellSources<1, INFPRE, false, FIX, RAINPRE>(
                 P, C, tile, j, i + k, at(r.d[0]), at(r.d[1]), at(r.d[2]), at(r.a[0]), at(r.a[1]),
                 at(r.a[2]), 0.f, 0.f, 0.f, 0.f, pk);
-            cellResult<1, INFPRE, FIX>(P, C, j, i + k, s, at(r.a[0]), at(r.a[1]), at(r.a[2]), pk,
-                                       led ? &L : nullptr, u[k][0], u[k][1], u[k][2]);
+            wet |= cellResult<1, INFPRE, FIX>(P, C, j, i + k, s, at(r.a[0]), at(r.a[1]), at(r.a[2]), pk,
+                                              led ? &L : nullptr, u[k][0], u[k][1], u[k][2]);
         }
 #pragma unroll
         for (int q = 0; q < 3; q++) {
@@ -99,6 +101,7 @@ __device__ __forceinline__ void updateRows(const Params& P, const StageConsts& C
             writeGhostRows(P, P.B, j, i, u[0][0], u[0][1], u[0][2]);
             if (inY) writeGhostRows(P, P.B, j, i + 1, u[1][0], u[1][1], u[1][2]);
         }
+        return wet;
     };
     const unsigned group = __match_any_sync(FULL, bx);
     const bool leader = inX && lane == __ffs(group) - 1;
@@ -106,8 +109,8 @@ __device__ __forceinline__ void updateRows(const Params& P, const StageConsts& C
     for (int j = j0; j < j1; j += 2) {
         const int by = (j - 2) / TH, by2 = (j - 1) / TH;
         const bool a0 = on(by, bx), a1 = j + 1 < j1 && (by2 == by ? a0 : on(by2, bx));
-        if (leader && a0 && by != byOld) clearTile(P, by * P.nBX + bx);
-        if (leader && a1 && by2 != by) clearTile(P, by2 * P.nBX + bx);
+        if (CLEAR && leader && a0 && by != byOld) clearTile(P, by * P.nBX + bx, euler);
+        if (CLEAR && leader && a1 && by2 != by) clearTile(P, by2 * P.nBX + bx, euler);
         const int src0 = a0 ? sourceTile(P, by * P.nBX + bx) : -1;
         const int src1 = a1 ? (by2 == by ? src0 : sourceTile(P, by2 * P.nBX + bx)) : -1;
         byOld = a1 ? by2 : by;
@@ -117,8 +120,15 @@ __device__ __forceinline__ void updateRows(const Params& P, const StageConsts& C
         if (FIX == 0 && a1) prefetchMaps(P, C.fl, c + pitch);
         if (a0) load(r0, c);
         if (a1) load(r1, c + pitch);
-        if (a0) cells(r0, src0, j);
-        if (a1) cells(r1, src1, j + 1);
+        const bool w0 = a0 && cells(r0, src0, j);
+        const bool w1 = a1 && cells(r1, src1, j + 1);
+        if (euler) {
+            const bool any0 = __reduce_or_sync(group, w0 ? 1u : 0u) != 0u;
+            const bool any1 = __reduce_or_sync(group, w1 ? 1u : 0u) != 0u;
+            const bool keep = !(cellFlags<FIX>(C.fl) & F_TILE_ACC);
+            if (leader && a0 && (any0 || keep)) P.wet[by * P.nBX + bx] = 1;
+            if (leader && a1 && (any1 || keep)) P.wet[by2 * P.nBX + bx] = 1;
+        }
     }
     if (edge) ghostColumns(P, P.B, seg, j0, j1, on);
 }
@@ -295,7 +305,7 @@ __global__ void __launch_bounds__(FLOW_T, 1) k_flow(const __grid_constant__ CUte
         dtPrev = sDt;
         L.v[LED_BOUND] += C1.wRate * L1.v[LED_BOUND];
         items([&](int seg, int j0, int j1) {
-            updateRows<FIX>(P, C1, seg, j0, j1, on, led, L);
+            updateRows<FIX, true>(P, C1, seg, j0, j1, on, led, L);
             return true;
         });
         FLOW_SYNC();

@@ -98,6 +98,17 @@ __device__ __forceinline__ GrowItem growItem(const Params& P, int base, int s1) 
     return t;
 }
 
+// The (60-column segment, tile row) pairs of scheduled tile b into P.items: the
+// first tile to set a pair's stamp appends it; the caller clears the listed
+// pairs' stamps after its barrier.
+__device__ __forceinline__ void listItems(const Params& P, int b, int* itemCnt) {
+    const int nSeg = segCount(P.nx), bx = b % P.nBX, by = b / P.nBX;
+    const int s1 = min(TW * bx + TW - 1, P.nx - 5) / SEG;
+    for (int s = TW * bx / SEG; s <= s1; s++)
+        if (atomicExch(&P.itemStamp[by * nSeg + s], 1) == 0)
+            P.items[atomicAdd(itemCnt, 1)] = by * nSeg + s;
+}
+
 // One pass: each CTA's chunk of strips appends its entries to the four lists
 // with one atomic per warp and list (the lists are sets: their order changes
 // no result), writes the new active flags, folds the stale speeds of the
@@ -106,9 +117,7 @@ __device__ __forceinline__ GrowItem growItem(const Params& P, int base, int s1) 
 // publishes the list sizes and clears the counters for the next step;
 // without, the caller reads the counters after a grid barrier and publishes
 // them later (publishGrow).
-// With ITEMS the (60-column segment, tile row) pairs that hold a scheduled tile
-// are listed too (P.items, *itemCnt): the first tile to set a pair's stamp
-// appends it; the caller clears the listed pairs' stamps after its barrier.
+// With ITEMS the scheduled tiles' pairs are listed too (listItems).
 template <bool PUBLISH = true, bool ITEMS = false>
 __device__ void growAppend(const Params& P, unsigned* staleDst = nullptr, int* itemCnt = nullptr) {
     DevState* s = P.st;
@@ -133,13 +142,7 @@ __device__ void growAppend(const Params& P, unsigned* staleDst = nullptr, int* i
             if (t.f[q]) lists[q][bq + __popc(bal[q] & below)] = q == 3 ? t.strip : t.b;
         }
         if (t.f[0]) cells += (unsigned long long)t.cells;
-        if (ITEMS && t.f[0]) {
-            const int nSeg = segCount(P.nx), bx = t.b % P.nBX, by = t.b / P.nBX;
-            const int s1 = min(TW * bx + TW - 1, P.nx - 5) / SEG;
-            for (int s = TW * bx / SEG; s <= s1; s++)
-                if (atomicExch(&P.itemStamp[by * nSeg + s], 1) == 0)
-                    P.items[atomicAdd(itemCnt, 1)] = by * nSeg + s;
-        }
+        if (ITEMS && t.f[0]) listItems(P, t.b, itemCnt);
         if (t.b >= 0) {
             if (t.v) {  // the march folds an active tile's speeds into a cleared entry
                 P.mx[t.b] = 0.f;

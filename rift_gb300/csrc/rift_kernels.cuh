@@ -623,17 +623,20 @@ __device__ __forceinline__ float seriesInterp(const float* T, const float* R, in
 
 // Start of a step, part 1, by one thread: reset of the step's reductions and
 // the map factors that follow t.  Runs before the step's grow.
-__device__ __forceinline__ void beginStepResets(DevState* s) {
+__device__ __forceinline__ void beginStepCounts(DevState* s) {
     s->stop = 0;
     s->steps_done += 1;
-    s->max_bits[0] = 0u;
-    s->max_bits[1] = 0u;
     s->ticket = 0u;
     // map factor following t (GridSeries::update computes it at the end
     // of the previous step from the same t, GridSeries.cu:398)
     for (int w = 0; w < 3; w++)
         if (s->map_timed[w])
             s->factor[w] = (float)((s->t - s->map_t0[w]) / (s->map_t1[w] - s->map_t0[w]));
+}
+__device__ __forceinline__ void beginStepResets(DevState* s) {
+    beginStepCounts(s);
+    s->max_bits[0] = 0u;
+    s->max_bits[1] = 0u;
 }
 
 // The step's uniform source rates at float(t) from the series state (one
@@ -991,14 +994,6 @@ __device__ __forceinline__ StageConsts stageConstsAt(const Params& P, double dtN
 // pre: the cell's own inputs loaded ahead of use -- stage 1: Manning n;
 // stage 2: U^n (h, hu, hv); with PREF also pre[3] = F entering the stage,
 // pre[4] = K, pre[5] = F^n (stage 2), else those are read here.
-// Bed-slope source of the momentum equations (grid.cu:701,751-752).
-__device__ __forceinline__ float bedSourceX(const Params& P, float hC, float eW, float eE) {
-    return -kG * hC * ((eE - eW) * P.inv_dx);
-}
-__device__ __forceinline__ float bedSourceY(const Params& P, float hC, float eS, float eN) {
-    return -kG * hC * ((eN - eS) * P.inv_dy);
-}
-
 // The per-cell update is split at dt: cellSources is everything that does
 // not need the step's dt (for stage 1: the bed slope, the mass sources with
 // their clamps at the previous dt, infiltration, Manning's G), cellFinish the
@@ -1029,8 +1024,6 @@ __device__ __forceinline__ CellSrc cellSources(const Params& P, const StageConst
                                                float eS, float eN, const float* pre) {
     const uint32_t fl = cellFlags<FIX>(C.fl);
     const size_t c = cidx(P, 0, j, i);
-    const float S1 = BED ? bedSourceX(P, hC, eW, eE) : 0.f;
-    const float S2 = BED ? bedSourceY(P, hC, eS, eN) : 0.f;
     // mass sources, grid.cu:763-807
     float S0 = 0.f;
     if (fl & F_RAIN_U) S0 += C.rainU;
@@ -1071,8 +1064,8 @@ __device__ __forceinline__ CellSrc cellSources(const Params& P, const StageConst
     }
     dh += S0;
     if (BED) {
-        dhu += S1;
-        dhv += S2;
+        dhu = addBed(dhu, hC, eW, eE, P.inv_dx);
+        dhv = addBed(dhv, hC, eS, eN, P.inv_dy);
     }
     CellSrc r;
     r.dh = dh;
@@ -1294,12 +1287,13 @@ __device__ __forceinline__ void tileFluxDiv(StageSmem& S, const TileBuf& T, cons
     const int tx = tid % TW, ty = tid / TW;
     dh = dhu = dhv = 0.f;
     if (tid < TH * TW) {
-        dh = -(S.FX[0][ty][tx + 1] - S.FX[0][ty][tx]) * P.inv_dx;
-        dhu = -(S.FX[1][ty][tx + 1] - S.FX[1][ty][tx]) * P.inv_dx;
-        dhv = -(S.FX[2][ty][tx + 1] - S.FX[2][ty][tx]) * P.inv_dx;
-        dh += -(S.FY[0][ty + 1][tx] - S.FY[0][ty][tx]) * P.inv_dy;
-        dhu += -(S.FY[1][ty + 1][tx] - S.FY[1][ty][tx]) * P.inv_dy;
-        dhv += -(S.FY[2][ty + 1][tx] - S.FY[2][ty][tx]) * P.inv_dy;
+        auto div = [&](int q) {
+            return divergence(vsub(S.FX[q][ty][tx + 1], S.FX[q][ty][tx]),
+                              vsub(S.FY[q][ty + 1][tx], S.FY[q][ty][tx]), P.inv_dx, P.inv_dy);
+        };
+        dh = div(0);
+        dhu = div(1);
+        dhv = div(2);
     }
     if (bin) {
         *bin = 0.f;

@@ -35,7 +35,6 @@
 // busy, DRAM moves at 4.6 and 5.0 TB/s.  A lone warp needs 0.56 us per row.
 #pragma once
 #include "rift_grow.cuh"
-#include "rift_pair.cuh"
 
 namespace rift {
 
@@ -87,12 +86,12 @@ struct Diff2 {  // differences of surface and momenta across the faces of two co
 };
 // from row a to the row b above it (their staged rows ra, rb)
 __device__ __forceinline__ Diff2 diffY(const Cell2& a, const float* ra, const Cell2& b, const float* rb) {
-    return Diff2{add2(sub2(row2(ra, 6), row2(rb, 5)), sub2(b.h, a.h)), sub2(b.u, a.u), sub2(b.v, a.v)};
+    return Diff2{vadd(vsub(row2(ra, 6), row2(rb, 5)), vsub(b.h, a.h)), vsub(b.u, a.u), vsub(b.v, a.v)};
 }
 __device__ __forceinline__ void constructY2(const Cell2& c, const float* r, const Diff2& dP,
-                                            const Diff2& dM, Face2& P, Face2& M) {
-    construct2(c.h, c.u, c.v, limit2(dP.w, dM.w), limit2(dP.u, dM.u), limit2(dP.v, dM.v), row2(r, 5),
-               row2(r, 6), P, M);
+                                            const Diff2& dM, Face<P2>& P, Face<P2>& M) {
+    construct(c.h, c.u, c.v, limited(dP.w, dM.w), limited(dP.u, dM.u), limited(dP.v, dM.v), row2(r, 5),
+              row2(r, 6), P, M);
 }
 // x reconstruction of a row and the fluxes through the east faces of both
 // columns; fx: the difference of each column's east and west fluxes, fW0, fE0
@@ -104,22 +103,22 @@ __device__ __forceinline__ void rowFluxX(const Cell2& c, P2 eW, P2 eE, float kap
     auto up = [](float a) { return __shfl_up_sync(FULL, a, 1); };
     // limited differences of both columns from d0 (across the face between
     // them) and d1 (across the east face of the second)
-    auto limit = [&](float d0, float d1) { return pack2(limit1(d0, up(d1)), limit1(d1, d0)); };
-    const P2 tw = limit((lo(eE) - hi(eW)) + (hi(c.h) - lo(c.h)),
-                        (hi(eE) - down(lo(eW))) + (down(lo(c.h)) - hi(c.h)));
-    const P2 tu = limit(hi(c.u) - lo(c.u), down(lo(c.u)) - hi(c.u));
-    const P2 tv = limit(hi(c.v) - lo(c.v), down(lo(c.v)) - hi(c.v));
-    Face2 Pf, Mf;
-    construct2(c.h, c.u, c.v, tw, tu, tv, eW, eE, Pf, Mf);
+    auto limit = [&](float d0, float d1) { return pack2(limited(d0, up(d1)), limited(d1, d0)); };
+    const P2 tw = limit(vadd(vsub(lo(eE), hi(eW)), vsub(hi(c.h), lo(c.h))),
+                        vadd(vsub(hi(eE), down(lo(eW))), vsub(down(lo(c.h)), hi(c.h))));
+    const P2 tu = limit(vsub(hi(c.u), lo(c.u)), vsub(down(lo(c.u)), hi(c.u)));
+    const P2 tv = limit(vsub(hi(c.v), lo(c.v)), vsub(down(lo(c.v)), hi(c.v)));
+    Face<P2> Pf, Mf;
+    construct(c.h, c.u, c.v, tw, tu, tv, eW, eE, Pf, Mf);
     auto east = [&](P2 a) { return pack2(hi(a), down(lo(a))); };
-    const Face2 R{east(Mf.h), east(Mf.u), east(Mf.v)};
+    const Face<P2> R{east(Mf.h), east(Mf.u), east(Mf.v)};
     P2 f[3];
-    faceFlux2<0>(Pf, R, kappa, f, spd);
+    spd = faceFlux<0>(Pf, R, kappa, f);
     float w[3];
 #pragma unroll
     for (int q = 0; q < 3; q++) {
         w[q] = up(hi(f[q]));
-        fx[q] = pack2(lo(f[q]) - w[q], hi(f[q]) - lo(f[q]));
+        fx[q] = pack2(vsub(lo(f[q]), w[q]), vsub(hi(f[q]), lo(f[q])));
     }
     fW0 = pack2(w[0], lo(f[0]));
     fE0 = f[0];
@@ -162,9 +161,11 @@ __device__ __forceinline__ void ghostColumns(const Params& P, float* U, int seg,
 
 // Stage 2 (RK2) folds an active tile's wet flag and speeds into cleared
 // entries: cleared between the grow and stage 2, by every item that holds
-// rows of the tile.
-__device__ __forceinline__ void clearTile(const Params& P, int tile) {
+// rows of the tile.  (Euler: the speeds are stage 1's, into entries the grow
+// cleared.)
+__device__ __forceinline__ void clearTile(const Params& P, int tile, bool euler) {
     P.wet[tile] = 0;
+    if (euler) return;
     P.mx[tile] = 0.f;
     P.my[tile] = 0.f;
 }
@@ -197,7 +198,6 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
     const size_t pl = (size_t)P.planeSize;
     const uint32_t fl = cellFlags<FIX>(C.fl);
     const bool euler = FIX ? (FIX & F_EULER) != 0 : C.euler;
-    const P2 nidx = both(-P.inv_dx), nidy = both(-P.inv_dy), idx = both(P.inv_dx), idy = both(P.inv_dy);
 
     // the line of plane lane / 4 this lane prefetches (3 lines hold the 64 columns)
     const float* pfB = nullptr;
@@ -236,7 +236,7 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
     const float* rn = rc + MBOX;
     const float* rl = &S.slot[2].s[0][0][2 * lane];
     Cell2 cur = loadCell2(rc), nxt = loadCell2(rn);
-    Face2 yP;      // the row's reconstruction at its north face
+    Face<P2> yP;      // the row's reconstruction at its north face
     P2 fS[3];      // flux through its south face
     Diff2 dN;      // differences to the row above
     {
@@ -245,11 +245,10 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
         const Cell2 m2 = loadCell2(r0), m1 = loadCell2(r1);
         const Diff2 d0 = diffY(m2, r0, m1, r1), d1 = diffY(m1, r1, cur, rc);
         dN = diffY(cur, rc, nxt, rn);
-        Face2 a, b, M;
+        Face<P2> a, b, M;
         constructY2(m1, r1, d1, d0, a, b);
         constructY2(cur, rc, dN, d1, yP, M);
-        P2 s;
-        faceFlux2<1>(a, M, kappa, fS, s);
+        faceFlux<1>(a, M, kappa, fS);
     }
     // the row's centre values (stage 2: U^n; rain maps or F, K, F^n when the
     // instantiation reads them ahead)
@@ -277,7 +276,7 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
     int src = STAGE == 2 && act ? sourceTile(P, by * P.nBX + bx) : -1;
     float ax = 0.f, ay = 0.f;
     bool wet = false;
-    if (CLEAR && !euler && leader && act) clearTile(P, by * P.nBX + bx);
+    if (CLEAR && leader && act) clearTile(P, by * P.nBX + bx, euler);
     constexpr int UNROLL = STAGE == 1 ? 2 : 1;
 #pragma unroll UNROLL
     for (int j = j0; j < j1; j++) {
@@ -300,20 +299,19 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
         // y: reconstruction of row j + 1, flux through the north face of row j
         const Cell2 ld = loadCell2(rl);
         const Diff2 dNN = diffY(nxt, rn, ld, rl);
-        Face2 yn, yM;
+        Face<P2> yn, yM;
         constructY2(nxt, rn, dNN, dN, yn, yM);
-        faceFlux2<1>(yP, yM, kappa, fN, sy);
+        sy = faceFlux<1>(yP, yM, kappa, fN);
         // divergence, with the bed-slope source in the momenta
         P2 d[3];
 #pragma unroll
         for (int q = 0; q < 3; q++)
-            d[q] = fma2(fx[q], nidx, mul2(sub2(fN[q], fS[q]), nidy));
-        const P2 gh = mul2(both(-kG), cur.h);
-        d[1] = fma2(gh, mul2(sub2(eE, eW), idx), d[1]);
-        d[2] = fma2(gh, mul2(sub2(row2(rc, 6), row2(rc, 5)), idy), d[2]);
+            d[q] = divergence(fx[q], vsub(fN[q], fS[q]), P.inv_dx, P.inv_dy);
+        d[1] = addBed(d[1], cur.h, eW, eE, P.inv_dx);
+        d[2] = addBed(d[2], cur.h, row2(rc, 5), row2(rc, 6), P.inv_dy);
         if (act) {
-            ax = max3(ax, lo(sx), inY ? hi(sx) : 0.f);
-            ay = max3(ay, lo(sy), inY ? hi(sy) : 0.f);
+            ax = fmaxf(fmaxf(ax, lo(sx)), inY ? hi(sx) : 0.f);
+            ay = fmaxf(fmaxf(ay, lo(sy)), inY ? hi(sy) : 0.f);
             const unsigned c = (unsigned)j * pitch + (unsigned)i;
             if (led && edge) {
                 float r = edgeInflow(P, j, i, lo(fW0), lo(fE0), lo(fS[0]), lo(fN[0]));
@@ -375,7 +373,7 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
                 by++;
                 act = on(by, bx);
                 src = STAGE == 2 && act ? sourceTile(P, by * P.nBX + bx) : -1;
-                if (CLEAR && !euler && leader && act) clearTile(P, by * P.nBX + bx);
+                if (CLEAR && leader && act) clearTile(P, by * P.nBX + bx, euler);
             }
         }
 #pragma unroll
