@@ -367,19 +367,33 @@ __host__ __device__ __forceinline__ int tileCount(const rift_closure_src& src) {
 //  layer 1: M = 512 rows (4 tiles of 128; the 18 x 18 region is rows
 //           m < 396 with m % 22 < 18), N = 32, K = 15 steps of 16: taps
 //           (dy, dx) and (dy+1, dx) for dy = 0, 2, 4 (dy = 5 carries zero
-//           weights), the two 8-channel K chunks 22 cells apart;
+//           weights), the two 8-channel K chunks 22 cells apart.  (Taps 2s and
+//           2s + 1 would need 13 steps, but another order of the sum rounds
+//           some activations to another BF16: 2.7e-5 off in the output.);
 //  layer 2: M = 384 rows (3 tiles; the 16 x 16 outputs are rows m < 352
 //           with m % 22 < 16), N = 32, K = 9 taps x 2 steps of 16 over the
 //           four 8-channel planes of the layer-1 activations.
-// Tensor memory: 128 columns, one 32-column accumulator per M tile (layer 2
-// reuses the columns of layer 1 once its epilogue has read them).  A CTA
-// holds 74 KB of shared memory and 80 registers per thread, so three run on
-// an SM (384 of the 512 tensor-memory columns); the epilogues read the
-// accumulators 8 columns at a time to stay within the registers.
+//
+// What bounds it: an MMA reads its 4 KB of A from shared memory whatever N is:
+// 61 cycles one after another in one CTA, 39 per SM with several CTAs (at N =
+// 32, 46 at 64), so a block's 114 take 4,400 cycles of the tensor pipe.  To
+// keep that pipe busy, one CTA per SM runs four blocks at a time, each on a
+// group of four warps and an issuing warp: the weights are staged once for the
+// four (three CTAs of 74 KB fitted before), the groups meet at no barrier, and
+// an M tile's epilogue and layer 2's MMAs start as soon as what they read is
+// there.  Tensor memory: 128 columns per
+// group, all 512; one 32-column accumulator per M tile, layer 2 reuses the
+// columns of layer 1 once its epilogue has read them.
+// 256 patches of 64 x 64 (4,096 blocks): 125 us with three CTAs per SM, tensor
+// pipe 59% busy; 89 with four groups and issuing warps, 77% busy; 78 with the
+// parameters read in their own order.
 constexpr int XBC = 640;             // BF16 input cells staged (reads reach m + 5*22 + 4 < 640)
 constexpr int A1C = 432;             // layer-1 cells kept per plane (layer 2 reads < 384 + 46)
 constexpr int M1TC = 4, M2TC = 3;    // M tiles of 128 rows
 constexpr int KS1 = 15, KS2 = 18;    // K steps of 16
+constexpr int TCG = 4;               // groups (blocks in flight) per CTA
+constexpr int GT = 128;              // threads per group
+constexpr int TCT = TCG * (GT + 32); // threads per CTA: the groups', then an issuing warp for each
 constexpr int NTAPT = 26;            // layer-1 weight blocks: the 25 taps, then one of zeros
 constexpr uint32_t TMEM_COLS = 128;
 constexpr uint32_t A1PLANE = A1C * 16;  // bytes per 8-channel plane
@@ -388,23 +402,53 @@ constexpr uint32_t A1PLANE = A1C * 16;  // bytes per 8-channel plane
 // bits 24-28
 constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((32u >> 3) << 17) | ((128u >> 4) << 24);
 
-struct __align__(128) TcSmem {
+struct __align__(128) TcGroup {  // one block in flight
     uint16_t xb[XBC * 8];        // input cells (BF16 x 8), zero past the 22 x 22 block
     uint16_t a1[4][A1C * 8];     // layer-1 activations, channels 8p..8p+7 in plane p
-    uint16_t w1t[NTAPT * 32 * 8];  // [dy*5 + dx][o][c8]; block 25 all zero
-    uint16_t w2t[36 * 32 * 8];   // [tap*4 + c/8][o][c%8]
     float xh[NRI];               // scaled FP32 depth of the input cells
     float xbed[NRI];             // scaled FP32 bed of the input cells
-    float w3[COUT][C1];
-    float b1[C1], b2[C1], b3[COUT], sbed[C1];
     float bref;
-    int red[2];
-    uint64_t bar;
+    int red;
+    int stop;                    // to the issuing warp: no more blocks
+    int next;                    // the group's next block
+    uint64_t bar[M1TC + M2TC];   // completion of each M tile's MMAs: layer 1, then layer 2
+    uint64_t in;                 // a block is staged, or `stop` set (1 arrival)
+    uint64_t act[M1TC];          // the tile's layer-1 epilogue is done (4 arrivals)
+};
+struct __align__(128) TcSmem {
+    TcGroup g[TCG];
+    uint16_t w1t[NTAPT * 32 * 8];  // [dy*5 + dx][o][c8]; block 25 all zero
+    uint16_t w2t[36 * 32 * 8];   // [tap*4 + c/8][o][c%8]
+    float w3[C1][COUT];
+    float b1[C1], b2[C1], b3[COUT], sbed[C1];
     uint32_t tmem;
 };
-static_assert(offsetof(TcSmem, a1) % 16 == 0 && offsetof(TcSmem, w1t) % 16 == 0 &&
-                  offsetof(TcSmem, w2t) % 16 == 0 && offsetof(TcSmem, bar) % 8 == 0,
+static_assert(sizeof(TcGroup) % 128 == 0 && offsetof(TcGroup, a1) % 16 == 0 &&
+                  offsetof(TcGroup, bar) % 8 == 0 && offsetof(TcSmem, w1t) % 16 == 0 &&
+                  offsetof(TcSmem, w2t) % 16 == 0 && offsetof(TcSmem, w3) % 16 == 0 &&
+                  offsetof(TcSmem, b1) % 16 == 0 && offsetof(TcSmem, sbed) % 16 == 0,
               "operand alignment");
+static_assert(sizeof(TcSmem) <= 227 * 1024, "shared memory of one CTA");
+
+// Group of this thread (of the group itself, or of its issuing warp).
+__device__ __forceinline__ int tcGroupOf() {
+    const int t = threadIdx.x;
+    return t < TCG * GT ? t / GT : (t - TCG * GT) / 32;
+}
+// Barrier of one group's threads (barrier 0 is the CTA's).
+__device__ __forceinline__ void groupSync(int g) {
+    asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(GT) : "memory");
+}
+__device__ __forceinline__ bool groupAnd(int g, bool p) {
+    uint32_t r;
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.and.pred q, %2, %3, p;\n"
+        " selp.u32 %0, 1, 0, q;\n}\n"
+        : "=r"(r)
+        : "r"((uint32_t)p), "r"(g + 1), "n"(GT)
+        : "memory");
+    return r != 0;
+}
 
 __device__ int g_tc_error;  // 1: a tensor-core completion wait gave up
 
@@ -431,9 +475,12 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
 __device__ __forceinline__ void tc_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void bar_init(uint64_t* bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(bar)) : "memory");
+__device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count = 1) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(bar)), "r"(count) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(bar)) : "memory");
 }
 // Bounded wait on an mbarrier phase: false after the spin limit.
 __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity) {
@@ -467,53 +514,73 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, float v[32]) {
     for (int k = 0; k < 32; k++) v[k] = __uint_as_float(r[k]);
 }
 
-// 8 consecutive FP32 columns of this thread's tensor-memory lane.
-__device__ __forceinline__ void tc_ld8(uint32_t taddr, float v[8]) {
-    uint32_t r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                   "=r"(r[7])
-                 : "r"(taddr)
-                 : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int k = 0; k < 8; k++) v[k] = __uint_as_float(r[k]);
-}
-
 // Weights in the operand layouts, biases, the bed-weight sums; the zero pad
-// of the input cells.  Tensor memory (warp 0) and the completion barrier.
+// of the input cells.  Tensor memory (warp 0) and the completion barriers.
+// The parameters are read in their own order, a run of independent coalesced
+// loads per thread, and scattered in shared memory: read in the order of the
+// operands, the setup was most of a one-block launch (19.8 us).
 __device__ void tcSetup(TcSmem& S, const float* __restrict__ P) {
     const int tid = threadIdx.x;
-    constexpr int MAP[CB] = {0, 1, 2, 3, 3, 4, 5, -1};
-    for (int i = tid; i < NTAPT * 32 * 8; i += NT) {
-        const int T = i / 256, o = (i / 8) % 32, c8 = i % 8, c = MAP[c8];
-        S.w1t[i] = bf(T < 25 && c >= 0 ? P[OFF_W1 + o * K1P + T * CIN + c] : 0.f);
+    constexpr int NP = RIFT_CLOSURE_NPARAM;
+    constexpr int PT = (NP + TCT - 1) / TCT;
+    float v[PT];
+#pragma unroll
+    for (int q = 0; q < PT; q++) v[q] = tid + q * TCT < NP ? __ldg(P + tid + q * TCT) : 0.f;
+    // channel 7 of every layer-1 cell and the last weight block are zero
+    for (int i = tid; i < NTAPT * 32; i += TCT) {
+        S.w1t[i * 8 + 7] = 0;
+        if (i >= 25 * 32) *reinterpret_cast<uint4*>(&S.w1t[i * 8]) = make_uint4(0u, 0u, 0u, 0u);
     }
-    for (int i = tid; i < 36 * 32 * 8; i += NT) {
-        const int blk = i / 256, o = (i / 8) % 32, c8 = i % 8;
-        S.w2t[i] = bf(P[OFF_W2 + o * K2 + (blk >> 2) * 32 + (blk & 3) * 8 + c8]);
+    for (int i = tid; i < TCG * (XBC - NRI) * 8; i += TCT)
+        S.g[i / ((XBC - NRI) * 8)].xb[NRI * 8 + i % ((XBC - NRI) * 8)] = 0;
+#pragma unroll
+    for (int q = 0; q < PT; q++) {
+        const int i = tid + q * TCT;
+        if (i < OFF_B1) {
+            const int o = i / K1P, k = i % K1P, tap = k / CIN, c = k % CIN;
+            if (k < K1) {  // both halves of the bed (channels 3, 4) take its weight
+                uint16_t* w = &S.w1t[(tap * 32 + o) * 8];
+                w[c < 4 ? c : c + 1] = bf(v[q]);
+                if (c == 3) w[4] = bf(v[q]);
+            }
+        } else if (i < OFF_W2) {
+            S.b1[i - OFF_B1] = v[q];
+        } else if (i < OFF_B2) {
+            const int o = (i - OFF_W2) / K2, k = (i - OFF_W2) % K2, tap = k / C1, c = k % C1;
+            S.w2t[((tap * 4 + c / 8) * 32 + o) * 8 + c % 8] = bf(v[q]);
+        } else if (i < OFF_W3) {
+            S.b2[i - OFF_B2] = v[q];
+        } else if (i < OFF_W3 + COUT * C1) {
+            S.w3[(i - OFF_W3) % C1][(i - OFF_W3) / C1] = v[q];
+        } else if (i >= OFF_B3 && i < OFF_B3 + COUT) {
+            S.b3[i - OFF_B3] = v[q];
+        }
     }
-    for (int i = tid; i < COUT * C1; i += NT) S.w3[i / C1][i % C1] = P[OFF_W3 + i];
-    for (int i = tid; i < (XBC - NRI) * 8; i += NT) S.xb[NRI * 8 + i] = 0;
-    if (tid < C1) {
-        S.b1[tid] = P[OFF_B1 + tid];
-        S.b2[tid] = P[OFF_B2 + tid];
-        float sb = 0.f;
-        for (int tap = 0; tap < 25; tap++) sb += fb(bf(P[OFF_W1 + tid * K1P + tap * CIN + 3]));
-        S.sbed[tid] = sb;
+    if (tid < TCG) {
+        TcGroup& G = S.g[tid];
+        for (int k = 0; k < M1TC + M2TC; k++) bar_init(&G.bar[k]);
+        for (int k = 0; k < M1TC; k++) bar_init(&G.act[k], GT / 32);
+        bar_init(&G.in);
+        G.stop = 0;
     }
-    if (tid < COUT) S.b3[tid] = P[OFF_B3 + tid];
-    if (tid == 0) bar_init(&S.bar);
     if (tid < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          saddr(&S.tmem)),
-                     "r"(TMEM_COLS)
+                     "r"(TCG * TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    proxy_fence();  // the weights are read by the tensor cores
     tc_before_sync();
     __syncthreads();
     tc_after_sync();
+    if (tid >= TCG * GT && tid < TCG * GT + C1) {
+        const int o = tid - TCG * GT;
+        float sb = 0.f;
+        for (int tap = 0; tap < 25; tap++) sb += fb(S.w1t[(tap * 32 + o) * 8 + 3]);
+        S.sbed[o] = sb;
+    }
+    __syncthreads();
 }
 
 __device__ void tcTeardown(TcSmem& S) {
@@ -522,18 +589,20 @@ __device__ void tcTeardown(TcSmem& S) {
     tc_after_sync();
     if (threadIdx.x < 32)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(S.tmem),
-                     "r"(TMEM_COLS)
+                     "r"(TCG * TMEM_COLS)
                      : "memory");
 }
 
-// A block's raw inputs in registers: this thread's cells i = tid and
-// tid + NT of the 22 x 22 block (484 < 2 NT), and the block's reference bed.
-// Loaded one block ahead, while the tensor cores work on the current one.
+// A block's raw inputs in registers: this thread's cells of the 22 x 22 block
+// (484 < 4 GT), and the block's reference bed.  Loaded one block ahead, while
+// the tensor cores work on the current one.
+constexpr int TCC = (NRI + GT - 1) / GT;
 struct TcInput {
-    float v[2][CIN];
+    float v[TCC][CIN];
     float bref;
 };
-__device__ void tcLoadInput(TcInput& R, const rift_closure_src& src, int s, int Y0, int X0) {
+__device__ __forceinline__ void tcLoadInput(TcInput& R, const rift_closure_src& src, int s, int Y0,
+                                            int X0) {
     const size_t sbase = (size_t)s * (size_t)src.sample_stride;
     auto at = [&](int ry, int rx) {
         int y = min(max(Y0 + ry, 0), src.H - 1), x = min(max(X0 + rx, 0), src.W - 1);
@@ -541,8 +610,8 @@ __device__ void tcLoadInput(TcInput& R, const rift_closure_src& src, int s, int 
     };
     R.bref = src.plane[3] ? __ldg(src.plane[3] + at(RI / 2, RI / 2)) : src.value[3];
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const int i = threadIdx.x + k * NT;
+    for (int k = 0; k < TCC; k++) {
+        const int i = threadIdx.x % GT + k * GT;
         if (i >= NRI) break;
         const size_t off = at(i / RI, i % RI);
 #pragma unroll
@@ -550,15 +619,15 @@ __device__ void tcLoadInput(TcInput& R, const rift_closure_src& src, int s, int 
     }
 }
 
-// The loaded block into shared memory: scaled FP32 values (xs) and the
+// The loaded block into shared memory: scaled FP32 depth and bed and the
 // BF16 cells of the layer-1 operand (the bed relative to bref in two
 // halves); each writer fences its shared stores for the async proxy.
-__device__ void tcStoreInput(TcSmem& S, const TcInput& R, const rift_closure_src& src) {
+__device__ __forceinline__ void tcStoreInput(TcGroup& S, const TcInput& R, const rift_closure_src& src) {
     const float bref = R.bref * src.scale[3];
-    if (threadIdx.x == 0) S.bref = bref;
+    if (threadIdx.x % GT == 0) S.bref = bref;
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const int i = threadIdx.x + k * NT;
+    for (int k = 0; k < TCC; k++) {
+        const int i = threadIdx.x % GT + k * GT;
         if (i >= NRI) break;
         float v[CIN];
 #pragma unroll
@@ -578,18 +647,19 @@ __device__ void tcStoreInput(TcSmem& S, const TcInput& R, const rift_closure_src
     proxy_fence();
 }
 
-// Thread 0: the MMAs of one layer, then their completion on the barrier.
-// The loops unroll completely: every operand offset is a compile-time
-// constant added to a base descriptor (its address field counts 16-byte
-// units, and no shared address reaches 256 KB, so the sum never carries out
-// of the field), so the issuing thread spends a few instructions per MMA.
-__device__ void tcIssue1(const TcSmem& S, uint32_t tmem) {
+// One thread: the MMAs of layer 1 / of M tile mt of layer 2, each
+// M tile's completion on a barrier of its own.  The loops unroll completely:
+// every operand offset is a compile-time constant added to a base descriptor
+// (its address field counts 16-byte units, and no shared address reaches 256
+// KB, so the sum never carries out of the field), so the issuing thread spends
+// a few instructions per MMA.
+__device__ __forceinline__ void tcIssue1(const TcSmem& S, TcGroup& G, uint32_t tmem) {
     tc_after_sync();
     // B: the K chunks of step s are taps (dy, dx) and (dy + 1, dx), dy = 2(s/5), five weight
     // blocks apart; for dy = 4 the second chunk is the zero block
-    const uint64_t a0 = sdesc(saddr(S.xb), RI * 16, 128), b0 = sdesc(saddr(S.w1t), 0, 128);
+    const uint64_t a0 = sdesc(saddr(G.xb), RI * 16, 128), b0 = sdesc(saddr(S.w1t), 0, 128);
 #pragma unroll
-    for (int mt = 0; mt < M1TC; mt++)
+    for (int mt = 0; mt < M1TC; mt++) {
 #pragma unroll
         for (int s = 0; s < KS1; s++) {
             const uint32_t cell = mt * 128 + (s / 5) * 2 * RI + s % 5;  // 16-byte cells
@@ -597,86 +667,133 @@ __device__ void tcIssue1(const TcSmem& S, uint32_t tmem) {
             const uint64_t lbo = (uint64_t)((T1 - T0) * 512 / 16) << 16;
             tc_mma(tmem + mt * 32, a0 + cell, b0 + T0 * (512 / 16) + lbo, s > 0);
         }
-    tc_commit(const_cast<uint64_t*>(&S.bar));
-}
-__device__ void tcIssue2(const TcSmem& S, uint32_t tmem) {
-    tc_after_sync();
-    const uint64_t a0 = sdesc(saddr(S.a1), A1PLANE, 128), b0 = sdesc(saddr(S.w2t), 512, 128);
-#pragma unroll
-    for (int mt = 0; mt < M2TC; mt++)
-#pragma unroll
-        for (int s = 0; s < KS2; s++) {
-            const int tap = s >> 1, kb = s & 1;
-            const uint32_t cell = kb * 2 * A1C + mt * 128 + (tap / 3) * RI + tap % 3;
-            tc_mma(tmem + mt * 32, a0 + cell, b0 + (tap * 4 + 2 * kb) * (512 / 16), s > 0);
-        }
-    tc_commit(const_cast<uint64_t*>(&S.bar));
-}
-
-// Wait for the layer's MMAs (every thread); false (and the device error
-// flag set) when the wait gave up, after a second bounded wait for them.
-__device__ bool tcWait(TcSmem& S, uint32_t& phase) {
-    const bool ok = __syncthreads_and(bar_wait(&S.bar, phase));
-    if (!ok) {
-        bar_wait(&S.bar, phase);
-        if (threadIdx.x == 0) atomicOr(&g_tc_error, 1);
+        tc_commit(&G.bar[mt]);
     }
-    phase ^= 1u;
+}
+__device__ __forceinline__ void tcIssue2(const TcSmem& S, TcGroup& G, uint32_t tmem, int mt) {
     tc_after_sync();
-    return ok;
+    const uint64_t a0 = sdesc(saddr(G.a1), A1PLANE, 128) + mt * 128, b0 = sdesc(saddr(S.w2t), 512, 128);
+#pragma unroll
+    for (int s = 0; s < KS2; s++) {
+        const int tap = s >> 1, kb = s & 1;
+        const uint32_t cell = kb * 2 * A1C + (tap / 3) * RI + tap % 3;
+        tc_mma(tmem + mt * 32, a0 + cell, b0 + (tap * 4 + 2 * kb) * (512 / 16), s > 0);
+    }
+    tc_commit(&G.bar[M1TC + mt]);
 }
 
-// Layer-1 epilogue: rows of M tiles warp/4 and warp/4 + 2 at this warp's
-// tensor-memory lanes -> relu(acc + b1 - (centre bed - bref) sbed) as BF16
-// into the activation planes.
-__device__ void tcEpilogue1(TcSmem& S, uint32_t tmem) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lg = warp & 3;
-    const float bref = S.bref;
-#pragma unroll 1
-    for (int mt = warp >> 2; mt < M1TC; mt += 2) {
-        const int m = mt * 128 + 32 * lg + lane;
-        const float cb = S.xbed[min(m, A1C - 1) + 2 * RI + 2] - bref;
+// The issuing warp of a group (one lane): each staged block's MMAs as their
+// operands come, until the group says stop.  A warp of its own, because
+// issuing an MMA waits while the tensor pipe's queue is full: issued from a
+// warp of the group, that warp's epilogue (and so the group's) started when
+// nearly all MMAs were done, and four groups were no faster than three CTAs.
+__device__ void tcIssuer(const TcSmem& S, TcGroup& G, uint32_t tmem) {
+    uint32_t phase = 0;
+    bool ok = true;
+    while (ok) {
+        ok = bar_wait(&G.in, phase);
+        if (!ok || *(volatile int*)&G.stop) break;
+        tcIssue1(S, G, tmem);
+        // layer 2 of tile mt reads rows up to 46 past the tile's: it follows
+        // the epilogues of tiles mt and mt + 1
+        ok = bar_wait(&G.act[0], phase);
+        for (int mt = 0; mt < M2TC && ok; mt++) {
+            ok = bar_wait(&G.act[mt + 1], phase);
+            if (ok) tcIssue2(S, G, tmem, mt);
+        }
+        phase ^= 1u;
+    }
+    if (!ok) atomicOr(&g_tc_error, 1);
+}
+
+// A completion wait of the group gave up: the device error flag, a bounded
+// wait for the MMAs in flight (before the CTA's memory goes).
+__device__ void tcFail(TcGroup& G, uint32_t phase) {
+    for (int k = 0; k < M1TC + M2TC; k++) bar_wait(&G.bar[k], phase);
+    if (threadIdx.x % GT == 0) atomicOr(&g_tc_error, 1);
+}
+// End of a group's blocks (every thread of the group).
+__device__ __forceinline__ void tcEnd(TcGroup& G, int g, uint32_t phase, bool ok) {
+    if (!groupAnd(g, ok)) tcFail(G, phase ^ 1u);
+    if (threadIdx.x % GT == 0) {
+        G.stop = 1;
+        bar_arrive(&G.in);
+    }
+}
+
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+// Layer-1 epilogue: this warp's quarter of the rows of M tile mt ->
+// relu(acc + b1 - (centre bed - bref) sbed) as BF16 into the activation planes.
+__device__ __forceinline__ void tcEpilogue1(const TcSmem& S, TcGroup& G, uint32_t tmem, int mt) {
+    const int lg = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
+    if (mt * 128 + 32 * lg >= A1C) return;  // (warp-uniform) rows that no output reads
+    const int m = mt * 128 + 32 * lg + lane;
+    const float cb = G.xbed[min(m, A1C - 1) + 2 * RI + 2] - G.bref;
+    float v[32];
+    tc_ld32(tmem + ((uint32_t)(32 * lg) << 16) + mt * 32, v);
+    if (m < A1C) {
 #pragma unroll
-        for (int p = 0; p < 4; p++) {  // 8 channels (one plane) at a time
-            float v[8];
-            tc_ld8(tmem + ((uint32_t)(32 * lg) << 16) + mt * 32 + 8 * p, v);
-            if (m >= A1C) continue;
-            uint4 w;
+        for (int p = 0; p < 4; p++) {  // 8 channels: one plane
             uint32_t q[4];
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const int o = 8 * p + 2 * e;
-                q[e] = pack2(relu(v[2 * e] + S.b1[o] - cb * S.sbed[o]),
-                             relu(v[2 * e + 1] + S.b1[o + 1] - cb * S.sbed[o + 1]));
+            for (int e = 0; e < 2; e++) {
+                const int o = 8 * p + 4 * e;
+                const float4 b = ld4(&S.b1[o]), w = ld4(&S.sbed[o]);
+                q[2 * e] = pack2(relu(v[o] + b.x - cb * w.x), relu(v[o + 1] + b.y - cb * w.y));
+                q[2 * e + 1] = pack2(relu(v[o + 2] + b.z - cb * w.z), relu(v[o + 3] + b.w - cb * w.w));
             }
-            w.x = q[0];
-            w.y = q[1];
-            w.z = q[2];
-            w.w = q[3];
-            *reinterpret_cast<uint4*>(&S.a1[p][m * 8]) = w;
+            *reinterpret_cast<uint4*>(&G.a1[p][m * 8]) = make_uint4(q[0], q[1], q[2], q[3]);
         }
     }
     proxy_fence();
     tc_before_sync();
 }
 
+// The staged block's layer 1 by its group (threads of the group, after their
+// barrier): an M tile's epilogue starts as soon as its own MMAs are done.
+// False when a wait of this thread's warp gave up.
+__device__ __forceinline__ bool tcLayer1(const TcSmem& S, TcGroup& G, uint32_t tmem, uint32_t phase) {
+    bool ok = true;
+#pragma unroll 1
+    for (int mt = 0; mt < M1TC; mt++) {
+        ok = __all_sync(0xffffffffu, bar_wait(&G.bar[mt], phase)) && ok;
+        tc_after_sync();
+        tcEpilogue1(S, G, tmem, mt);
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) bar_arrive(&G.act[mt]);
+    }
+    return ok;
+}
+// Wait for M tile mt of layer 2.
+__device__ __forceinline__ bool tcWait2(TcGroup& G, int mt, uint32_t phase) {
+    const bool ok = bar_wait(&G.bar[M1TC + mt], phase);
+    tc_after_sync();
+    return ok;
+}
+
 // Layer-2 epilogue and layer 3 for the row of M tile mt at this thread's
 // lane: out = W3 relu(acc + b2) + b3.  Returns the output cell's index in
 // the 16 x 16 tile (oy*16 + ox), or -1 for a row that is not an output.
-__device__ int tcOutputs(const TcSmem& S, uint32_t tmem, int mt, float out[COUT]) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lg = warp & 3;
+__device__ __forceinline__ int tcOutputs(const TcSmem& S, uint32_t tmem, int mt, float out[COUT]) {
+    const int lg = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
     const int m = mt * 128 + 32 * lg + lane, oy = m / RI, ox = m % RI;
 #pragma unroll
     for (int c = 0; c < COUT; c++) out[c] = S.b3[c];
+    float v[32];
+    tc_ld32(tmem + ((uint32_t)(32 * lg) << 16) + mt * 32, v);
 #pragma unroll
-    for (int q = 0; q < 4; q++) {  // 8 channels at a time
-        float v[8];
-        tc_ld8(tmem + ((uint32_t)(32 * lg) << 16) + mt * 32 + 8 * q, v);
+    for (int q = 0; q < 8; q++) {
+        const float4 b = ld4(&S.b2[4 * q]);
+        const float bq[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const float a = relu(v[k] + S.b2[8 * q + k]);
-#pragma unroll
-            for (int c = 0; c < COUT; c++) out[c] = fmaf(S.w3[c][8 * q + k], a, out[c]);
+        for (int k = 0; k < 4; k++) {
+            const float a = relu(v[4 * q + k] + bq[k]);
+            const float4 w = ld4(S.w3[4 * q + k]);
+            out[0] = fmaf(w.x, a, out[0]);
+            out[1] = fmaf(w.y, a, out[1]);
+            out[2] = fmaf(w.z, a, out[2]);
+            out[3] = fmaf(w.w, a, out[3]);
         }
     }
     return (oy >= OT || ox >= OT) ? -1 : oy * OT + ox;
@@ -744,42 +861,45 @@ __global__ void __launch_bounds__(128) k_tc_selftest(float* __restrict__ out) {
 
 // ------------------------------------------------------------------ forward
 // Raw net outputs of every output cell of src.
-__global__ void __launch_bounds__(NT, 3) k_forward(rift_closure_src src, const float* __restrict__ P,
-                                                   float* __restrict__ out) {
+__global__ void __launch_bounds__(TCT, 1) k_forward(rift_closure_src src, const float* __restrict__ P,
+                                                    float* __restrict__ out) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     TcSmem& S = *reinterpret_cast<TcSmem*>(smem_raw);
-    const int warp = threadIdx.x >> 5;
-    tcSetup(S, P);
-    const uint32_t tmem = S.tmem;
-    uint32_t phase = 0;
-    const int ntile = tileCount(src);
+    const int g = tcGroupOf(), lane = threadIdx.x & 31;
+    TcGroup& T = S.g[g];
+    const int ntile = tileCount(src), stride = TCG * (int)gridDim.x;
+    int tile = g * (int)gridDim.x + (int)blockIdx.x;
     TcInput R;
-    if ((int)blockIdx.x < ntile) {
-        const TileGeom G0 = tileGeom(src, blockIdx.x);
+    if (threadIdx.x < TCG * GT && tile < ntile) {
+        const TileGeom G0 = tileGeom(src, tile);
         tcLoadInput(R, src, G0.s, G0.Y - 3, G0.X - 3);
     }
-    for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+    tcSetup(S, P);
+    const uint32_t tmem = S.tmem + g * TMEM_COLS;
+    if (threadIdx.x >= TCG * GT) {
+        if (lane == 0) tcIssuer(S, T, tmem);
+        __syncwarp();
+        tcTeardown(S);
+        return;
+    }
+    uint32_t phase = 0;
+    bool ok = true;
+    for (; tile < ntile; tile += stride, phase ^= 1u) {
         const TileGeom G = tileGeom(src, tile);
-        __syncthreads();
-        tcStoreInput(S, R, src);
-        __syncthreads();
-        if (threadIdx.x == 0) tcIssue1(S, tmem);
-        if (tile + (int)gridDim.x < ntile) {  // the next block's inputs, during the MMAs
-            const TileGeom Gn = tileGeom(src, tile + gridDim.x);
+        tcStoreInput(T, R, src);
+        if (!groupAnd(g, ok)) break;
+        if (threadIdx.x % GT == 0) bar_arrive(&T.in);
+        if (tile + stride < ntile) {  // the next block's inputs, during the MMAs
+            const TileGeom Gn = tileGeom(src, tile + stride);
             tcLoadInput(R, src, Gn.s, Gn.Y - 3, Gn.X - 3);
         }
-        if (!tcWait(S, phase)) break;
-        tcEpilogue1(S, tmem);
-        __syncthreads();
-        if (threadIdx.x == 0) tcIssue2(S, tmem);
-        if (!tcWait(S, phase)) break;
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const int mt = (warp >> 2) + 2 * k;
-            if (mt >= M2TC) break;
+        ok = tcLayer1(S, T, tmem, phase);
+#pragma unroll 1
+        for (int mt = 0; mt < M2TC; mt++) {
+            ok = __all_sync(0xffffffffu, tcWait2(T, mt, phase)) && ok;
             float o[COUT];
             const int q = tcOutputs(S, tmem, mt, o);
-            if (q < 0) continue;
+            if (q < 0 || !ok) continue;
             const int y = G.Y + q / OT - src.oy0, x = G.X + q % OT - src.ox0;
             if (y >= src.OH || x >= src.OW) continue;
 #pragma unroll
@@ -788,6 +908,7 @@ __global__ void __launch_bounds__(NT, 3) k_forward(rift_closure_src src, const f
         }
         tc_before_sync();
     }
+    tcEnd(T, g, phase, ok);
     tcTeardown(S);
 }
 
@@ -1133,45 +1254,67 @@ struct ApplyArgs {
     size_t plane;
     int pitch, nx, ny;
     float dtw, inv_dx, inv_dy, hmin, lim, tau;
+    int* ticket;    // blocks drawn so far (zero at the launch)
     uint8_t* fell;  // per 16 x 16 block: 1 when it fell back to the plain solve
     int* counters;
 };
 
 // Net outputs -> gated, limited face corrections of every 16 x 16 block of
 // interior cells (zeros for dry blocks and blocks that fall back).
-__global__ void __launch_bounds__(NT, 3) k_closure(ApplyArgs A) {
+// The groups draw their blocks from a ticket (dry blocks cost next to nothing,
+// and water lies in patches: with fixed shares an SM held up to 1.4 times the
+// mean of the wet ones).  A leader draws two blocks ahead, so no one waits for
+// the ticket.
+__global__ void __launch_bounds__(TCT, 1) k_closure(ApplyArgs A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     TcSmem& S = *reinterpret_cast<TcSmem*>(smem_raw);
     const rift_closure_src& src = A.src;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    tcSetup(S, A.P);
-    const uint32_t tmem = S.tmem;
-    uint32_t phase = 0;
+    const int g = tcGroupOf(), tid = threadIdx.x % GT, lane = tid & 31;
+    TcGroup& T = S.g[g];
     const float hminS = A.hmin * src.scale[0], invS0 = 1.f / src.scale[0];
-    const int ntile = tileCount(src);
+    const int ntile = tileCount(src), first = TCG * (int)gridDim.x;
+    int tile = g * (int)gridDim.x + (int)blockIdx.x, next = 0;
+    int drawn = 0;  // leader: the ticket after the next
+    if (threadIdx.x < TCG * GT && tid == 0) drawn = first + atomicAdd(A.ticket, 1);
     TcInput R;
-    if ((int)blockIdx.x < ntile) {
-        const TileGeom G0 = tileGeom(src, blockIdx.x);
+    if (threadIdx.x < TCG * GT && tile < ntile) {
+        const TileGeom G0 = tileGeom(src, tile);
         tcLoadInput(R, src, 0, G0.Y - 3, G0.X - 3);
     }
-    for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+    tcSetup(S, A.P);
+    const uint32_t tmem = S.tmem + g * TMEM_COLS;
+    if (threadIdx.x >= TCG * GT) {
+        if (lane == 0) tcIssuer(S, T, tmem);
+        __syncwarp();
+        tcTeardown(S);
+        return;
+    }
+    uint32_t phase = 0;
+    bool ok = true;
+    for (; tile < ntile; tile = next) {
         const TileGeom G = tileGeom(src, tile);
-        __syncthreads();
-        if (tid == 0) S.red[0] = 0;
-        tcStoreInput(S, R, src);
-        if (tile + (int)gridDim.x < ntile) {  // the next block's inputs, in flight meanwhile
-            const TileGeom Gn = tileGeom(src, tile + gridDim.x);
+        if (tid == 0) {
+            T.red = 0;
+            T.next = drawn;
+            drawn = first + atomicAdd(A.ticket, 1);
+        }
+        tcStoreInput(T, R, src);
+        if (!groupAnd(g, ok)) break;
+        bool dry = true;
+        for (int i = tid; i < (OT + 1) * (OT + 1); i += GT) {
+            int ry = 3 + i / (OT + 1), rx = 3 + i % (OT + 1);
+            dry &= !(T.xh[ry * RI + rx] > hminS);
+        }
+        dry = groupAnd(g, dry);
+        if (tid == 0 && !dry) bar_arrive(&T.in);
+        next = T.next;
+        if (next < ntile) {  // the next block's inputs, in flight meanwhile
+            const TileGeom Gn = tileGeom(src, next);
             tcLoadInput(R, src, 0, Gn.Y - 3, Gn.X - 3);
         }
-        __syncthreads();
-        int wet = 0;
-        for (int i = tid; i < (OT + 1) * (OT + 1); i += NT) {
-            int ry = 3 + i / (OT + 1), rx = 3 + i % (OT + 1);
-            wet |= S.xh[ry * RI + rx] > hminS;
-        }
-        if (!__syncthreads_or(wet)) {
+        if (dry) {
             if (tid == 0) A.fell[tile] = 0;
-            for (int i = tid; i < OT * OT; i += NT) {
+            for (int i = tid; i < OT * OT; i += GT) {
                 int y = G.Y + i / OT, x = G.X + i % OT;
                 if (y - src.oy0 >= src.OH || x - src.ox0 >= src.OW) continue;
                 size_t c = (size_t)y * A.pitch + x;
@@ -1180,34 +1323,28 @@ __global__ void __launch_bounds__(NT, 3) k_closure(ApplyArgs A) {
             }
             continue;
         }
-        if (tid == 0) tcIssue1(S, tmem);
-        if (!tcWait(S, phase)) break;
-        tcEpilogue1(S, tmem);
-        __syncthreads();
-        if (tid == 0) tcIssue2(S, tmem);
-        if (!tcWait(S, phase)) break;
-        // this thread's output cells (up to two) and their four corrections:
+        ok = tcLayer1(S, T, tmem, phase);
+        // this thread's output cells (up to three) and their four corrections:
         // east-face mass and momentum, north-face mass and momentum
-        int cell[2] = {-1, -1};
-        float cv[2][4] = {};
+        int cell[M2TC] = {-1, -1, -1};
+        float cv[M2TC][4] = {};
         float ind = 0.f;
 #pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const int mt = (warp >> 2) + 2 * k;
-            if (mt >= M2TC) break;
+        for (int k = 0; k < M2TC; k++) {
+            ok = __all_sync(0xffffffffu, tcWait2(T, k, phase)) && ok;
             float o[COUT];
-            const int q = tcOutputs(S, tmem, mt, o);
-            if (q < 0) continue;
+            const int q = tcOutputs(S, tmem, k, o);
+            if (q < 0 || !ok) continue;
             const int oy = q / OT, ox = q % OT, y = G.Y + oy, x = G.X + ox;
             if (y - src.oy0 >= src.OH || x - src.ox0 >= src.OW) continue;
             cell[k] = q;
-            const float hc = S.xh[(oy + 3) * RI + ox + 3] * invS0;
+            const float hc = T.xh[(oy + 3) * RI + ox + 3] * invS0;
 #pragma unroll
             for (int f = 0; f < 2; f++) {
                 const bool east = f == 0;
                 const float inv = east ? A.inv_dx : A.inv_dy;
                 const int yn = east ? y : y + 1, xn = east ? x + 1 : x;
-                const float hn = S.xh[(oy + 3 + (east ? 0 : 1)) * RI + ox + 3 + (east ? 1 : 0)] * invS0;
+                const float hn = T.xh[(oy + 3 + (east ? 0 : 1)) * RI + ox + 3 + (east ? 1 : 0)] * invS0;
                 const bool ok = x >= 3 && y >= 3 && xn <= A.nx - 4 && yn <= A.ny - 4 && hc > A.hmin &&
                                 hn > A.hmin;
                 float vm = ok ? o[2 * f] * A.osc[2 * f] : 0.f;
@@ -1224,11 +1361,11 @@ __global__ void __launch_bounds__(NT, 3) k_closure(ApplyArgs A) {
         }
         tc_before_sync();
         for (int s = 16; s > 0; s >>= 1) ind = fmaxf(ind, __shfl_xor_sync(0xffffffffu, ind, s));
-        if (lane == 0) atomicMax(&S.red[0], __float_as_int(ind));
-        __syncthreads();
-        const bool fallback = __int_as_float(S.red[0]) > A.tau;
+        if (lane == 0) atomicMax(&T.red, __float_as_int(ind));
+        groupSync(g);
+        const bool fallback = __int_as_float(T.red) > A.tau;
 #pragma unroll
-        for (int k = 0; k < 2; k++) {
+        for (int k = 0; k < M2TC; k++) {
             if (cell[k] < 0) continue;
             const size_t c = (size_t)(G.Y + cell[k] / OT) * A.pitch + G.X + cell[k] % OT;
 #pragma unroll
@@ -1239,7 +1376,10 @@ __global__ void __launch_bounds__(NT, 3) k_closure(ApplyArgs A) {
             atomicAdd(&A.counters[0], 1);
             if (fallback) atomicAdd(&A.counters[1], 1);
         }
+        groupSync(g);  // red is read before the next block clears it
+        phase ^= 1u;
     }
+    tcEnd(T, g, phase, ok);
     tcTeardown(S);
 }
 
@@ -1248,34 +1388,39 @@ __global__ void __launch_bounds__(NT, 3) k_closure(ApplyArgs A) {
 // 16 x 16 blocks of its two cells fell back: both cells then see the same
 // correction (mass stays conserved) and every cell of a fallen-back block
 // keeps the plain solve exactly.
+// (Loads first, tests after: behind the tests each load waited for the last,
+// 17 us on 1024^2 cells.)
 __global__ void k_apply(float* __restrict__ h, float* __restrict__ hu, float* __restrict__ hv,
-                        const float* __restrict__ corr, const uint8_t* __restrict__ fell, size_t plane,
+                        float* __restrict__ corr, const uint8_t* __restrict__ fell, size_t plane,
                         int pitch, int nx, int ny, float sx, float sy) {
     const int i = 3 + blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 3 + blockIdx.y * blockDim.y + threadIdx.y;
+    if (i == 3 && j == 3) corr[0] = 0.f;  // k_closure's ticket (a corner of the ghost ring)
     if (i > nx - 4 || j > ny - 4) return;
+    const size_t c = (size_t)j * pitch + i;
+    const float cE = corr[c], cW = corr[c - 1], dE = corr[plane + c], dW = corr[plane + c - 1];
+    const float cN = corr[2 * plane + c], cS = corr[2 * plane + c - pitch];
+    const float dN = corr[3 * plane + c], dS = corr[3 * plane + c - pitch];
+    const float h0 = h[c], u0 = hu[c], v0 = hv[c];
+    const int tx = (nx - 4 + OT - 1) / OT;
+    const int bx = (i - 2) / OT, by = (j - 2) / OT, b = by * tx + bx;
+    const bool w = (i - 2) % OT == 0, e = (i - 1) % OT == 0 && i + 1 <= nx - 3;
+    const bool s = (j - 2) % OT == 0, n = (j - 1) % OT == 0 && j + 1 <= ny - 3;
+    // (i, j >= 3: a cell on its block's west or south side has a block there)
+    const bool own = fell[b] != 0, fW = fell[w ? b - 1 : b], fE = fell[e ? b + 1 : b];
+    const bool fS = fell[s ? b - tx : b], fN = fell[n ? b + tx : b];
     // a tensor-core wait of k_closure gave up: some blocks' corrections were
     // not written, so the whole step keeps the plain solve
-    if (*(volatile int*)&g_tc_error) return;
-    const int tx = (nx - 4 + OT - 1) / OT;
-    const int bx = (i - 2) / OT, by = (j - 2) / OT;
-    const bool own = fell[by * tx + bx] != 0;
-    if (own) return;  // every face of this cell touches its own block
-    const bool westOff = ((i - 2) % OT == 0) && fell[by * tx + bx - 1];
-    const bool eastOff = ((i - 1) % OT == 0) && (i + 1 <= nx - 3) && fell[by * tx + bx + 1];
-    const bool southOff = ((j - 2) % OT == 0) && fell[(by - 1) * tx + bx];
-    const bool northOff = ((j - 1) % OT == 0) && (j + 1 <= ny - 3) && fell[(by + 1) * tx + bx];
-    const size_t c = (size_t)j * pitch + i;
-    const float mE = eastOff ? 0.f : corr[c], mW = westOff ? 0.f : corr[c - 1];
-    const float mN = northOff ? 0.f : corr[2 * plane + c], mS = southOff ? 0.f : corr[2 * plane + c - pitch];
-    const float uE = eastOff ? 0.f : corr[plane + c], uW = westOff ? 0.f : corr[plane + c - 1];
-    const float vN = northOff ? 0.f : corr[3 * plane + c], vS = southOff ? 0.f : corr[3 * plane + c - pitch];
+    const bool failed = *(volatile int*)&g_tc_error != 0;
+    if (own || failed) return;  // own: every face of this cell touches its own block
+    const float mE = fE ? 0.f : cE, mW = fW ? 0.f : cW, mN = fN ? 0.f : cN, mS = fS ? 0.f : cS;
+    const float uE = fE ? 0.f : dE, uW = fW ? 0.f : dW, vN = fN ? 0.f : dN, vS = fS ? 0.f : dS;
     if (mE == 0.f && mW == 0.f && mN == 0.f && mS == 0.f && uE == 0.f && uW == 0.f && vN == 0.f &&
         vS == 0.f)
         return;
-    h[c] -= sx * (mE - mW) + sy * (mN - mS);
-    hu[c] -= sx * (uE - uW);
-    hv[c] -= sy * (vN - vS);
+    h[c] = h0 - (sx * (mE - mW) + sy * (mN - mS));
+    hu[c] = u0 - sx * (uE - uW);
+    hv[c] = v0 - sy * (vN - vS);
 }
 
 }  // namespace rc
@@ -1301,42 +1446,14 @@ bool srcOk(const rift_closure_src* s) {
            (s->samples == 1 || s->sample_stride >= (int64_t)s->pitch * s->H);
 }
 
-// Resident CTAs of kernel k with `smem` bytes, over every SM, capped by the
-// tile count.
-int residentGrid(const void* k, size_t smem, int tiles, int* out) {
-    int dev = 0, sms = 0, occ = 0;
+// CTAs of kernel k with `smem` bytes: one per SM, capped by the tile count.
+int onePerSM(const void* k, size_t smem, int tiles, int* out) {
+    int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return fail(RIFT_ERR_CUDA, "no device");
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    // the whole shared-memory carveout, so that the occupancy below (and the
-    // launch) can place three 74 KB tensor-core CTAs on an SM
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 (int)cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return fail(RIFT_ERR_CUDA, cudaGetErrorString(e));
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, rc::NT, smem);
-    if (e != cudaSuccess || occ < 1) return fail(RIFT_ERR_CUDA, "closure kernel does not fit an SM");
-    // The same count from the SM's own limits (the occupancy call above gave
-    // one CTA per SM for an 85 KB tensor-core kernel on GB300, where two fit
-    // in shared memory and registers): CTAs per SM by shared memory (with
-    // the per-block reservation) and by registers (allocated per warp in
-    // units of 256), at most 4 (4 x 128 tensor-memory columns).  The kernels
-    // loop over tiles with no CTA waiting on another, so a CTA that does not
-    // fit simply starts when one ends.
-    cudaFuncAttributes fa{};
-    int smemSM = 0, resv = 0;
-    if (cudaFuncGetAttributes(&fa, k) == cudaSuccess &&
-        cudaDeviceGetAttribute(&smemSM, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&resv, cudaDevAttrReservedSharedMemoryPerBlock, dev) == cudaSuccess) {
-        const size_t perBlock = smem + fa.sharedSizeBytes + (size_t)resv;
-        const int bySmem = (int)((size_t)smemSM / perBlock);
-        const int regsWarp = ((fa.numRegs * 32 + 255) / 256) * 256;
-        const int byRegs = regsWarp > 0 ? 65536 / (regsWarp * (rc::NT / 32)) : 1;
-        int mine = bySmem < byRegs ? bySmem : byRegs;
-        mine = mine < 4 ? mine : 4;
-        occ = occ > mine ? occ : mine;
-    }
-    *out = tiles < sms * occ ? tiles : sms * occ;
+    *out = tiles < sms ? tiles : sms;
     return RIFT_OK;
 }
 }  // namespace
@@ -1348,8 +1465,8 @@ int rift_closure_forward(const rift_closure_src* src, const float* params, float
     const size_t smem = sizeof(rc::TcSmem);
     const int tiles = rc::tileCount(*src);
     int grid = 0, rc_;
-    if ((rc_ = residentGrid((const void*)rc::k_forward, smem, tiles, &grid))) return rc_;
-    rc::k_forward<<<grid, rc::NT, smem, (cudaStream_t)stream>>>(*src, params, out);
+    if ((rc_ = onePerSM((const void*)rc::k_forward, smem, tiles, &grid))) return rc_;
+    rc::k_forward<<<grid, rc::TCT, smem, (cudaStream_t)stream>>>(*src, params, out);
     return launched("k_forward");
 }
 
@@ -1360,7 +1477,7 @@ int rift_closure_train(const rift_closure_src* src, const float* params, const f
     const size_t smem = sizeof(rc::TrainSmem);
     const int tiles = rc::tileCount(*src);
     int grid = 0, rc_;
-    if ((rc_ = residentGrid((const void*)rc::k_train, smem, tiles, &grid))) return rc_;
+    if ((rc_ = onePerSM((const void*)rc::k_train, smem, tiles, &grid))) return rc_;
     rc::TrainArgs A{*src, params, target, weight, loss_scale, grad, loss};
     rc::k_train<<<grid, rc::NT, smem, (cudaStream_t)stream>>>(A);
     return launched("k_train");
@@ -1425,8 +1542,11 @@ int rift_closure_apply(const rift_device_view* view, const rift_closure_src* src
     const size_t smem = sizeof(rc::TcSmem);
     const int tiles = rc::tileCount(*src);
     int grid = 0, rc_;
-    if ((rc_ = residentGrid((const void*)rc::k_closure, smem, tiles, &grid))) return rc_;
-    rc::k_closure<<<grid, rc::NT, smem, st>>>(A);
+    if ((rc_ = onePerSM((const void*)rc::k_closure, smem, tiles, &grid))) return rc_;
+    // the blocks' ticket: a corner of the ghost ring of corr, which holds no correction
+    A.ticket = reinterpret_cast<int*>(corr);
+    if (cudaMemsetAsync(A.ticket, 0, sizeof(int), st) != cudaSuccess) return launched("ticket");
+    rc::k_closure<<<grid, rc::TCT, smem, st>>>(A);
     if ((rc_ = launched("k_closure"))) return rc_;
     dim3 blk(32, 8), grd((view->h_nx - 6 + 31) / 32, (view->h_ny - 6 + 7) / 8);
     rc::k_apply<<<grd, blk, 0, st>>>(view->h, view->hu, view->hv, corr, block_fell, A.plane, view->pitch,
@@ -1441,13 +1561,15 @@ int rift_closure_selftest(float* out, void* stream) {
 }
 
 int rift_closure_check(void* stream) {
-    cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
-    if (e != cudaSuccess) return fail(RIFT_ERR_CUDA, std::string("rift_closure_check: ") + cudaGetErrorString(e));
+    // one copy on the stream and one wait; the flag is written back only when it was set
+    const cudaStream_t st = (cudaStream_t)stream;
     int flag = 0;
     const int zero = 0;
-    if (cudaMemcpyFromSymbol(&flag, rc::g_tc_error, sizeof(int)) != cudaSuccess ||
-        cudaMemcpyToSymbol(rc::g_tc_error, &zero, sizeof(int)) != cudaSuccess)
-        return fail(RIFT_ERR_CUDA, "rift_closure_check: status read failed");
+    cudaError_t e = cudaMemcpyFromSymbolAsync(&flag, rc::g_tc_error, sizeof(int), 0, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return fail(RIFT_ERR_CUDA, std::string("rift_closure_check: ") + cudaGetErrorString(e));
+    if (flag && cudaMemcpyToSymbol(rc::g_tc_error, &zero, sizeof(int)) != cudaSuccess)
+        return fail(RIFT_ERR_CUDA, "rift_closure_check: status reset failed");
     if (flag) return fail(RIFT_ERR_CUDA, "rift_closure_check: a tensor-core completion wait gave up");
     return RIFT_OK;
 }
