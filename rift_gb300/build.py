@@ -57,7 +57,7 @@ def build_host(force: bool = False) -> str:
 
 
 CLOSURE_LIB = os.path.join(LIB_DIR, "librift_closure.so")
-CLOSURE_DEPS = ["rift_closure.cu", "rift_device.cuh"]
+CLOSURE_DEPS = ["rift_closure.cu", "rift_device.cuh", "rift_pair.cuh"]
 
 
 def build(force: bool = False, verbose: bool = False) -> str:

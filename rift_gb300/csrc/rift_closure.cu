@@ -1,23 +1,19 @@
 // rift_closure.cu -- learned sub-grid flux closure on a 2x-coarsened grid.
 //
 // The net (6 -> 32 channels 5x5, 32 -> 32 3x3, 32 -> 4 1x1, ReLU between)
-// runs tile by tile: a CTA stages a 22 x 22 block of the six input channels,
-// computes layer 1 on the 18 x 18 cells that layer 2 needs, and layers 2 and
-// 3 on the 16 x 16 output cells.  Every contraction is an implicit GEMM on
-// the BF16 tensor cores (mma.sync m16n8k16, FP32 accumulation): the rows of
-// an MMA tile are 16 cells, the columns output channels, and the reduction
-// runs over (tap, input channel).  Layer 1 activations stay in shared memory
-// as BF16 in channels-last rows of 40 (32 channels + 8 of padding, so the
-// fragment loads of eight consecutive cells fall in distinct banks); layer 2
-// outputs stay in registers, and their accumulator fragments are the A
-// fragments of layer 3 without leaving the thread.
+// runs tile by tile: a 22 x 22 block of the six input channels, layer 1 on the
+// 18 x 18 cells that layer 2 needs, layers 2 and 3 on the 16 x 16 output cells.
+// Every contraction is an implicit GEMM on BF16 operands with FP32
+// accumulation: rows are cells, columns output channels, and the reduction
+// runs over (tap, input channel).
 //
-// The training kernel recomputes the forward pass of its tile and runs the
-// backward pass in the same CTA: layer-3 gradients on the CUDA cores (4 x 32
-// weights), the layer-2 and layer-1 weight gradients and the layer-1
-// activation gradient as tensor-core GEMMs.  Weight gradients stay in
-// registers across every tile a CTA visits and are added to the global
-// gradient once per CTA.
+// Inference (k_forward, k_closure) runs on tcgen05.mma with accumulators in
+// tensor memory, four blocks in flight per SM.  Training (k_train) recomputes
+// the forward pass of its tile and runs the backward pass in the same CTA, on
+// mma.sync with fragments by ldmatrix: layer-3 gradients on the CUDA cores
+// (4 x 32 weights), the layer-2 and layer-1 weight gradients and the layer-1
+// activation gradient as GEMMs.  Weight gradients stay in registers across
+// every tile a CTA visits and are added to the global gradient once per CTA.
 //
 // The flux kernel evaluates the step's central-upwind face flux
 // (rift_device.cuh) on a handle's state, for the time-integrated fluxes
@@ -46,8 +42,7 @@ constexpr int CB = 8;            // BF16 input channels per cell: h, hu, hv, b_h
 constexpr int NTAP1 = 26;        // layer-1 taps, the 26th a zero-weight pad
 constexpr int K1B = NTAP1 * CB;  // 208: layer-1 reduction over the BF16 inputs
 constexpr int SW1 = K1B + 8, SW2 = 296, SW3 = 40;  // BF16 row strides of the weights
-constexpr int NT = 256;
-constexpr int BEDBIT = 1 << 20, OFFMASK = BEDBIT - 1;
+constexpr int TT = 512;          // threads of a training CTA: 16 warps
 
 constexpr int OFF_W1 = RIFT_CLOSURE_OFF_W1, OFF_B1 = RIFT_CLOSURE_OFF_B1;
 constexpr int OFF_W2 = RIFT_CLOSURE_OFF_W2, OFF_B2 = RIFT_CLOSURE_OFF_B2;
@@ -57,29 +52,29 @@ static_assert(OFF_B1 == OFF_W1 + C1 * K1P && OFF_W2 == OFF_B1 + C1 && OFF_B2 == 
                   RIFT_CLOSURE_NPARAM == OFF_B3 + 8,
               "parameter layout");
 
-struct NetSmem {
-    float xs[NRI * CIN];       // scaled inputs (FP32), channels last
-    uint16_t xb[NRI * CB];     // the same as BF16 rows of 8; the bed relative to bref, in two halves
-    uint16_t a1[NR1 * SA];     // layer-1 activations (BF16); dZ1 in the backward pass
-    uint16_t w1[C1 * SW1];     // W1 over the BF16 inputs: [o][tap*8 + c8]
-    uint16_t w2[C1 * SW2];     // W2[o][k]
-    uint16_t w3[8 * SW3];      // W3[o][c], rows 4..7 zero
-    float b1[C1], b2[C1], b3[8];
-    float sbed[C1];            // sum over taps of layer 1's (BF16) bed weights
-    int toff[NTAP1];           // cell offset of each layer-1 tap in the input block
-    int koffE[K1P];            // xs offset of each layer-1 reduction index (weight gradient)
-    float bref;                // the block's reference bed (scaled)
-    int red[4];
-};
-
-struct TrainSmem {
-    NetSmem n;
+struct __align__(128) TrainSmem {
+    uint16_t xb[NRI * CB];      // input cells: BF16 rows of 8, the bed relative to bref in two halves
+    uint16_t a1[NR1 * SA];      // layer-1 activations (BF16); dZ1 in the backward pass
     uint16_t a2[OT * OT * SA];  // layer-2 activations, then dZ2
-    uint16_t w2t[K2 * SA];      // W2 transposed: [k][o]
+    uint16_t w1[C1 * SW1];      // W1 over the BF16 inputs: [o][tap*8 + c8]
+    uint16_t w2[C1 * SW2];      // W2[o][k]
+    uint16_t w3[8 * SW3];       // W3[o][c], rows 4..7 zero
+    uint16_t zero[SA];          // a row of zeros, for cells outside
     float dout[OT * OT * 4];
-    float w3f[4 * C1];
-    double red[NT / 32];
+    float w3q[C1][4];           // W3 (FP32), a channel's four weights together
+    float xbed[NRI];            // scaled FP32 bed of the input cells
+    float b1[C1], b2[C1], b3[8];
+    float sbed[C1];             // sum over taps of layer 1's (BF16) bed weights
+    int toff[NTAP1];            // cell offset of each layer-1 tap in the input block
+    int qcell[M1T * 16];        // input cell of each layer-1 cell (its window's corner)
+    float bref;                 // the block's reference bed (scaled)
+    double red[TT / 32];
 };
+static_assert(offsetof(TrainSmem, a1) % 16 == 0 && offsetof(TrainSmem, a2) % 16 == 0 &&
+                  offsetof(TrainSmem, w1) % 16 == 0 && offsetof(TrainSmem, w2) % 16 == 0 &&
+                  offsetof(TrainSmem, zero) % 16 == 0 && offsetof(TrainSmem, dout) % 16 == 0 &&
+                  offsetof(TrainSmem, w3q) % 16 == 0 && SA % 8 == 0 && SW1 % 8 == 0 && SW2 % 8 == 0,
+              "fragment loads are 16-byte aligned");
 
 __device__ __forceinline__ uint16_t bf(float x) { return __bfloat16_as_ushort(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ float fb(uint16_t x) { return __bfloat162float(__ushort_as_bfloat16(x)); }
@@ -119,24 +114,38 @@ __device__ __forceinline__ void ldsm4(uint32_t r[4], const void* p) {
                  : "r"(a));
 }
 
-// Weights (BF16), biases and the layer-1 offset tables, once per CTA.
-// Layer 1 reads the BF16 input rows (h, hu, hv, b_hi, b_lo, n, rain, 0):
-// both bed halves take the bed weight.
-__device__ void stageNet(NetSmem& S, const float* __restrict__ P) {
+// The same, each matrix transposed: thread T receives rows 2(T%4), 2(T%4)+1 of
+// column T/4.
+__device__ __forceinline__ void ldsm4t(uint32_t r[4], const void* p) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a));
+}
+
+// Weights (BF16), biases and the offset tables, once per CTA.  Layer 1 reads
+// the BF16 input rows (h, hu, hv, b_hi, b_lo, n, rain, 0): both bed halves
+// take the bed weight.
+// Cell offset of a layer-1 tap in the input block (0 for a pad tap).
+__device__ __forceinline__ int tapCell(int tap) { return tap < 25 ? (tap / 5) * RI + tap % 5 : 0; }
+
+__device__ void stageNet(TrainSmem& S, const float* __restrict__ P) {
     const int tid = threadIdx.x;
     constexpr int MAP[CB] = {0, 1, 2, 3, 3, 4, 5, -1};
-    for (int i = tid; i < C1 * SW1; i += NT) {
+    for (int i = tid; i < C1 * SW1; i += TT) {
         const int o = i / SW1, k = i % SW1, tap = k / CB, c = MAP[k % CB];
         S.w1[i] = bf(k < K1B && tap < 25 && c >= 0 ? P[OFF_W1 + o * K1P + tap * CIN + c] : 0.f);
     }
-    for (int i = tid; i < C1 * SW2; i += NT) {
+    for (int i = tid; i < C1 * SW2; i += TT) {
         int o = i / SW2, k = i % SW2;
         S.w2[i] = bf(k < K2 ? P[OFF_W2 + o * K2 + k] : 0.f);
     }
-    for (int i = tid; i < 8 * SW3; i += NT) {
+    for (int i = tid; i < 8 * SW3; i += TT) {
         int o = i / SW3, k = i % SW3;
         S.w3[i] = bf(o < COUT && k < C1 ? P[OFF_W3 + o * C1 + k] : 0.f);
     }
+    if (tid < 4 * C1) S.w3q[tid % C1][tid / C1] = P[OFF_W3 + tid];
+    if (tid < SA) S.zero[tid] = 0;
     if (tid < C1) {
         S.b1[tid] = P[OFF_B1 + tid];
         S.b2[tid] = P[OFF_B2 + tid];
@@ -145,119 +154,100 @@ __device__ void stageNet(NetSmem& S, const float* __restrict__ P) {
         S.sbed[tid] = sb;
     }
     if (tid < 8) S.b3[tid] = tid < COUT ? P[OFF_B3 + tid] : 0.f;
-    if (tid < NTAP1) S.toff[tid] = tid < 25 ? (tid / 5) * RI + tid % 5 : 0;
-    for (int k = tid; k < K1P; k += NT) {
-        int e = -1;
-        if (k < K1) {
-            int tap = k / CIN, c = k % CIN;
-            e = ((tap / 5) * RI + tap % 5) * CIN + c;
-            if (c == 3) e |= BEDBIT;
-        }
-        S.koffE[k] = e;
+    if (tid < NTAP1) S.toff[tid] = tapCell(tid);
+    if (tid < M1T * 16) {
+        const int q = min(tid, NR1 - 1);
+        S.qcell[tid] = (q / R1) * RI + q % R1;
     }
 }
 
-// The 22 x 22 input block whose corner is image cell (Y0, X0) of sample s:
-// FP32 (xs) and BF16 rows (xb).  The BF16 bed is b - bref, bref the bed of
-// the block's centre cell, split into a BF16 value and its BF16 remainder
-// (16 significant bits together).
-__device__ void stageInput(NetSmem& S, const rift_closure_src& src, int s, int Y0, int X0) {
+// This thread's cell of the 22 x 22 input block whose corner is image cell (Y0,
+// X0) of sample s, and the block's reference bed (its centre cell's): loaded one
+// block ahead.
+struct TrainInput {
+    float v[CIN];
+    float bref;
+};
+__device__ __forceinline__ void loadInput(TrainInput& R, const rift_closure_src& src, int s, int Y0, int X0) {
     const size_t sbase = (size_t)s * (size_t)src.sample_stride;
     auto at = [&](int ry, int rx) {
         int y = min(max(Y0 + ry, 0), src.H - 1), x = min(max(X0 + rx, 0), src.W - 1);
         return sbase + (size_t)y * (size_t)src.pitch + (size_t)x;
     };
-    const float bref = (src.plane[3] ? __ldg(src.plane[3] + at(RI / 2, RI / 2)) : src.value[3]) * src.scale[3];
-    if (threadIdx.x == 0) S.bref = bref;
-    for (int i = threadIdx.x; i < NRI; i += NT) {
-        const size_t off = at(i / RI, i % RI);
-        float v[CIN];
+    const int i = min((int)threadIdx.x, NRI - 1);
+    const size_t off = at(i / RI, i % RI);
+    R.bref = src.plane[3] ? __ldg(src.plane[3] + at(RI / 2, RI / 2)) : src.value[3];
 #pragma unroll
-        for (int c = 0; c < CIN; c++) {
-            v[c] = (src.plane[c] ? __ldg(src.plane[c] + off) : src.value[c]) * src.scale[c];
-            S.xs[i * CIN + c] = v[c];
-        }
-        const float br = v[3] - bref;
-        const uint16_t bh = bf(br);
-        const uint16_t bl = bf(br - fb(bh));
-        uint4 w;
-        w.x = pack2(v[0], v[1]);
-        w.y = pack16(bf(v[2]), bh);
-        w.z = pack16(bl, bf(v[4]));
-        w.w = pack16(bf(v[5]), 0);
-        *reinterpret_cast<uint4*>(&S.xb[i * CB]) = w;
-    }
+    for (int c = 0; c < CIN; c++) R.v[c] = src.plane[c] ? __ldg(src.plane[c] + off) : src.value[c];
+}
+// ... into shared memory.  The BF16 bed is b - bref, split into a BF16 value and
+// its BF16 remainder (16 significant bits together).
+__device__ __forceinline__ void storeInput(TrainSmem& S, const TrainInput& R, const rift_closure_src& src) {
+    const int i = threadIdx.x;
+    const float bref = R.bref * src.scale[3];
+    if (i == 0) S.bref = bref;
+    if (i >= NRI) return;
+    float v[CIN];
+#pragma unroll
+    for (int c = 0; c < CIN; c++) v[c] = R.v[c] * src.scale[c];
+    S.xbed[i] = v[3];
+    const float br = v[3] - bref;
+    const uint16_t bh = bf(br);
+    const uint16_t bl = bf(br - fb(bh));
+    uint4 w;
+    w.x = pack2(v[0], v[1]);
+    w.y = pack16(bf(v[2]), bh);
+    w.z = pack16(bl, bf(v[4]));
+    w.w = pack16(bf(v[5]), 0);
+    *reinterpret_cast<uint4*>(&S.xb[i * CB]) = w;
 }
 
-// Layer-1 input k (tap, channel) of the cell whose 5x5 window starts at xs
-// offset `base`, FP32: the bed relative to the window's centre bc.
-__device__ __forceinline__ float featElem(const NetSmem& S, int base, float bc, int e) {
-    if (e < 0) return 0.f;
-    float v = S.xs[base + (e & OFFMASK)];
-    return (e & BEDBIT) ? v - bc : v;
-}
-__device__ __forceinline__ int winBase(int q) { return ((q / R1) * RI + q % R1) * CIN; }
-__device__ __forceinline__ float winBed(const NetSmem& S, int base) {
-    return S.xs[base + (2 * RI + 2) * CIN + 3];
-}
+// Passes over the 18 x 18 layer-1 cells: a warp takes one half of the 32
+// channels and up to three of the 21 row tiles of 16 cells.
+constexpr int WPH = TT / 64, UPW = (M1T + WPH - 1) / WPH;
 
-// Layer 1 on the 18 x 18 region: a1 = relu(W1 x + b1), BF16.  A warp owns
-// row tiles warp, warp+8 and (warps 0..4) warp+16.  One k step covers two
-// taps of the 8-channel BF16 input rows, so each 8 x 8 block of an A
+// Layer 1 on the 18 x 18 region: a1 = relu(W1 x + b1), BF16.  One k step covers
+// two taps of the 8-channel BF16 input rows, so each 8 x 8 block of an A
 // fragment is 8 cells' rows of one tap and comes with one ldmatrix; the
 // bed enters relative to bref and the epilogue subtracts (centre bed -
 // bref) x (sum of the bed weights), which makes it relative to the
 // window's centre.
-__device__ void conv1(NetSmem& S, int warp, int lane) {
+__device__ __forceinline__ void conv1(TrainSmem& S, int warp, int lane) {
     const int g = lane >> 2, t = lane & 3;
-    constexpr int MPW = (M1T + 7) / 8;  // 3
-    const bool third = warp + 16 < M1T;
     // this lane's ldmatrix rows: row (lane & 15) of each of its row tiles,
     // the tap of the k step's second half for lanes 16..31
     const int lrow = lane & 15, lhalf = lane >> 4;
-    int rowCell[MPW];
-#pragma unroll
-    for (int j = 0; j < MPW; j++) {
-        const int q = min(min(warp + 8 * j, M1T - 1) * 16 + lrow, NR1 - 1);
-        rowCell[j] = (q / R1) * RI + q % R1;
-    }
-    // weights: lanes address rows n (two column tiles per ldmatrix)
     const int wrow = (lane & 7) + ((lane >> 4) << 3), wk = ((lane >> 3) & 1) * 8;
-    float acc[MPW][4][4] = {};
-#pragma unroll 1
+    const int half = warp & 1, mt0 = warp >> 1;
+    int cell[UPW];
+#pragma unroll
+    for (int j = 0; j < UPW; j++) cell[j] = S.qcell[min(mt0 + WPH * j, M1T - 1) * 16 + lrow];
+    const uint16_t* wp = &S.w1[(half * 16 + wrow) * SW1 + wk];
+    float acc[UPW][2][4] = {};
+#pragma unroll 13
     for (int ks = 0; ks < K1B / 16; ks++) {
-        uint32_t bw[4][2];
-#pragma unroll
-        for (int np = 0; np < 2; np++) {
-            uint32_t r[4];
-            ldsm4(r, &S.w1[(np * 16 + wrow) * SW1 + ks * 16 + wk]);
-            bw[2 * np][0] = r[0];
-            bw[2 * np][1] = r[1];
-            bw[2 * np + 1][0] = r[2];
-            bw[2 * np + 1][1] = r[3];
-        }
         const int toff = S.toff[2 * ks + lhalf];
+        uint32_t b[4];
+        ldsm4(b, wp + ks * 16);
 #pragma unroll
-        for (int j = 0; j < MPW; j++) {
-            if (j == MPW - 1 && !third) break;
+        for (int j = 0; j < UPW; j++) {
+            if (mt0 + WPH * j >= M1T) break;
             uint32_t a[4];
-            ldsm4(a, &S.xb[(rowCell[j] + toff) * CB]);
-            // ldmatrix order: rows 0-7 tap A, rows 8-15 tap A, rows 0-7 tap B, rows 8-15 tap B
-#pragma unroll
-            for (int nt = 0; nt < 4; nt++) mma16816(acc[j][nt], a, bw[nt][0], bw[nt][1]);
+            ldsm4(a, &S.xb[(cell[j] + toff) * CB]);
+            mma16816(acc[j][0], a, b[0], b[1]);
+            mma16816(acc[j][1], a, b[2], b[3]);
         }
     }
     const float bref = S.bref;
 #pragma unroll
-    for (int j = 0; j < MPW; j++) {
-        const int mt = warp + 8 * j;
-        if (mt >= M1T) break;
-        const int r0 = mt * 16 + g, r1 = r0 + 8;
-        const float c0 = winBed(S, winBase(min(r0, NR1 - 1))) - bref;
-        const float c1 = winBed(S, winBase(min(r1, NR1 - 1))) - bref;
+    for (int j = 0; j < UPW; j++) {
+        if (mt0 + WPH * j >= M1T) break;
+        const int r0 = (mt0 + WPH * j) * 16 + g, r1 = r0 + 8;
+        const float c0 = S.xbed[S.qcell[r0] + 2 * RI + 2] - bref;
+        const float c1 = S.xbed[S.qcell[r1] + 2 * RI + 2] - bref;
 #pragma unroll
-        for (int nt = 0; nt < 4; nt++) {
-            const int o = nt * 8 + 2 * t;
+        for (int nt = 0; nt < 2; nt++) {
+            const int o = half * 16 + nt * 8 + 2 * t;
             const float s0 = S.sbed[o], s1 = S.sbed[o + 1];
             if (r0 < NR1)
                 st32(&S.a1[r0 * SA + o], pack2(relu(acc[j][nt][0] + S.b1[o] - c0 * s0),
@@ -269,69 +259,55 @@ __device__ void conv1(NetSmem& S, int warp, int lane) {
     }
 }
 
-// Layers 2 and 3 on output rows warp and warp+8 (one weight fragment load
-// for both; A and B fragments by ldmatrix).  z2: layer-2 pre-activations
-// (accumulator fragments); out[m]: layer-3 outputs of rows g and g+8 of
-// output row warp+8m, channels 2t and 2t+1 (t < 2 valid).
-__device__ void conv23(const NetSmem& S, int warp, int lane, float z2[2][4][4], float out[2][4]) {
+// Layers 2 and 3 on output row `warp` (A and B fragments by ldmatrix).  z2:
+// layer-2 pre-activations (accumulator fragments); out: layer-3 outputs of rows
+// g and g+8, channels 2t and 2t+1 (t < 2 valid).
+__device__ __forceinline__ void conv23(const TrainSmem& S, int warp, int lane, float z2[4][4], float out[4]) {
     const int g = lane >> 2, t = lane & 3;
     const int lrow = lane & 15, lk = (lane >> 4) * 8;  // A: row, k offset of this lane's address
     const int wrow = (lane & 7) + ((lane >> 4) << 3), wk = ((lane >> 3) & 1) * 8;
-    float acc[2][4][4] = {};
-#pragma unroll 1
+    float acc[4][4] = {};
+#pragma unroll 3
     for (int tap = 0; tap < 9; tap++) {
         const int dy = tap / 3, dx = tap % 3;
-        const uint16_t* p0 = &S.a1[((warp + dy) * R1 + lrow + dx) * SA + lk];
-        const uint16_t* p1 = p0 + 8 * R1 * SA;
+        const uint16_t* p = &S.a1[((warp + dy) * R1 + lrow + dx) * SA + lk];
 #pragma unroll
         for (int kb = 0; kb < 2; kb++) {
             const int kk = tap * 32 + kb * 16;
-            uint32_t bw[4][2];
-#pragma unroll
-            for (int np = 0; np < 2; np++) {
-                uint32_t r[4];
-                ldsm4(r, &S.w2[(np * 16 + wrow) * SW2 + kk + wk]);
-                bw[2 * np][0] = r[0];
-                bw[2 * np][1] = r[1];
-                bw[2 * np + 1][0] = r[2];
-                bw[2 * np + 1][1] = r[3];
-            }
-#pragma unroll
-            for (int m = 0; m < 2; m++) {
-                uint32_t a[4];
-                ldsm4(a, (m ? p1 : p0) + kb * 16);
-#pragma unroll
-                for (int nt = 0; nt < 4; nt++) mma16816(acc[m][nt], a, bw[nt][0], bw[nt][1]);
-            }
+            uint32_t a[4], b0[4], b1[4];
+            ldsm4(b0, &S.w2[wrow * SW2 + kk + wk]);
+            ldsm4(b1, &S.w2[(16 + wrow) * SW2 + kk + wk]);
+            ldsm4(a, p + kb * 16);
+            mma16816(acc[0], a, b0[0], b0[1]);
+            mma16816(acc[1], a, b0[2], b0[3]);
+            mma16816(acc[2], a, b1[0], b1[1]);
+            mma16816(acc[3], a, b1[2], b1[3]);
         }
     }
 #pragma unroll
-    for (int m = 0; m < 2; m++) {
-#pragma unroll
-        for (int nt = 0; nt < 4; nt++) {
-            const int o = nt * 8 + 2 * t;
-            z2[m][nt][0] = acc[m][nt][0] + S.b2[o];
-            z2[m][nt][1] = acc[m][nt][1] + S.b2[o + 1];
-            z2[m][nt][2] = acc[m][nt][2] + S.b2[o];
-            z2[m][nt][3] = acc[m][nt][3] + S.b2[o + 1];
-        }
-        float acc3[4] = {};
-#pragma unroll
-        for (int kb = 0; kb < 2; kb++) {
-            uint32_t a[4];
-            a[0] = pack2(relu(z2[m][2 * kb][0]), relu(z2[m][2 * kb][1]));
-            a[1] = pack2(relu(z2[m][2 * kb][2]), relu(z2[m][2 * kb][3]));
-            a[2] = pack2(relu(z2[m][2 * kb + 1][0]), relu(z2[m][2 * kb + 1][1]));
-            a[3] = pack2(relu(z2[m][2 * kb + 1][2]), relu(z2[m][2 * kb + 1][3]));
-            const uint16_t* w = &S.w3[g * SW3 + kb * 16 + 2 * t];
-            mma16816(acc3, a, ld32(w), ld32(w + 8));
-        }
-        const int c = 2 * t;  // b3 holds 8 entries, zero past the fourth
-        out[m][0] = acc3[0] + S.b3[c];
-        out[m][1] = acc3[1] + S.b3[c + 1];
-        out[m][2] = acc3[2] + S.b3[c];
-        out[m][3] = acc3[3] + S.b3[c + 1];
+    for (int nt = 0; nt < 4; nt++) {
+        const int o = nt * 8 + 2 * t;
+        z2[nt][0] = acc[nt][0] + S.b2[o];
+        z2[nt][1] = acc[nt][1] + S.b2[o + 1];
+        z2[nt][2] = acc[nt][2] + S.b2[o];
+        z2[nt][3] = acc[nt][3] + S.b2[o + 1];
     }
+    float acc3[4] = {};
+#pragma unroll
+    for (int kb = 0; kb < 2; kb++) {
+        uint32_t a[4];
+        a[0] = pack2(relu(z2[2 * kb][0]), relu(z2[2 * kb][1]));
+        a[1] = pack2(relu(z2[2 * kb][2]), relu(z2[2 * kb][3]));
+        a[2] = pack2(relu(z2[2 * kb + 1][0]), relu(z2[2 * kb + 1][1]));
+        a[3] = pack2(relu(z2[2 * kb + 1][2]), relu(z2[2 * kb + 1][3]));
+        const uint16_t* w = &S.w3[g * SW3 + kb * 16 + 2 * t];
+        mma16816(acc3, a, ld32(w), ld32(w + 8));
+    }
+    const int c = 2 * t;  // b3 holds 8 entries, zero past the fourth
+    out[0] = acc3[0] + S.b3[c];
+    out[1] = acc3[1] + S.b3[c + 1];
+    out[2] = acc3[2] + S.b3[c];
+    out[3] = acc3[3] + S.b3[c + 1];
 }
 
 struct TileGeom {
@@ -923,45 +899,64 @@ struct TrainArgs {
     double* loss;
 };
 
-__global__ void __launch_bounds__(NT, 1) k_train(TrainArgs A) {
+// One CTA of 16 warps per SM.  Every contraction is a GEMM on mma.sync whose
+// fragments all come by ldmatrix: where an operand lies transposed (the weight
+// gradients reduce over cells, the activation gradient over output channels),
+// by its .trans form, so nothing is staged twice.  The layer-1 weight gradient
+// takes its inputs from the BF16 cells of the forward pass; only the bed, which
+// enters relative to each window's centre, is formed again from FP32.
+// What bounds it: @TRAIN@
+__global__ void __launch_bounds__(TT, 1) k_train(TrainArgs A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    TrainSmem& T = *reinterpret_cast<TrainSmem*>(smem_raw);
-    NetSmem& S = T.n;
+    TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
     const rift_closure_src& src = A.src;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    stageNet(S, A.P);
-    for (int i = tid; i < K2 * SA; i += NT) {
-        int k = i / SA, o = i % SA;
-        T.w2t[i] = bf(o < C1 ? A.P[OFF_W2 + o * K2 + k] : 0.f);
-    }
-    for (int i = tid; i < 4 * C1; i += NT) T.w3f[i] = A.P[OFF_W3 + i];
-
-    // gradient accumulators held across tiles
-    float gW2[9][4] = {};   // layer-2 weight tiles (rows k, cols o), see w2Tile
-    float gW1[5][4] = {};   // layer-1 weight tiles, see w1Tile
-    float gW3 = 0.f, gB3 = 0.f, gB2 = 0.f, gB1 = 0.f;
-    double lossAcc = 0.0;
-
+    // lane addresses of the fragment loads: rows of an A operand, of a
+    // transposed A operand, of a transposed B operand
+    const int lrow = lane & 15, lk = (lane >> 4) * 8;
+    const int tr = (lane & 7) + (lane >> 4) * 8, tc = ((lane >> 3) & 1) * 8;  // A^T: k row, m column
+    const int br = (lane & 7) + ((lane >> 3) & 1) * 8, bc = (lane >> 4) * 8;   // B^T: k row, n column
+    TrainInput R;
     const int ntile = tileCount(src);
+    if ((int)blockIdx.x < ntile) {
+        const TileGeom G0 = tileGeom(src, blockIdx.x);
+        loadInput(R, src, G0.s, G0.Y - 3, G0.X - 3);
+    }
+    stageNet(S, A.P);
+
+    // gradient accumulators held across tiles.  Layer 2: row tile `warp` of 18
+    // (16 k each) with every column tile, and of tiles 16 and 17 one column
+    // tile each on warps 0..7.  Layer 1: over half of the cells, taps 4 p ..
+    // 4 p + 3 of the BF16 channels on warp pair p = 0..6, the bed's 25 taps on
+    // the last pair; the two row tiles of a warp share their B fragments.
+    float gW2[5][4] = {}, gW1[2][4][4] = {};
+    const bool bed = warp >= 14;
+    const int toff0 = CB * tapCell((warp >> 1) * 4 + (tc >> 3));
+    const int toff1 = CB * tapCell((warp >> 1) * 4 + 2 + (tc >> 3));
+    float gW3 = 0.f, gB3[COUT] = {}, gB2 = 0.f, gB1 = 0.f;
+    double lossAcc = 0.0;
+    const int mtX = 16 + ((warp >> 2) & 1), ntX = warp & 3;  // the extra layer-2 tile
+
     for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
         const TileGeom G = tileGeom(src, tile);
         __syncthreads();
-        stageInput(S, src, G.s, G.Y - 3, G.X - 3);
+        storeInput(S, R, src);
+        if (tile + (int)gridDim.x < ntile) {
+            const TileGeom Gn = tileGeom(src, tile + gridDim.x);
+            loadInput(R, src, Gn.s, Gn.Y - 3, Gn.X - 3);
+        }
         __syncthreads();
         conv1(S, warp, lane);
         __syncthreads();
-        float z2[2][4][4], o[2][4];
-        conv23(S, warp, lane, z2, o);
-
-        // loss and d loss / d out; layer-2 activations to shared memory
-#pragma unroll
-        for (int m = 0; m < 2; m++) {
-            const int oy = warp + 8 * m;
+        {
+            float z2[4][4], o[4];
+            conv23(S, warp, lane, z2, o);
+            // loss and d loss / d out; layer-2 activations to shared memory
 #pragma unroll
             for (int r = 0; r < 2; r++) {
-                const int ox = g + 8 * r, p = oy * OT + ox;
+                const int ox = g + 8 * r, p = warp * OT + ox;
                 if (t < 2) {
-                    const int y = G.Y + oy - src.oy0, x = G.X + ox - src.ox0;
+                    const int y = G.Y + warp - src.oy0, x = G.X + ox - src.ox0;
                     const bool in = y < src.OH && x < src.OW;
 #pragma unroll
                     for (int e = 0; e < 2; e++) {
@@ -970,203 +965,230 @@ __global__ void __launch_bounds__(NT, 1) k_train(TrainArgs A) {
                         if (in) {
                             size_t at = (((size_t)G.s * COUT + ch) * src.OH + y) * src.OW + x;
                             float w = __ldg(A.weight + at);
-                            float diff = o[m][2 * r + e] - __ldg(A.target + at);
+                            float diff = o[2 * r + e] - __ldg(A.target + at);
                             lossAcc += (double)(w * diff * diff);
                             d = 2.f * w * diff * A.lossScale;
                         }
-                        T.dout[p * 4 + ch] = d;
+                        S.dout[p * 4 + ch] = d;
                     }
                 }
 #pragma unroll
                 for (int nt = 0; nt < 4; nt++)
-                    st32(&T.a2[p * SA + nt * 8 + 2 * t],
-                         pack2(relu(z2[m][nt][2 * r]), relu(z2[m][nt][2 * r + 1])));
+                    st32(&S.a2[p * SA + nt * 8 + 2 * t], pack2(relu(z2[nt][2 * r]), relu(z2[nt][2 * r + 1])));
             }
         }
         __syncthreads();
         // layer 3: dW3, db3 (CUDA cores)
         {
-            const int pr = tid & 127, half = tid >> 7, oc = pr >> 5, c = pr & 31;
+            const int oc = (tid >> 5) & 3, c = lane, part = tid >> 7;
             float acc = 0.f;
-            for (int p = half * 128; p < half * 128 + 128; p++) acc += T.dout[p * 4 + oc] * fb(T.a2[p * SA + c]);
-            gW3 += acc;
-            if (tid < COUT) {
-                float b = 0.f;
-                for (int p = 0; p < OT * OT; p++) b += T.dout[p * 4 + tid];
-                gB3 += b;
-            }
-        }
-        __syncthreads();
-        // dZ2 = (W3^T dout) * relu'(z2), in place of a2
-        {
-            const int p = tid;
-            const float d0 = T.dout[p * 4], d1 = T.dout[p * 4 + 1], d2 = T.dout[p * 4 + 2],
-                        d3 = T.dout[p * 4 + 3];
 #pragma unroll 8
-            for (int c = 0; c < C1; c++) {
-                float a = fb(T.a2[p * SA + c]);
-                float v = d0 * T.w3f[c] + d1 * T.w3f[C1 + c] + d2 * T.w3f[2 * C1 + c] + d3 * T.w3f[3 * C1 + c];
-                T.a2[p * SA + c] = bf(a > 0.f ? v : 0.f);
+            for (int p = part * 64; p < part * 64 + 64; p++) acc += S.dout[p * 4 + oc] * fb(S.a2[p * SA + c]);
+            gW3 += acc;
+            if (tid < OT * OT) {
+                const float4 d = *reinterpret_cast<const float4*>(&S.dout[tid * 4]);
+                float v[COUT] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+                for (int k = 0; k < COUT; k++) {
+                    for (int s = 16; s > 0; s >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], s);
+                    gB3[k] += v[k];
+                }
             }
         }
         __syncthreads();
+        // dZ2 = (W3^T dout) * relu'(z2), in place of a2: 16 channels per thread
         {
-            const int c = tid & 31, part = tid >> 5;
+            const int p = tid >> 1, c0 = (tid & 1) * 16;
+            const float4 d = *reinterpret_cast<const float4*>(&S.dout[p * 4]);
+            uint4* z = reinterpret_cast<uint4*>(&S.a2[p * SA + c0]);
+            uint32_t q[8];
+            *reinterpret_cast<uint4*>(&q[0]) = z[0];
+            *reinterpret_cast<uint4*>(&q[4]) = z[1];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                float v[2];
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const float4 w = *reinterpret_cast<const float4*>(S.w3q[c0 + 2 * k + e]);
+                    const float a = fb((uint16_t)(q[k] >> (16 * e)));
+                    const float x = d.x * w.x + d.y * w.y + d.z * w.z + d.w * w.w;
+                    v[e] = a > 0.f ? x : 0.f;
+                }
+                q[k] = pack2(v[0], v[1]);
+            }
+            z[0] = *reinterpret_cast<uint4*>(&q[0]);
+            z[1] = *reinterpret_cast<uint4*>(&q[4]);
+        }
+        __syncthreads();
+        {
             float b = 0.f;
-            for (int p = part; p < OT * OT; p += 8) b += fb(T.a2[p * SA + c]);
+#pragma unroll 8
+            for (int p = warp; p < OT * OT; p += TT / 32) b += fb(S.a2[p * SA + lane]);
             gB2 += b;
         }
-        // dW2[k][o] += sum_p a1[p + tap(k)][ch(k)] dZ2[p][o]: 18 x 4 MMA tiles,
-        // nine per warp (rows w and w+8 with every column tile, then one of
-        // the rows 16..17)
-#pragma unroll 1
-        for (int oyp = 0; oyp < OT; oyp++) {
-            uint32_t bfr[4][2];
-#pragma unroll
-            for (int nt = 0; nt < 4; nt++) {
-                const uint16_t* d = &T.a2[(oyp * OT + 2 * t) * SA + nt * 8 + g];
-                bfr[nt][0] = pack16(d[0], d[SA]);
-                bfr[nt][1] = pack16(d[8 * SA], d[9 * SA]);
-            }
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                const int mt = j < 2 ? warp + 8 * j : 16 + (warp >> 2);
-                const int tap = mt >> 1, ch = (mt & 1) * 16 + g, dy = tap / 3, dx = tap % 3;
-                const uint16_t* r = &S.a1[((oyp + dy) * R1 + 2 * t + dx) * SA + ch];
-                uint32_t a[4];
-                a[0] = pack16(r[0], r[SA]);
-                a[1] = pack16(r[8], r[SA + 8]);
-                a[2] = pack16(r[8 * SA], r[9 * SA]);
-                a[3] = pack16(r[8 * SA + 8], r[9 * SA + 8]);
-                if (j < 2) {
-#pragma unroll
-                    for (int nt = 0; nt < 4; nt++) mma16816(gW2[4 * j + nt], a, bfr[nt][0], bfr[nt][1]);
-                } else {
-                    const int nt = warp & 3;
-                    mma16816(gW2[8], a, bfr[nt][0], bfr[nt][1]);
+        // dW2[k][o] += sum_p a1[p + tap(k)][ch(k)] dZ2[p][o]
+        {
+            const int tap = warp >> 1, tapX = mtX >> 1;
+            const uint16_t* pa = &S.a1[((tap / 3) * R1 + tap % 3 + tr) * SA + (warp & 1) * 16 + tc];
+            const uint16_t* px = &S.a1[((tapX / 3) * R1 + tapX % 3 + tr) * SA + (mtX & 1) * 16 + tc];
+            const uint16_t* pb = &S.a2[br * SA + bc];
+#pragma unroll 4
+            for (int oyp = 0; oyp < OT; oyp++) {
+                uint32_t a[4], b0[4], b1[4];
+                ldsm4t(b0, pb + oyp * OT * SA);
+                ldsm4t(b1, pb + oyp * OT * SA + 16);
+                ldsm4t(a, pa + oyp * R1 * SA);
+                mma16816(gW2[0], a, b0[0], b0[1]);
+                mma16816(gW2[1], a, b0[2], b0[3]);
+                mma16816(gW2[2], a, b1[0], b1[1]);
+                mma16816(gW2[3], a, b1[2], b1[3]);
+                if (warp < 8) {
+                    ldsm4t(a, px + oyp * R1 * SA);
+                    const uint32_t x0 = ntX & 2 ? (ntX & 1 ? b1[2] : b1[0]) : (ntX & 1 ? b0[2] : b0[0]);
+                    const uint32_t x1 = ntX & 2 ? (ntX & 1 ? b1[3] : b1[1]) : (ntX & 1 ? b0[3] : b0[1]);
+                    mma16816(gW2[4], a, x0, x1);
                 }
             }
         }
         __syncthreads();
         // dA1[q][c] = sum_{tap,o} dZ2[q - tap][o] W2[o][tap*32 + c]; dZ1 = dA1 * relu'(z1),
         // written over a1 (each element read and written by the same thread)
-        for (int mt = warp; mt < M1T; mt += NT / 32) {
-            const int q0 = mt * 16 + g, q1 = q0 + 8;
-            const int qy0 = q0 / R1, qx0 = q0 % R1, qy1 = q1 / R1, qx1 = q1 % R1;
-            float acc[4][4] = {};
-#pragma unroll 1
+        {
+            const int half = warp & 1, mt0 = warp >> 1;
+            int qy[UPW], qx[UPW];
+#pragma unroll
+            for (int j = 0; j < UPW; j++) {
+                const int q = (mt0 + WPH * j) * 16 + lrow;
+                qy[j] = q < NR1 ? q / R1 : -OT;  // (a row past the region: outside for every tap)
+                qx[j] = q % R1;
+            }
+            const uint16_t* wp = &S.w2[br * SW2 + half * 16 + bc];
+            float acc[UPW][2][4] = {};
+#pragma unroll 3
             for (int tap = 0; tap < 9; tap++) {
                 const int dy = tap / 3, dx = tap % 3;
-                const int py0 = qy0 - dy, px0 = qx0 - dx, py1 = qy1 - dy, px1 = qx1 - dx;
-                const bool v0 = q0 < NR1 && py0 >= 0 && py0 < OT && px0 >= 0 && px0 < OT;
-                const bool v1 = q1 < NR1 && py1 >= 0 && py1 < OT && px1 >= 0 && px1 < OT;
-                const uint16_t* d0 = &T.a2[(v0 ? py0 * OT + px0 : 0) * SA + 2 * t];
-                const uint16_t* d1 = &T.a2[(v1 ? py1 * OT + px1 : 0) * SA + 2 * t];
+                uint32_t b[2][4];
+                ldsm4t(b[0], wp + tap * 32);
+                ldsm4t(b[1], wp + 16 * SW2 + tap * 32);
 #pragma unroll
-                for (int ob = 0; ob < 2; ob++) {
-                    uint32_t a[4];
-                    a[0] = v0 ? ld32(d0 + ob * 16) : 0u;
-                    a[1] = v1 ? ld32(d1 + ob * 16) : 0u;
-                    a[2] = v0 ? ld32(d0 + ob * 16 + 8) : 0u;
-                    a[3] = v1 ? ld32(d1 + ob * 16 + 8) : 0u;
+                for (int j = 0; j < UPW; j++) {
+                    if (mt0 + WPH * j >= M1T) break;
+                    const int py = qy[j] - dy, px = qx[j] - dx;
+                    const bool in = (unsigned)py < (unsigned)OT && (unsigned)px < (unsigned)OT;
+                    const uint16_t* d = (in ? &S.a2[(py * OT + px) * SA] : S.zero) + lk;
 #pragma unroll
-                    for (int nt = 0; nt < 4; nt++) {
-                        const uint16_t* w = &T.w2t[(tap * 32 + nt * 8 + g) * SA + ob * 16 + 2 * t];
-                        mma16816(acc[nt], a, ld32(w), ld32(w + 8));
+                    for (int ob = 0; ob < 2; ob++) {
+                        uint32_t a[4];
+                        ldsm4(a, d + ob * 16);
+                        mma16816(acc[j][0], a, b[ob][0], b[ob][1]);
+                        mma16816(acc[j][1], a, b[ob][2], b[ob][3]);
                     }
                 }
             }
 #pragma unroll
-            for (int nt = 0; nt < 4; nt++) {
-                const int c = nt * 8 + 2 * t;
-                if (q0 < NR1) {
-                    uint16_t* z = &S.a1[q0 * SA + c];
-                    st32(z, pack2(fb(z[0]) > 0.f ? acc[nt][0] : 0.f, fb(z[1]) > 0.f ? acc[nt][1] : 0.f));
-                }
-                if (q1 < NR1) {
-                    uint16_t* z = &S.a1[q1 * SA + c];
-                    st32(z, pack2(fb(z[0]) > 0.f ? acc[nt][2] : 0.f, fb(z[1]) > 0.f ? acc[nt][3] : 0.f));
+            for (int j = 0; j < UPW; j++) {
+                if (mt0 + WPH * j >= M1T) break;
+                const int q0 = (mt0 + WPH * j) * 16 + g, q1 = q0 + 8;
+#pragma unroll
+                for (int nt = 0; nt < 2; nt++) {
+                    const int c = half * 16 + nt * 8 + 2 * t;
+                    if (q0 < NR1) {
+                        uint16_t* z = &S.a1[q0 * SA + c];
+                        st32(z, pack2(fb(z[0]) > 0.f ? acc[j][nt][0] : 0.f, fb(z[1]) > 0.f ? acc[j][nt][1] : 0.f));
+                    }
+                    if (q1 < NR1) {
+                        uint16_t* z = &S.a1[q1 * SA + c];
+                        st32(z, pack2(fb(z[0]) > 0.f ? acc[j][nt][2] : 0.f, fb(z[1]) > 0.f ? acc[j][nt][3] : 0.f));
+                    }
                 }
             }
         }
         __syncthreads();
         {
-            const int c = tid & 31, part = tid >> 5;
             float b = 0.f;
-            for (int q = part; q < NR1; q += 8) b += fb(S.a1[q * SA + c]);
+#pragma unroll 4
+            for (int q = warp; q < NR1; q += TT / 32) b += fb(S.a1[q * SA + lane]);
             gB1 += b;
         }
-        // dW1[k][o] += sum_q x(q, k) dZ1[q][o]: 10 x 4 MMA tiles, five per warp
-        {
-            const int mtA = warp, mtB = 8 + (warp >> 2), ntB = warp & 3;
-            const int eA0 = S.koffE[mtA * 16 + g], eA1 = S.koffE[mtA * 16 + g + 8];
-            const int eB0 = S.koffE[mtB * 16 + g], eB1 = S.koffE[mtB * 16 + g + 8];
-#pragma unroll 1
-            for (int ks = 0; ks < M1T; ks++) {
-                int bs[4];
-                float bc[4];
-                uint16_t dz[4][4];
+        // dW1[k][o] += sum_q x(q, k) dZ1[q][o]
+#pragma unroll 2
+        for (int ks = warp & 1; ks < M1T; ks += 2) {
+            uint32_t a[2][4], b0[4], b1[4];
+            const int qb = ks * 16 + br;
+            const uint16_t* pb = (qb < NR1 ? &S.a1[qb * SA] : S.zero) + bc;
+            ldsm4t(b0, pb);
+            ldsm4t(b1, pb + 16);
+            if (!bed) {
+                const uint16_t* px = &S.xb[S.qcell[ks * 16 + tr] * CB];
+                ldsm4t(a[0], px + toff0);
+                ldsm4t(a[1], px + toff1);
+            } else {
+                float x[4][4];  // this thread's taps g, g + 8, g + 16 and g + 24
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int q = ks * 16 + 2 * t + (u & 1) + 8 * (u >> 1);
-                    bs[u] = winBase(min(q, NR1 - 1));
-                    bc[u] = winBed(S, bs[u]);
+                for (int u = 0; u < 4; u++) {  // cells 2t, 2t + 1, 2t + 8, 2t + 9
+                    const int cell = S.qcell[ks * 16 + 2 * t + (u & 1) + 8 * (u >> 1)];
+                    const float mid = S.xbed[cell + 2 * RI + 2];
 #pragma unroll
-                    for (int nt = 0; nt < 4; nt++) dz[u][nt] = q < NR1 ? S.a1[q * SA + nt * 8 + g] : (uint16_t)0;
+                    for (int r = 0; r < 3; r++) x[r][u] = S.xbed[cell + S.toff[g + 8 * r]] - mid;
+                    x[3][u] = g == 0 ? S.xbed[cell + 4 * RI + 4] - mid : 0.f;
                 }
-                uint32_t a[4];
-                a[0] = pack2(featElem(S, bs[0], bc[0], eA0), featElem(S, bs[1], bc[1], eA0));
-                a[1] = pack2(featElem(S, bs[0], bc[0], eA1), featElem(S, bs[1], bc[1], eA1));
-                a[2] = pack2(featElem(S, bs[2], bc[2], eA0), featElem(S, bs[3], bc[3], eA0));
-                a[3] = pack2(featElem(S, bs[2], bc[2], eA1), featElem(S, bs[3], bc[3], eA1));
 #pragma unroll
-                for (int nt = 0; nt < 4; nt++)
-                    mma16816(gW1[nt], a, pack16(dz[0][nt], dz[1][nt]), pack16(dz[2][nt], dz[3][nt]));
-                a[0] = pack2(featElem(S, bs[0], bc[0], eB0), featElem(S, bs[1], bc[1], eB0));
-                a[1] = pack2(featElem(S, bs[0], bc[0], eB1), featElem(S, bs[1], bc[1], eB1));
-                a[2] = pack2(featElem(S, bs[2], bc[2], eB0), featElem(S, bs[3], bc[3], eB0));
-                a[3] = pack2(featElem(S, bs[2], bc[2], eB1), featElem(S, bs[3], bc[3], eB1));
-                mma16816(gW1[4], a, pack16(dz[0][ntB], dz[1][ntB]), pack16(dz[2][ntB], dz[3][ntB]));
+                for (int m = 0; m < 2; m++) {
+                    a[m][0] = pack2(x[2 * m][0], x[2 * m][1]);
+                    a[m][1] = pack2(x[2 * m + 1][0], x[2 * m + 1][1]);
+                    a[m][2] = pack2(x[2 * m][2], x[2 * m][3]);
+                    a[m][3] = pack2(x[2 * m + 1][2], x[2 * m + 1][3]);
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+                mma16816(gW1[m][0], a[m], b0[0], b0[1]);
+                mma16816(gW1[m][1], a[m], b0[2], b0[3]);
+                mma16816(gW1[m][2], a[m], b1[0], b1[1]);
+                mma16816(gW1[m][3], a[m], b1[2], b1[3]);
             }
         }
     }
 
     // one addition per CTA of every gradient it holds
 #pragma unroll
-    for (int j = 0; j < 9; j++) {
-        const int mt = j < 8 ? warp + 8 * (j >> 2) : 16 + (warp >> 2);
-        const int nt = j < 8 ? (j & 3) : (warp & 3);
+    for (int j = 0; j < 5; j++) {
+        if (j == 4 && warp >= 8) break;
+        const int mt = j < 4 ? warp : mtX, nt = j < 4 ? j : ntX;
         const int k0 = mt * 16 + g, o0 = nt * 8 + 2 * t;
         atomicAdd(&A.grad[OFF_W2 + o0 * K2 + k0], gW2[j][0]);
         atomicAdd(&A.grad[OFF_W2 + (o0 + 1) * K2 + k0], gW2[j][1]);
         atomicAdd(&A.grad[OFF_W2 + o0 * K2 + k0 + 8], gW2[j][2]);
         atomicAdd(&A.grad[OFF_W2 + (o0 + 1) * K2 + k0 + 8], gW2[j][3]);
     }
+    {
+        // the two rows of a fragment: channel g of two taps (h, hu, hv, -, -, n,
+        // rain, -), or the bed of two taps
+        const int c = bed ? 3 : g < 3 ? g : g == 5 ? 4 : g == 6 ? 5 : -1;
 #pragma unroll
-    for (int j = 0; j < 5; j++) {
-        const int mt = j < 4 ? warp : 8 + (warp >> 2);
-        const int nt = j < 4 ? j : (warp & 3);
-        const int k0 = mt * 16 + g, o0 = nt * 8 + 2 * t;
-        if (k0 < K1) {
-            atomicAdd(&A.grad[OFF_W1 + o0 * K1P + k0], gW1[j][0]);
-            atomicAdd(&A.grad[OFF_W1 + (o0 + 1) * K1P + k0], gW1[j][1]);
-        }
-        if (k0 + 8 < K1) {
-            atomicAdd(&A.grad[OFF_W1 + o0 * K1P + k0 + 8], gW1[j][2]);
-            atomicAdd(&A.grad[OFF_W1 + (o0 + 1) * K1P + k0 + 8], gW1[j][3]);
+        for (int r = 0; r < 4; r++) {
+            const int tap = bed ? g + 8 * r : (warp >> 1) * 4 + r;
+            if (c < 0 || tap >= 25) continue;
+#pragma unroll
+            for (int nt = 0; nt < 4; nt++) {
+                const int o0 = nt * 8 + 2 * t, k = tap * CIN + c;
+                atomicAdd(&A.grad[OFF_W1 + o0 * K1P + k], gW1[r >> 1][nt][2 * (r & 1)]);
+                atomicAdd(&A.grad[OFF_W1 + (o0 + 1) * K1P + k], gW1[r >> 1][nt][2 * (r & 1) + 1]);
+            }
         }
     }
     atomicAdd(&A.grad[OFF_W3 + (tid & 127)], gW3);
-    if (tid < COUT) atomicAdd(&A.grad[OFF_B3 + tid], gB3);
-    atomicAdd(&A.grad[OFF_B2 + (tid & 31)], gB2);
-    atomicAdd(&A.grad[OFF_B1 + (tid & 31)], gB1);
+    if (tid < OT * OT && lane == 0)
+        for (int k = 0; k < COUT; k++) atomicAdd(&A.grad[OFF_B3 + k], gB3[k]);
+    atomicAdd(&A.grad[OFF_B2 + lane], gB2);
+    atomicAdd(&A.grad[OFF_B1 + lane], gB1);
     // loss: warp sums, then one atomic per CTA
     for (int s = 16; s > 0; s >>= 1) lossAcc += __shfl_xor_sync(0xffffffffu, lossAcc, s);
-    if (lane == 0) T.red[warp] = lossAcc;
+    if (lane == 0) S.red[warp] = lossAcc;
     __syncthreads();
     if (tid == 0) {
         double s = 0.0;
-        for (int w = 0; w < NT / 32; w++) s += T.red[w];
+        for (int w = 0; w < TT / 32; w++) s += S.red[w];
         atomicAdd(A.loss, s * (double)A.lossScale);
     }
 }
@@ -1479,7 +1501,7 @@ int rift_closure_train(const rift_closure_src* src, const float* params, const f
     int grid = 0, rc_;
     if ((rc_ = onePerSM((const void*)rc::k_train, smem, tiles, &grid))) return rc_;
     rc::TrainArgs A{*src, params, target, weight, loss_scale, grad, loss};
-    rc::k_train<<<grid, rc::NT, smem, (cudaStream_t)stream>>>(A);
+    rc::k_train<<<grid, rc::TT, smem, (cudaStream_t)stream>>>(A);
     return launched("k_train");
 }
 
