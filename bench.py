@@ -267,17 +267,18 @@ def run_ours(args, device=0, sync=None):
     active_rate = active_cells / (ms * 1e-3)
     peak, peak_kind = peaks()
     bytes_per = 4 * WORDS[cfg]
-    if persist_steps > 0 and graph_steps == 0:
+    one_launch = persist_steps > 0 and graph_steps == 0
+    if one_launch:
         # one cooperative launch ran every timed step: the kernel is the step
         kernel = ("k_persist (whole step in one cooperative launch: grow, speeds + dt, "
                   "RK stages 1+2)")
         achieved = active_cells * bytes_per / (ms * 1e-3) / 1e9
-        launches = 1
+        launches = 3  # the loop, and the kernels that bring its state and take it back
     else:
         kernel = ("RK stages 1+2 (k_march<1>, k_update1, k_march<2> or k_stage<1>, k_stage<2>; one "
                   "schedule runs, the other exits at entry)")
         achieved = stage_cells * bytes_per / (stage_ms * 1e-3) / 1e9 if stage_ms > 0 else None
-        launches = graph_steps * launches_per_step(case.flags) + (1 if persist_steps else 0)
+        launches = graph_steps * launches_per_step(case.flags) + (3 if persist_steps else 0)
     # DRAM bytes (read + write) of the reported kernel per launch, from the
     # ncu capture summarised under profiles/ (per step there)
     traffic = None
@@ -285,8 +286,8 @@ def run_ours(args, device=0, sync=None):
     if os.path.exists(prof) and args.N is None:
         try:
             rec = json.load(open(prof))
-            if rec.get("kernel") == ("k_persist" if launches == 1 else "stages"):
-                traffic = rec["bytes_per_step"] * (steps if launches == 1 else 1)
+            if rec.get("kernel") == ("k_persist" if one_launch else "stages"):
+                traffic = rec["bytes_per_step"] * (steps if one_launch else 1)
         except Exception:
             traffic = None
     line = {

@@ -1099,10 +1099,11 @@ bool useFlow(const rift_handle* h) {
     return h->flowOk && !h->has(RIFT_F_EULER) && h->hst->nActive > h->gridPersist;
 }
 
-// One cooperative launch of the chosen loop (also under capture).
-cudaError_t enqueuePersist(rift_handle* h, int nsteps) {
-    cudaError_t e = cudaMemsetAsync(h->gbar, 0, GRIDBAR_CLEAR, h->stream);
-    if (e != cudaSuccess) return e;
+// One cooperative launch of the chosen loop (also under capture), with the
+// device state from the host's mirror before it and back after it.
+constexpr int kLoopKernels = 3;
+
+cudaError_t enqueueLoop(rift_handle* h, int nsteps) {
     Params P = makeParams(h);
     if (useFlow(h)) {
         int rows = marchItemRows(h->nx, h->ny, h->numSMs * FLOW_WARPS);
@@ -1118,14 +1119,25 @@ cudaError_t enqueuePersist(rift_handle* h, int nsteps) {
                                        h->stream);
 }
 
-int launchPersist(rift_handle* h, int nsteps) {
+cudaError_t enqueuePersist(rift_handle* h, int nsteps) {
+    k_loop_begin<<<1, STATE_T, 0, h->stream>>>(h->hst, h->st, h->gbar);
+    cudaError_t e = enqueueLoop(h, nsteps);
+    if (e != cudaSuccess) return e;
+    k_loop_end<<<1, STATE_T, 0, h->stream>>>(h->hst, h->st);
+    return cudaGetLastError();
+}
+
+// Runs the loop and waits; the mirror then holds the state it left.
+int runPersist(rift_handle* h, int nsteps) {
     CUDA_TRY(h, enqueuePersist(h, nsteps));
-    h->launches += 1;
+    h->launches += kLoopKernels;
+    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    if (h->hst->error) return fail(h, RIFT_ERR_CUDA, deviceErrorText(h->hst->error));
     return RIFT_OK;
 }
 
-// Runs up to `nsteps` steps (state pushed, t_stop set; the host mirror of
-// the device state current).  While the active set is small the cooperative
+// Runs up to `nsteps` steps (t_stop set; the host mirror is the state to start
+// from).  While the active set is small the cooperative
 // step kernel runs the steps in one launch; once the active tiles outnumber
 // persistMax it leaves at a step boundary and the per-step graph (tile or
 // march kernels, chosen on the device) continues, in chunks of
@@ -1136,12 +1148,13 @@ constexpr int kGraphChunk = 64;
 int runSteps(rift_handle* h, int nsteps, bool* mirrorCurrent) {
     int rc;
     int left = nsteps;
-    *mirrorCurrent = false;
+    bool pushed = false;  // the device holds the state
+    *mirrorCurrent = nsteps <= 0;
     while (left > 0) {
         if (h->persistMax > 0 && h->hst->nActive <= h->persistMax) {
             const int before = h->hst->steps_done;
-            if ((rc = launchPersist(h, left)) || (rc = pullState(h))) return rc;
-            *mirrorCurrent = true;
+            if ((rc = runPersist(h, left))) return rc;
+            pushed = *mirrorCurrent = true;
             const int ran = h->hst->steps_done - before;
             h->persistSteps += ran;
             left -= ran;
@@ -1150,7 +1163,8 @@ int runSteps(rift_handle* h, int nsteps, bool* mirrorCurrent) {
         }
         if (left <= 0) break;
         const int chunk = std::min(left, kGraphChunk);
-        if ((rc = buildGraph(h))) return rc;
+        if ((rc = buildGraph(h)) || (!pushed && (rc = pushStateAsync(h)))) return rc;
+        pushed = true;
         for (int k = 0; k < chunk; k++) CUDA_TRY(h, cudaGraphLaunch(h->graphExec, h->stream));
         h->graphSteps += chunk;
         h->launches += (long long)chunk * h->graphKernels;
@@ -1169,9 +1183,8 @@ int runSteps(rift_handle* h, int nsteps, bool* mirrorCurrent) {
 }  // namespace
 
 namespace {
-// rift_step on the persistent loop as one graph: state push, barrier reset,
-// the one-step cooperative launch, state pull -- one launch and one wait
-// per step.  Rebuilt when the grid changes; false if the graph cannot be
+// rift_step on the persistent loop as one graph (enqueuePersist for one step):
+// one launch and one wait per step.  Rebuilt when the grid changes; false if the graph cannot be
 // made (the caller launches directly).
 bool stepGraph(rift_handle* h, int& rc) {
     rc = RIFT_OK;
@@ -1191,9 +1204,7 @@ bool stepGraph(rift_handle* h, int& rc) {
             cudaGetLastError();
             return false;
         }
-        cudaMemcpyAsync(h->st, h->hst, sizeof(DevState), cudaMemcpyHostToDevice, h->stream);
         enqueuePersist(h, 1);
-        cudaMemcpyAsync(h->hst, h->st, sizeof(DevState), cudaMemcpyDeviceToHost, h->stream);
         cudaError_t e = cudaStreamEndCapture(h->stream, &g);
         if (e != cudaSuccess || !g ||
             cudaGraphInstantiate(&h->stepExec[slot], g, 0) != cudaSuccess) {
@@ -1218,7 +1229,7 @@ bool stepGraph(rift_handle* h, int& rc) {
         return true;
     }
     h->persistSteps += h->hst->steps_done - before;
-    h->launches += 1;
+    h->launches += kLoopKernels;
     return true;
 }
 }  // namespace
@@ -1240,7 +1251,7 @@ int rift_run(rift_handle* h, int32_t nsteps, double t_stop, double* t, double* d
         if (steps_done) *steps_done = h->hst->steps_done;
         return RIFT_OK;
     }
-    if ((rc = pushStateAsync(h)) || (rc = runSteps(h, nsteps, &current))) return rc;
+    if ((rc = runSteps(h, nsteps, &current))) return rc;
     if (!current && (rc = pullState(h))) return rc;
     if (t) *t = h->hst->t;
     if (dt) *dt = h->hst->dt;

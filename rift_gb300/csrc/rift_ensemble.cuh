@@ -85,11 +85,6 @@ struct EnsArgs {
 // The members' device states from the block the host sent, and back: one
 // copy each way for all members (a copy per member each way, with a wait
 // each, took 330 us a run of 20 members).
-__device__ __forceinline__ void copyState(DevState* dst, const DevState* src) {
-    static_assert(sizeof(DevState) % 4 == 0, "copied in words");
-    for (int k = threadIdx.x; k < (int)(sizeof(DevState) / 4); k += blockDim.x)
-        reinterpret_cast<unsigned*>(dst)[k] = reinterpret_cast<const unsigned*>(src)[k];
-}
 __global__ void k_ens_begin(const EnsMember* M, EnsDev* D) {
     const EnsMember& m = M[blockIdx.x];
     copyState(m.P.st, &m.st);
