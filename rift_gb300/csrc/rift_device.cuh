@@ -23,14 +23,13 @@ constexpr float kTheta = 1.3f;         // grid.cu:30
 // low word of a double and is never negative, so minmod(a,b,c) evaluates to
 // +min(|a|,|b|,|c|) (times a factor within 1.5e-6 of 1) and the slope is
 //   0.5 * min(theta|d+|, 0.5|d+ + d-|, theta|d-|)  >= 0
-// = kSlope * min(|d+|, kMid |d+ + d-|, |d-|), the minimum given here: the
-// factor goes into the fma that adds the slope.  It is zero whenever one
-// argument is zero, which min() already gives.
-constexpr float kSlope = 0.5f * kTheta;
-constexpr float kMid = 0.5f / kTheta;
+// = 1/4 * min(2 theta min(|d+|, |d-|), |d+ + d-|), the minimum given here: the
+// quarter, exact, goes into the fma that adds the slope.  It is zero whenever
+// one argument is zero, which min() already gives.
+constexpr float kSlope = 0.25f;
 template <class V>
 __device__ __forceinline__ V limited(V dp, V dm) {
-    return minAbs3(dp, dm, vmul(splat<V>(kMid), vadd(dp, dm)));
+    return minAbs(vmul(splat<V>(2.f * kTheta), minAbs(dp, dm)), vadd(dp, dm));
 }
 
 // State at one face of a cell (of two cells: V = P2): depth, hu, hv.
@@ -104,21 +103,22 @@ __device__ __forceinline__ V velFactor(V h, float kappa) {
 // the depth is not positive (formed from the depth clamped at 0).
 template <class V>
 struct Side {
-    V qn, qt, sp, sm, f0, fn, ft;
+    V t, qn, qt, sp, sm, f0, fn, ft;
 };
 template <class V>
 __device__ __forceinline__ Side<V> faceSide(V h, V qn, V qt, float kappa) {
     Side<V> s;
     const V r = velFactor(h, kappa);
     const V n = vmul(qn, r), t = vmul(qt, r);
+    s.t = t;
     s.qn = vmul(h, n);
     s.qt = vmul(h, t);
     const V c = vsqrt(vmul(splat<V>(kG), h));
-    s.sp = vadd(c, n);
-    s.sm = vsub(c, n);
+    s.sp = vaddOfMul(c, n);
+    s.sm = vsubOfMul(c, n);
     const V hp = vmax(h, splat<V>(0.f));
     s.f0 = vmul(hp, n);
-    s.fn = vfma(s.f0, n, vmul(vmul(splat<V>(0.5f * kG), hp), hp));
+    s.fn = vfma(vmul(splat<V>(0.5f * kG), hp), hp, vmul(s.f0, n));
     s.ft = vmul(s.f0, t);
     return s;
 }
@@ -137,8 +137,8 @@ __device__ __forceinline__ V faceFlux(const Face<V>& L, const Face<V>& R, float 
     const V r = vrcp(vmax(vadd(ap, am), splat<V>(1e-30f)));
     const V k = vmul(vmul(ap, am), r);
     f[0] = vfma(vfma(ap, a.f0, vmul(am, b.f0)), r, vmul(k, vsub(L.h, R.h)));
-    const V fn = vfma(vfma(ap, a.fn, vmul(am, b.fn)), r, vmul(k, vsub(a.qn, b.qn)));
-    const V ft = vfma(vfma(ap, a.ft, vmul(am, b.ft)), r, vmul(k, vsub(a.qt, b.qt)));
+    const V fn = vfma(vfma(ap, a.fn, vmul(am, b.fn)), r, vmul(k, vsubOfMul(a.qn, b.qn)));
+    const V ft = vfma(vfma(ap, a.ft, vmul(am, b.ft)), r, vmul(k, vfnma(R.h, b.t, a.qt)));
     f[1] = DIR == 0 ? fn : ft;
     f[2] = DIR == 0 ? ft : fn;
     return vmax(ap, am);
@@ -149,11 +149,14 @@ __device__ __forceinline__ float faceFlux(float hL, float huL, float hvL, float 
     return faceFlux<DIR>(Face<float>{hL, huL, hvL}, Face<float>{hR, huR, hvR}, kappa, f);
 }
 
-// Local speed at a face (the mx / my of getHX / getHY, grid.cu:118-214); qn is
-// the momentum normal to the face.
+// Local speed at a face (the mx / my of getHX / getHY, grid.cu:118-214) as the
+// speed pass takes it, without the fluxes; qn is the momentum normal to the
+// face.  Its sums n + c and c - n are fmas, faceFlux's are not: the two may
+// differ in the last bit.
 __device__ __forceinline__ float faceSpeed(float hL, float qL, float hR, float qR, float kappa) {
-    float f[3];
-    return faceFlux<0>(Face<float>{hL, qL, 0.f}, Face<float>{hR, qR, 0.f}, kappa, f);
+    const float rL = velFactor(hL, kappa), rR = velFactor(hR, kappa);
+    const float cL = vsqrt(vmul(kG, hL)), cR = vsqrt(vmul(kG, hR));
+    return fmaxf(vmaxz(vfma(qL, rL, cL), vfma(qR, rR, cR)), vmaxz(vfnma(qL, rL, cL), vfnma(qR, rR, cR)));
 }
 
 // Flux divergence from the differences of the fluxes through a cell's east and
@@ -167,15 +170,19 @@ __device__ __forceinline__ V divergence(V fx, V fy, float inv_dx, float inv_dy) 
 // and eP are the cell's face offsets in the direction, inv its inverse width.
 template <class V>
 __device__ __forceinline__ V addBed(V d, V hC, V eM, V eP, float inv) {
-    return vfma(vmul(splat<V>(-kG), hC), vmul(vsub(eP, eM), splat<V>(inv)), d);
+    return vaddOfMul(d, vmul(vmul(splat<V>(-kG), hC), vmul(vsub(eP, eM), splat<V>(inv))));
 }
+
+// The sums below state which product goes into an fma: left to the compiler,
+// the choice changes with the kernel they are inlined in, and the schedules
+// would round apart.
 
 // Green-Ampt infiltration rate (grid.cu:791-805), clamped to [0, h/dt].
 // The quadratic root is taken in the cancellation-free form when p1 < 0.
 __device__ __forceinline__ float greenAmpt(float K, float F, float psiDtheta, float dt, float hC) {
-    float p1 = K * dt - 2.f * F;
-    float p2 = K * (F + psiDtheta);
-    float s = sqrtf(p1 * p1 + 8.f * p2 * dt);
+    float p1 = vfma(K, dt, -2.f * F);
+    float p2 = vmul(K, vadd(F, psiDtheta));
+    float s = sqrtf(vfma(p1, p1, vmul(8.f * p2, dt)));
     float f = (p1 >= 0.f) ? (p1 + s) / (2.f * dt) : (4.f * p2) / (s - p1);
     float cap = hC / dt;
     f = (f > cap) ? cap : f;
@@ -185,9 +192,9 @@ __device__ __forceinline__ float greenAmpt(float K, float F, float psiDtheta, fl
 
 // Semi-implicit Manning coefficient G (grid.cu:754-760).
 __device__ __forceinline__ float manningG(float n, float hu, float hv, float hC, float kappa) {
-    float h2 = hC * hC;
-    float den = h2 + fmaxf(h2, kappa);
-    return -4.f * kG * n * n * sqrtf(hu * hu + hv * hv) * powf(hC, 5.f / 3.f) / (den * den);
+    float h2 = vmul(hC, hC);
+    float den = vadd(h2, fmaxf(h2, kappa));
+    return -4.f * kG * n * n * sqrtf(vfma(hu, hu, vmul(hv, hv))) * powf(hC, 5.f / 3.f) / (den * den);
 }
 
 // Critical-depth ghost value (ApplyBoundariesX_k / Y_k, grid.cu:1325-1406):

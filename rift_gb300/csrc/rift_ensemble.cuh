@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(ENS_T, 1) k_ensemble(EnsArgs E) {
             const Params& P = W.P;
             auto on = [&](int by, int bx) { return bx >= 0 && P.prevAct[by * P.nBX + bx] != 0; };
             float tmx = 0.f, tmy = 0.f;
-            const bool ok = marchRows<1, 0, false>(P, W.C, &E.M[m].maps[0], &E.M[m].maps[2], S,
+            const bool ok = marchRows<1, 0, false, false>(P, W.C, &E.M[m].maps[0], &E.M[m].maps[2], S,
                                                    par, seg, j0, j1, on, false, L, tmx, tmy, false);
             tmx = warpMax(tmx);
             tmy = warpMax(tmy);
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(ENS_T, 1) k_ensemble(EnsArgs E) {
             auto on = [&](int by, int bx) { return bx >= 0 && P.prevAct[by * P.nBX + bx] != 0; };
             float tmx = 0.f, tmy = 0.f;
             return byFlags(P, [&](auto fix) {
-                return marchRows<2, decltype(fix)::value, false>(P, C, &E.M[m].maps[1],
+                return marchRows<2, decltype(fix)::value, false, false>(P, C, &E.M[m].maps[1],
                                                                  &E.M[m].maps[2], S, par, seg, j0, j1,
                                                                  on, false, L, tmx, tmy, false);
             });

@@ -145,7 +145,8 @@ __global__ void __launch_bounds__(FLOW_T, 1) k_flow(const __grid_constant__ CUte
     __shared__ double sDt, sT;
     __shared__ float wmax[2][FLOW_WARPS];
     __shared__ unsigned sStale[2];
-    __shared__ int sErr;
+    __shared__ float sSeed[2];
+    __shared__ int sErr, sRedo;
     StageConsts& C1 = *reinterpret_cast<StageConsts*>(cbuf[0]);
     StageConsts& C2 = *reinterpret_cast<StageConsts*>(cbuf[1]);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -167,6 +168,7 @@ __global__ void __launch_bounds__(FLOW_T, 1) k_flow(const __grid_constant__ CUte
         prefetch_tmap(&tmB);
         prefetch_tmap(&tmE);
         sStale[0] = sStale[1] = 0u;
+        sSeed[0] = sSeed[1] = 0.f;
         C1 = stageConsts<1>(P);  // (the flux phase reads what no step changes)
         C2 = stageConsts<2>(P);
     }
@@ -198,6 +200,10 @@ __global__ void __launch_bounds__(FLOW_T, 1) k_flow(const __grid_constant__ CUte
         // the grow is a no-op when no tile's activity changes: from the second
         // step on the flux phase runs on the last step's set and checks that
         bool rated = false;  // this step's source rates are formed
+        bool grown = false;  // and its set is the grow's
+        // the dt speeds are sought from 15/16 of the last step's maxima upward;
+        // where none is found, once more from 0
+        float seedX = sSeed[0], seedY = sSeed[1];
         // (inactive tiles without interior cells are never tracked into the set)
         const bool trackNow = track && (step == 0 ? nInact != 0 : nAct < allTiles);
         bool guess = step > 0 && !trackNow;
@@ -207,7 +213,8 @@ __global__ void __launch_bounds__(FLOW_T, 1) k_flow(const __grid_constant__ CUte
         }
         if (blockIdx.x == 0 && tid == 0) beginStepResets(st);
     flux:
-        if (!guess) {
+        if (!guess && !grown) {
+            grown = true;
             if (tid < NT) growAppend<false, true>(P, T->staleb[pr], &T->itemCnt[pr]);
             FLOW_SYNC();
             nAct = (int)ld_relaxed_gpu((const unsigned*)&st->appendCnt[0]);
@@ -220,7 +227,7 @@ __global__ void __launch_bounds__(FLOW_T, 1) k_flow(const __grid_constant__ CUte
             }
             for (int k = blockIdx.x * FLOW_T + tid; k < nList; k += gridDim.x * FLOW_T)
                 P.itemStamp[P.items[k]] = 0;  // for the next grow
-        } else {
+        } else if (guess) {
             nDe = 0;
         }
         const bool all = nAct == allTiles;
@@ -253,8 +260,8 @@ __global__ void __launch_bounds__(FLOW_T, 1) k_flow(const __grid_constant__ CUte
         Led L1;  // stage 1's edge inflow rates: dt is not known yet
         ledZero(L1);
         bool ok = items([&](int seg, int j0, int j1) {
-            return marchRows<1, 0, false>(P, C1, &tmA, &tmE, S, par, seg, j0, j1, on, led, L1, tmx, tmy,
-                                          false);
+            return marchRows<1, 0, false, true>(P, C1, &tmA, &tmE, S, par, seg, j0, j1, on, led, L1, tmx, tmy,
+                                          false, seedX, seedY);
         });
         if (!ok && lane == 0) atomicOr(&st->error, ERR_TMA_TIMEOUT);
         if (guess) {
@@ -282,25 +289,37 @@ __global__ void __launch_bounds__(FLOW_T, 1) k_flow(const __grid_constant__ CUte
             atomicMax(guess ? &T->guess[pr][tid] : &T->maxb[pr][tid], __float_as_uint(m));
         }
         FLOW_SYNC();
-        if (guess && ld_relaxed_gpu((const unsigned*)&T->changed[pr]) != 0u) {
-            guess = false;  // every CTA reads the same flag
-            goto flux;
-        }
         // ---- dt (Simulator::ComputeTimestep) and the stage constants, by
-        // thread 0 of every CTA; then stage 1's update
+        // thread 0 of every CTA (which all see the same counts and maxima);
+        // then stage 1's update
         if (tid == 0) {
-            const unsigned* m = guess ? T->guess[pr] : T->maxb[pr];
-            const unsigned mx = max(ld_relaxed_gpu(&m[0]), sStale[0]);
-            const unsigned my = max(ld_relaxed_gpu(&m[1]), sStale[1]);
-            const double dtNew = stepDtAt(P, tNow, __uint_as_float(mx), __uint_as_float(my));
-            sDt = dtNew;
-            sT = tNow + dtNew;
-            C1 = stageConstsAt<1>(P, dtNew, dtPrev, sT);
-            C2 = stageConstsAt<2>(P, dtNew, dtPrev, sT);
+            const unsigned* const m = guess ? T->guess[pr] : T->maxb[pr];
+            const unsigned mx = ld_relaxed_gpu(&m[0]), my = ld_relaxed_gpu(&m[1]);
+            const unsigned ch = ld_relaxed_gpu((const unsigned*)&T->changed[pr]);
             sErr = (int)ld_relaxed_gpu((const unsigned*)&st->error);
+            sRedo = guess && ch != 0u ? 1 : __uint_as_float(mx) < seedX || __uint_as_float(my) < seedY ? 2 : 0;
+            if (sRedo == 0) {
+                const double dtNew = stepDtAt(P, tNow, __uint_as_float(max(mx, sStale[0])),
+                                              __uint_as_float(max(my, sStale[1])));
+                sDt = dtNew;
+                sT = tNow + dtNew;
+                C1 = stageConstsAt<1>(P, dtNew, dtPrev, sT);
+                C2 = stageConstsAt<2>(P, dtNew, dtPrev, sT);
+                sSeed[0] = 0.9375f * __uint_as_float(mx);
+                sSeed[1] = 0.9375f * __uint_as_float(my);
+            }
         }
         __syncthreads();
         if (sErr) return;  // a wait gave up before the barrier: every CTA sees it
+        if (sRedo == 1) {  // the set changes
+            guess = false;
+            goto flux;
+        }
+        if (sRedo == 2) {  // no speed as high as the seed (the next maxima join these)
+            seedX = seedY = 0.f;
+            FLOW_SYNC();
+            goto flux;
+        }
         tNow = sT;
         dtPrev = sDt;
         L.v[LED_BOUND] += C1.wRate * L1.v[LED_BOUND];
@@ -311,7 +330,7 @@ __global__ void __launch_bounds__(FLOW_T, 1) k_flow(const __grid_constant__ CUte
         FLOW_SYNC();
         // ---- stage 2; the spare CTA publishes dt and the grow's counts
         ok = items([&](int seg, int j0, int j1) {
-            return marchRows<2, FIX, false>(P, C2, &tmB, &tmE, S, par, seg, j0, j1, on, led, L, tmx, tmy, false);
+            return marchRows<2, FIX, false, false>(P, C2, &tmB, &tmE, S, par, seg, j0, j1, on, led, L, tmx, tmy, false);
         });
         if (!ok && lane == 0) atomicOr(&st->error, ERR_TMA_TIMEOUT);
         if (spare && tid == 0) {

@@ -1097,14 +1097,14 @@ __device__ __forceinline__ void rk1Core(const Params& P, const StageConsts& C, s
         float sg = mapValue(P, 2, c, C.fac2);
         if (sg != P.nodata && sg > 0.f) {
             const float d0 = dh;
-            dh = (sg - (hc + dh * dtNew)) / dtNew;
+            dh = (sg - vfma(dh, dtNew, hc)) / dtNew;
             if (L) L->v[LED_SURGE] += C.wRate * (dh - d0);
         }
     }
-    hN = hc + dh * dtNew;
-    const float den = 1.f / (1.f - dtNew * src.G);
-    huN = (hu0 + src.dhu * dtNew) * den;
-    hvN = (hv0 + src.dhv * dtNew) * den;
+    hN = vfma(dh, dtNew, hc);
+    const float den = 1.f / vfma(-dtNew, src.G, 1.f);
+    huN = vmul(vfma(src.dhu, dtNew, hu0), den);
+    hvN = vmul(vfma(src.dhv, dtNew, hv0), den);
     if (L) L->v[LED_CLAMP] += C.wHalf * ((hC - hc) + ((hN > kEps) ? 0.f : hN));
     hN = (hN > kEps) ? hN : 0.f;
 }
@@ -1129,7 +1129,7 @@ __device__ __forceinline__ bool cellResult(const Params& P, const StageConsts& C
     if (STAGE == 1) {
         // Integrate_1_k (grid.cu:856-922)
         rk1Core<FIX>(P, C, c, src, hC, hu0, hv0, L, hN, huN, hvN);
-        if (fl & F_INFIL) C.Fout[c] = Fc + dF * dtNew;
+        if (fl & F_INFIL) C.Fout[c] = vfma(dF, dtNew, Fc);
         if (euler) {
             // Euler-mode outputs and wet flags (grid.cu:926-1023)
             const float uC = huN * velFactor(hN, C.kappa), vC = hvN * velFactor(hN, C.kappa);
@@ -1154,12 +1154,12 @@ __device__ __forceinline__ bool cellResult(const Params& P, const StageConsts& C
         // Integrate_2_k (grid.cu:1043-1171)
         const float hOld = pre[0];
         const float hOc = (hOld > kEps) ? hOld : 0.f;
-        hN = 0.5f * (hOc + hc + dh * dtNew);
-        huN = 0.5f * (pre[1] + hu0 + dhu * dtNew);
-        hvN = 0.5f * (pre[2] + hv0 + dhv * dtNew);
+        hN = 0.5f * vfma(dh, dtNew, vadd(hOc, hc));
+        huN = 0.5f * vfma(dhu, dtNew, vadd(pre[1], hu0));
+        hvN = 0.5f * vfma(dhv, dtNew, vadd(pre[2], hv0));
         if (L) L->v[LED_CLAMP] += 0.5f * ((hOld - hOc) + (hC - hc)) + ((hN > kEps) ? 0.f : hN);
         hN = (hN > kEps) ? hN : 0.f;
-        if (fl & F_INFIL) C.Fout[c] = 0.5f * ((PREF ? pre[5] : P.FA[c]) + Fc + dF * dtNew);
+        if (fl & F_INFIL) C.Fout[c] = 0.5f * vfma(dF, dtNew, vadd(PREF ? pre[5] : P.FA[c], Fc));
         if (fl & F_SAVE_MAX) {
             const float uC = huN * velFactor(hN, C.kappa);
             const float vC = hvN * velFactor(hN, C.kappa);

@@ -74,6 +74,11 @@ struct __align__(128) MarchRing {
 // lane's columns; r points at plane 0 of the row.
 __device__ __forceinline__ P2 row2(const float* r, int p) { return ld2(r + p * MCR * MBOX); }
 
+// Maximum of a warp's speeds in every lane.
+__device__ __forceinline__ float warpMax(float v) {
+    return __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(v)));
+}
+
 struct Cell2 {  // state of this lane's two columns in one row
     P2 h, u, v;
 };
@@ -93,12 +98,10 @@ __device__ __forceinline__ void constructY2(const Cell2& c, const float* r, cons
     construct(c.h, c.u, c.v, limited(dP.w, dM.w), limited(dP.u, dM.u), limited(dP.v, dM.v), row2(r, 5),
               row2(r, 6), P, M);
 }
-// x reconstruction of a row and the fluxes through the east faces of both
-// columns; fx: the difference of each column's east and west fluxes, fW0, fE0
-// the mass fluxes through both.  The differences mix neighbours of a pair, so
-// they stay scalar (packing them would cost a move each).
-__device__ __forceinline__ void rowFluxX(const Cell2& c, P2 eW, P2 eE, float kappa, P2 fx[3], P2& fW0,
-                                         P2& fE0, P2& spd) {
+// x reconstruction of a row: the states L, R on both sides of the east faces of
+// both columns.  The differences mix neighbours of a pair, so they stay scalar
+// (packing them would cost a move each).
+__device__ __forceinline__ void rowFacesX(const Cell2& c, P2 eW, P2 eE, Face<P2>& L, Face<P2>& R) {
     auto down = [](float a) { return __shfl_down_sync(FULL, a, 1); };
     auto up = [](float a) { return __shfl_up_sync(FULL, a, 1); };
     // limited differences of both columns from d0 (across the face between
@@ -108,16 +111,21 @@ __device__ __forceinline__ void rowFluxX(const Cell2& c, P2 eW, P2 eE, float kap
                         vadd(vsub(hi(eE), down(lo(eW))), vsub(down(lo(c.h)), hi(c.h))));
     const P2 tu = limit(vsub(hi(c.u), lo(c.u)), vsub(down(lo(c.u)), hi(c.u)));
     const P2 tv = limit(vsub(hi(c.v), lo(c.v)), vsub(down(lo(c.v)), hi(c.v)));
-    Face<P2> Pf, Mf;
-    construct(c.h, c.u, c.v, tw, tu, tv, eW, eE, Pf, Mf);
+    Face<P2> M;
+    construct(c.h, c.u, c.v, tw, tu, tv, eW, eE, L, M);
     auto east = [&](P2 a) { return pack2(hi(a), down(lo(a))); };
-    const Face<P2> R{east(Mf.h), east(Mf.u), east(Mf.v)};
+    R = Face<P2>{east(M.h), east(M.u), east(M.v)};
+}
+// The fluxes through the faces between L and R; fx: the difference of each
+// column's east and west fluxes, fW0, fE0 the mass fluxes through both.
+__device__ __forceinline__ void rowFluxX(const Face<P2>& L, const Face<P2>& R, float kappa, P2 fx[3],
+                                         P2& fW0, P2& fE0, P2& spd) {
     P2 f[3];
-    spd = faceFlux<0>(Pf, R, kappa, f);
+    spd = faceFlux<0>(L, R, kappa, f);
     float w[3];
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-        w[q] = up(hi(f[q]));
+        w[q] = __shfl_up_sync(FULL, hi(f[q]), 1);
         fx[q] = pack2(vsub(lo(f[q]), w[q]), vsub(hi(f[q]), lo(f[q])));
     }
     fW0 = pack2(w[0], lo(f[0]));
@@ -172,16 +180,18 @@ __device__ __forceinline__ void clearTile(const Params& P, int tile, bool euler)
 
 // Rows [j0, j1) of segment seg by one warp.  on(by, bx): is the tile active?
 // (called by all lanes; false for lanes that own no interior column).
-// CLEAR (stage 1): see clearTile.
+// CLEAR (stage 1): see clearTile.  DTS (stage 1): tmx, tmy are the warp's, of
+// faceSpeed, instead of this lane's, of faceFlux; maxima below seedX, seedY may
+// be missed.
 // STAGE 1: reads U^n (A) -> flux divergence + bed source (D), the speed
 //          maxima of active cells (tmx, tmy); Euler mode: tile speeds.
 // STAGE 2: reads U* (B) and U^n (A) at the cell -> writes U^{n+1} (A),
 //          F^{n+1} (FA), outputs, tile wet flags and tile speeds.
-template <int STAGE, uint32_t FIX, bool CLEAR, class On>
+template <int STAGE, uint32_t FIX, bool CLEAR, bool DTS, class On>
 __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C, const CUtensorMap* tmIn,
                                           const CUtensorMap* tmE, MarchRing& S, uint32_t& par, int seg,
                                           int j0, int j1, On on, bool led, Led& L, float& tmx,
-                                          float& tmy, bool pf) {
+                                          float& tmy, bool pf, float seedX = 0.f, float seedY = 0.f) {
     constexpr bool RAINPRE = STAGE == 2 && (FIX & F_RAIN_G) != 0;
     constexpr bool INFPRE = STAGE == 2 && (FIX & F_INFIL) != 0;
     const int lane = threadIdx.x & 31;
@@ -273,6 +283,15 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
     int sl = 1;  // slot of the chunk that holds row j + 1
     int by = (j0 - 2) / TH, rt = (j0 - 2) % TH;  // tile row, row in it
     bool act = on(by, bx);
+    // the active cells' speeds as the speed pass rounds them, into the maximum m
+    // of the warp: formed only where the fluxes' speeds, within 2e-7 of them,
+    // come near it, and above the seed
+    auto dtSpeeds = [&](P2 s, P2 hL, P2 qL, P2 hR, P2 qR, float& m, float seed) {
+        auto top = [&](P2 v) { return act ? fmaxf(lo(v), inY ? hi(v) : 0.f) : 0.f; };
+        if (!__any_sync(FULL, top(s) > fmaxf(m, seed) * (1.f - 1e-6f))) return;
+        m = fmaxf(m, warpMax(top(pack2(faceSpeed(lo(hL), lo(qL), lo(hR), lo(qR), kappa),
+                                       faceSpeed(hi(hL), hi(qL), hi(hR), hi(qR), kappa)))));
+    };
     int src = STAGE == 2 && act ? sourceTile(P, by * P.nBX + bx) : -1;
     float ax = 0.f, ay = 0.f;
     bool wet = false;
@@ -295,13 +314,17 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
         if (STAGE == 2 && pfB) prefetch_l2(pfB + (size_t)((unsigned)min(j + MPF, P.rows - 1) * pitch));
         const P2 eW = row2(rc, 3), eE = row2(rc, 4);
         P2 fN[3], sy, fx[3], fW0, fE0, sx;
-        rowFluxX(cur, eW, eE, kappa, fx, fW0, fE0, sx);
+        Face<P2> xL, xR;
+        rowFacesX(cur, eW, eE, xL, xR);
+        rowFluxX(xL, xR, kappa, fx, fW0, fE0, sx);
+        if (DTS) dtSpeeds(sx, xL.h, xL.u, xR.h, xR.u, tmx, seedX);
         // y: reconstruction of row j + 1, flux through the north face of row j
         const Cell2 ld = loadCell2(rl);
         const Diff2 dNN = diffY(nxt, rn, ld, rl);
         Face<P2> yn, yM;
         constructY2(nxt, rn, dNN, dN, yn, yM);
         sy = faceFlux<1>(yP, yM, kappa, fN);
+        if (DTS) dtSpeeds(sy, yP.h, yP.v, yM.h, yM.v, tmy, seedY);
         // divergence, with the bed-slope source in the momenta
         P2 d[3];
 #pragma unroll
@@ -310,8 +333,10 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
         d[1] = addBed(d[1], cur.h, eW, eE, P.inv_dx);
         d[2] = addBed(d[2], cur.h, row2(rc, 5), row2(rc, 6), P.inv_dy);
         if (act) {
-            ax = fmaxf(fmaxf(ax, lo(sx)), inY ? hi(sx) : 0.f);
-            ay = fmaxf(fmaxf(ay, lo(sy)), inY ? hi(sy) : 0.f);
+            if (!DTS) {
+                ax = fmaxf(fmaxf(ax, lo(sx)), inY ? hi(sx) : 0.f);
+                ay = fmaxf(fmaxf(ay, lo(sy)), inY ? hi(sy) : 0.f);
+            }
             const unsigned c = (unsigned)j * pitch + (unsigned)i;
             if (led && edge) {
                 float r = edgeInflow(P, j, i, lo(fW0), lo(fE0), lo(fS[0]), lo(fN[0]));
@@ -351,7 +376,7 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
             }
         }
         if (++rt == TH || j + 1 == j1) {  // the item's last row of a tile row (warp-uniform)
-            if (STAGE == 1) {
+            if (STAGE == 1 && !DTS) {
                 tmx = fmaxf(tmx, ax);
                 tmy = fmaxf(tmy, ay);
             }
@@ -388,11 +413,6 @@ __device__ __forceinline__ bool marchRows(const Params& P, const StageConsts& C,
     }
     if (STAGE == 2 && edge) ghostColumns(P, P.A, seg, j0, j1, on);
     return true;
-}
-
-// Maximum of a warp's speeds in every lane.
-__device__ __forceinline__ float warpMax(float v) {
-    return __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(v)));
 }
 
 // Resident CTAs per SM the march is compiled for: 128 registers a thread.
@@ -442,7 +462,7 @@ __global__ void __launch_bounds__(MT, MARCH_CTAS) k_march(const __grid_constant_
         for (int q = lane; q < nb * (by1 - by0 + 1); q += 32)
             any |= on(by0 + q / nb, bx0 + q % nb);
         if (!__any_sync(FULL, any)) continue;
-        if (!marchRows<STAGE, FIX, STAGE == 1>(P, C, &tmIn, &tmE, S, par, seg, j0, j1, on, led, L, tmx, tmy, pf != 0)) {
+        if (!marchRows<STAGE, FIX, STAGE == 1, false>(P, C, &tmIn, &tmE, S, par, seg, j0, j1, on, led, L, tmx, tmy, pf != 0)) {
             if (lane == 0) atomicOr(&P.st->error, ERR_TMA_TIMEOUT);
             break;
         }

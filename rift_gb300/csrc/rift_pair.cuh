@@ -48,6 +48,22 @@ __device__ __forceinline__ P2 vfma(P2 a, P2 b, P2 c) {
     asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
     return r;
 }
+// a + b, a - b where an operand is a product: the assembler contracts a packed
+// product and sum into one fma (in some kernels and not in others), scalar ones
+// with a rounding mode it leaves alone.
+__device__ __forceinline__ float vaddOfMul(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float vsubOfMul(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ P2 vaddOfMul(P2 a, P2 b) {
+    return pack2(__fadd_rn(lo(a), lo(b)), __fadd_rn(hi(a), hi(b)));
+}
+__device__ __forceinline__ P2 vsubOfMul(P2 a, P2 b) {
+    return pack2(__fsub_rn(lo(a), lo(b)), __fsub_rn(hi(a), hi(b)));
+}
+// c - a b
+__device__ __forceinline__ float vfnma(float a, float b, float c) { return __fmaf_rn(-a, b, c); }
+__device__ __forceinline__ P2 vfnma(P2 a, P2 b, P2 c) {
+    return pack2(vfnma(lo(a), lo(b), lo(c)), vfnma(hi(a), hi(b), hi(c)));
+}
 // a constant in every lane of V
 template <class V>
 __device__ __forceinline__ V splat(float x);
@@ -70,15 +86,9 @@ __device__ __forceinline__ float vmaxz(float a, float b) {
 }
 __device__ __forceinline__ P2 vmaxz(P2 a, P2 b) { return pack2(vmaxz(lo(a), lo(b)), vmaxz(hi(a), hi(b))); }
 
-// min(|a|, |b|, |c|)
-__device__ __forceinline__ float minAbs3(float a, float b, float c) {
-    float r;
-    asm("min.ftz.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-__device__ __forceinline__ P2 minAbs3(P2 a, P2 b, P2 c) {
-    return pack2(minAbs3(lo(a), lo(b), lo(c)), minAbs3(hi(a), hi(b), hi(c)));
-}
+// min(|a|, |b|)
+__device__ __forceinline__ float minAbs(float a, float b) { return fminf(fabsf(a), fabsf(b)); }
+__device__ __forceinline__ P2 minAbs(P2 a, P2 b) { return pack2(minAbs(lo(a), lo(b)), minAbs(hi(a), hi(b))); }
 __device__ __forceinline__ float vrcp(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
