@@ -27,7 +27,7 @@
 // wait is bounded (TMA mbarriers, grid barriers), as in k_persist.
 //
 // What bounds it: 20 members of 96 to 480 cells a side, uniform rain (1.58 M
-// cells), 100 us per iteration (191 on per-tile queues with a grow in every
+// cells), 102 us per iteration (191 on per-tile queues with a grow in every
 // iteration): flux 20.7, update 22, stage 2 29.9 (issue and the latency of a
 // warp's chain, 15.5 rows a warp), dt 4, the rest barriers and waits.  A run of
 // 8 steps also takes 109 us on the host (336 with a copy and a wait each way

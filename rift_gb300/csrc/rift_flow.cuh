@@ -22,11 +22,16 @@
 // to take them: a lone warp needs about 0.6 us per row, so a sparse set is
 // spread thin.
 //
-// What bounds it (us per step, GB300).  512^2 rain, 1221 tiles: 23.6 = flux
-// 4.7, dt 1.0, update 3.1, stage 2 6.7 and three barriers of 1.3 to 1.8 with
-// the wait for the slowest CTA on top: latency.  1024^2 rain: 49 = 11.6 + 1.0
-// + 8.7 + 17.0 + barriers and waits 10: issue in the flux passes, L2 in the
-// update (52 bytes per cell).
+// dt takes the speeds as the per-tile schedule's speed pass rounds them
+// (faceSpeed), so both give the same dt; the fluxes' own differ in the last
+// bit.  They are formed only for faces near the maximum and above 15/16 of the
+// last step's (1117 x 1531 rain: 94 us a step, 96 without that seed).
+//
+// What bounds it (us per step, GB300).  512^2 rain, 1221 tiles: 24.2 (34 with
+// the per-tile phases) = flux 5, dt 1.0, update 3.1, stage 2 7 and three
+// barriers of 1.3 to 1.8 with the wait for the slowest CTA on top: latency.
+// 1024^2 rain: 50 (86) = 12 + 1.0 + 8.7 + 17 + barriers and waits 10: issue in
+// the flux passes, L2 in the update (52 bytes per cell).
 #pragma once
 #include "rift_grow.cuh"
 #include "rift_march.cuh"
@@ -131,6 +136,27 @@ __device__ __forceinline__ void updateRows(const Params& P, const StageConsts& C
         }
     }
     if (edge) ghostColumns(P, P.B, seg, j0, j1, on);
+}
+
+// flushLed for the whole CTA: one atomic per term.  (One per term and warp has
+// 2432 of them queue at each address: 500 x 701 with a surge 43.7 us a step,
+// 42.9 with one per CTA.)
+__device__ __forceinline__ void flushLedBlock(Led& L, double* dst) {
+    __shared__ float part[LED_N][FLOW_WARPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < LED_N; k++) {
+        float v = L.v[k];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
+        if (lane == 0) part[k][warp] = v;
+        L.v[k] = 0.f;
+    }
+    __syncthreads();
+    if (warp < LED_N) {
+        double sum = lane < FLOW_WARPS ? (double)part[warp][lane] : 0.0;
+        for (int o = FLOW_WARPS / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
+        if (lane == 0 && sum != 0.0) atomicAdd(&dst[warp], sum);
+    }
 }
 
 // Step loop.  itemRows: rows per item while every tile is active.
@@ -347,7 +373,7 @@ __global__ void __launch_bounds__(FLOW_T, 1) k_flow(const __grid_constant__ CUte
                 st->nDeact = 0;
             }
         }
-        if (led) flushLed(L, st->led);
+        if (led) flushLedBlock(L, st->led);
         FLOW_SYNC();
     }
 #undef FLOW_SYNC

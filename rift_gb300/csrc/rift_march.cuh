@@ -30,7 +30,7 @@
 //
 // What bounds it: on 4096^2 cells of urban rain the passes issue 201 and 292
 // lane instructions per cell (397 and 505 with one column per lane, a CTA of
-// four warps in step and scalar arithmetic) and take 153 and 222 us (219 and
+// four warps in step and scalar arithmetic) and take 154 and 226 us (219 and
 // 294); they issue on 60% of cycles, the packed instructions' FMA pipe is 60%
 // busy, DRAM moves at 4.6 and 5.0 TB/s.  A lone warp needs 0.56 us per row.
 #pragma once
