@@ -1095,8 +1095,20 @@ int persistGrid(const rift_handle* h) {
 // 400^2 rain and infiltration, 754 tiles, 38 -> 22; 512^2 rain, 1221 tiles,
 // 34 -> 24; a 2048^2 channel flood, 651 tiles, 34 -> 27; 1024^2 rain, 4810
 // tiles, 86 -> 49.
-bool useFlow(const rift_handle* h) {
-    return h->flowOk && !h->has(RIFT_F_EULER) && h->hst->nActive > h->gridPersist;
+bool aboveOnePerCta(const rift_handle* h) { return h->hst->nActive > h->gridPersist; }
+
+// Under gridded rain k_persist cannot keep its tile table and grows and tracks
+// every step; while every tile is active k_flow needs neither.  Rain maps and
+// drain, us per step of a run: 110 tiles 18.8 -> 17.4, 195 21.4 -> 18.0, 418
+// 25.1 -> 19.1, 550 29.2 -> 20.3.  A call of one step costs more up to about 400
+// tiles (195 tiles 37 -> 42), hence the least number of steps.
+bool fullRainGrid(const rift_handle* h, int nsteps) {
+    const int all = ((h->nx - 4 + TW - 1) / TW) * ((h->ny - 4 + TH - 1) / TH);
+    return marchFix(h) == FIX_RAINMAP_DRAIN && nsteps >= 8 && h->hst->nActive == all && all > h->numSMs;
+}
+
+bool useFlow(const rift_handle* h, int nsteps) {
+    return h->flowOk && !h->has(RIFT_F_EULER) && (aboveOnePerCta(h) || fullRainGrid(h, nsteps));
 }
 
 // One cooperative launch of the chosen loop (also under capture), with the
@@ -1105,9 +1117,10 @@ constexpr int kLoopKernels = 3;
 
 cudaError_t enqueueLoop(rift_handle* h, int nsteps) {
     Params P = makeParams(h);
-    if (useFlow(h)) {
+    if (useFlow(h, nsteps)) {
         int rows = marchItemRows(h->nx, h->ny, h->numSMs * FLOW_WARPS);
-        int minTiles = h->gridPersist * 3 / 4;  // (hysteresis between the two loops)
+        // (hysteresis between the two loops; under fullRainGrid: every tile)
+        int minTiles = aboveOnePerCta(h) ? h->gridPersist * 3 / 4 : h->hst->nActive;
         void* args[] = {(void*)&h->tmAm, (void*)&h->tmBm, (void*)&h->tmEm, (void*)&P, (void*)&nsteps,
                         (void*)&rows, (void*)&minTiles};
         return cudaLaunchCooperativeKernel(flowKernel(h), dim3(h->numSMs), dim3(FLOW_T), args, FLOW_SMEM,
@@ -1189,7 +1202,7 @@ namespace {
 bool stepGraph(rift_handle* h, int& rc) {
     rc = RIFT_OK;
     if (h->stepGraphBroken) return false;
-    const int grid = useFlow(h) ? -1 : persistGrid(h);  // -1: k_flow
+    const int grid = useFlow(h, 1) ? -1 : persistGrid(h);  // -1: k_flow
     int slot = -1;
     for (int k = 0; k < rift_handle::STEP_CACHE; k++)
         if (h->stepExec[k] && h->stepGrid[k] == grid) slot = k;

@@ -106,3 +106,35 @@ def test_flow_matches_tiles(engine_api, name):
         la, lb = a.ledger(), b.ledger()
         moved = sum(abs(lb[k]) for k in ("added", "drained", "surge", "boundary"))
         assert all(abs(la[k] - lb[k]) <= 1e-4 * moved for k in lb if k != "residual"), (la, lb)
+
+
+@pytest.mark.parametrize("dries", [False, True])
+@pytest.mark.parametrize("n", [150, 200, 340])  # 110, 195 and 550 tiles: around one per SM, below one per CTA
+def test_full_rain_grid_matches_tiles(engine_api, n, dries):
+    """Runs under rain maps and a drain with every tile active (and, with dries,
+    a corner whose rain stops and drains away, so that the set shrinks)."""
+    z, mann = _plane(n, n)
+    case = synth.Case(name="rows", B=z, cell=10.0, n=mann, series={1: synth.csv_series([0, 1], [2, 2])},
+                      flags=synth.RAIN_GRID | synth.DRAIN_UNIFORM | synth.TILE_ACCEL)
+    sims = []
+    for persist in (1 << 30, 0):
+        sim = capi.Sim(case, api=engine_api).set_schedule(1 << 30).set_persistent(persist).setup()
+        r = np.zeros((n + 4, n + 4))
+        r[2:-2, 2:-2] = 30.0 / 3.6e6
+        sim.set_map(0, r)
+        sim.run(12)
+        if dries:
+            r[:n // 2, :n // 2] = 0.0
+            sim.set_map(0, r)
+            w = np.where(r > 0, sim.field("W"), sim.field("BC"))
+            sim.set_state(*sim.time(), w, sim.field("HU") * (r > 0), sim.field("HV") * (r > 0))
+        for k in (1, 20, 7, 30):
+            sim.run(k)
+        sims.append(sim)
+    a, b = sims
+    assert a.path_stats() == (70, 0) and b.path_stats() == (0, 70)
+    (wa, aa), (wb, ab) = a.tiles(), b.tiles()
+    assert (aa.size < a.grid_size) == dries
+    assert np.array_equal(wa, wb) and np.array_equal(aa, ab)
+    d = np.abs(a.field("W") - b.field("W"))[2:-2, 2:-2]
+    assert np.quantile(d, 0.99) <= Q99 and d.max() <= MAX
