@@ -66,7 +66,7 @@ def fatbin_path():
 def build_ref_fatbin(force=False):
     """Compile the reference's grid.cu (device code only) where the reference
     tree exists; a no-op elsewhere (the prebuilt fatbin is used)."""
-    if not os.path.isdir(REFERENCE_TREE) or shutil.which("nvcc") is None:
+    if not os.path.exists(os.path.join(REFERENCE_TREE, "grid.cu")) or shutil.which("nvcc") is None:
         return fatbin_path() if os.path.exists(fatbin_path()) else None
     os.makedirs(REF_OUT, exist_ok=True)
     src = os.path.join(HERE, "refkit", "ref_device.cu")
