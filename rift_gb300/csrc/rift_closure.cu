@@ -1322,6 +1322,10 @@ __global__ void __launch_bounds__(TCT, 1) k_closure(ApplyArgs A) {
         }
         tcStoreInput(T, R, src);
         if (!groupAnd(g, ok)) break;
+        // T.next is read between the block's first two barriers: after the first
+        // it is written, and after the second the leader may write it again (a
+        // dry block has no barrier after that one)
+        next = T.next;
         bool dry = true;
         for (int i = tid; i < (OT + 1) * (OT + 1); i += GT) {
             int ry = 3 + i / (OT + 1), rx = 3 + i % (OT + 1);
@@ -1329,7 +1333,6 @@ __global__ void __launch_bounds__(TCT, 1) k_closure(ApplyArgs A) {
         }
         dry = groupAnd(g, dry);
         if (tid == 0 && !dry) bar_arrive(&T.in);
-        next = T.next;
         if (next < ntile) {  // the next block's inputs, in flight meanwhile
             const TileGeom Gn = tileGeom(src, next);
             tcLoadInput(R, src, 0, Gn.Y - 3, Gn.X - 3);
