@@ -13,7 +13,9 @@
 //      of each member's step (one warp per member); U* re-sync of the tiles
 //      that went inactive
 //   D  dt: one thread per member -> dt, t, ledger, list sizes, liveness of
-//      the member's next step
+//      the member's next step; the wet flags of the Euler members' active
+//      tiles are cleared (phase 1 sets those of the wet ones: warps share
+//      tiles, so a clear has to lie a barrier away from it)
 //   1  the rest of RK stage 1
 //   2  stage 2, or the Euler commit of (member, active tile) items
 // S, 1 and 2 run the march's code (rift_march.cuh, rift_flow.cuh) on the warps
@@ -49,6 +51,7 @@ struct EnsDev {
     GridBar bar;
     int live[2][ENS_MAX];  // liveness per step parity
     int nAlive[2];
+    int nEuler[2];         // live members in Euler mode
     int itemCnt[ENS_MAX];  // the grow's count of a member's (segment, tile row) pairs
     int nItems[ENS_MAX];   // the pairs of the member's current set
     int all[ENS_MAX];      // every tile with interior cells is active
@@ -91,6 +94,7 @@ __global__ void k_ens_begin(const EnsMember* M, EnsDev* D) {
     if (threadIdx.x == 0) {
         D->live[0][blockIdx.x] = m.live;
         if (m.live) atomicAdd(&D->nAlive[0], 1);
+        if (m.live && (m.P.flags & F_EULER)) atomicAdd(&D->nEuler[0], 1);
     }
 }
 __global__ void k_ens_end(EnsMember* M) {
@@ -315,7 +319,7 @@ __global__ void __launch_bounds__(ENS_T, 1) k_ensemble(EnsArgs E) {
             ENS_SYNC();
         }
         // the other parity's counts were last read in the previous step
-        if (tid == 0 && blockIdx.x == 0) D->nAlive[cur ^ 1] = D->changed[cur ^ 1] = 0;
+        if (tid == 0 && blockIdx.x == 0) D->nAlive[cur ^ 1] = D->nEuler[cur ^ 1] = D->changed[cur ^ 1] = 0;
         Led L;  // members keep no ledger (rift_ensemble_create)
         bool begun = false;
     flux:
@@ -460,6 +464,16 @@ __global__ void __launch_bounds__(ENS_T, 1) k_ensemble(EnsArgs E) {
             }
             D->live[cur ^ 1][m] = next;
             if (next) atomicAdd(&D->nAlive[cur ^ 1], 1);
+            if (next && (E.M[m].P.flags & F_EULER)) atomicAdd(&D->nEuler[cur ^ 1], 1);
+        }
+        if (D->nEuler[cur] > 0) {
+            ensPrefix(n, [&](int m) { return live[m] && (E.M[m].P.flags & F_EULER) ? E.M[m].P.gridSize : 0; },
+                      Q.offs2);
+            for (int g = blockIdx.x * ENS_T + tid; g < Q.offs2[n]; g += gridDim.x * ENS_T) {
+                const int m = ensMember(Q.offs2, n, g), b = g - Q.offs2[m];
+                const Params& P = E.M[m].P;
+                if (P.prevAct[b] && tileCells(P, b) > 0) P.wet[b] = 0;
+            }
         }
         ENS_SYNC();
         // ---- 1: the rest of RK stage 1 from U^n and the stored divergence

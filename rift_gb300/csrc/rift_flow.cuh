@@ -45,8 +45,10 @@ constexpr uint32_t FLOW_SMEM = FLOW_WARPS * sizeof(MarchRing);
 
 // The rest of Integrate_1_k (grid.cu:856-922) on rows [j0, j1) of segment seg,
 // once dt is known: U* and F* from U^n and the stored divergence.  CLEAR: see
-// clearTile.  Euler mode: the tiles' wet flags (cleared before).  One warp, the
-// lanes and columns of marchRows; two rows of loads in flight.
+// clearTile.  Euler mode: sets the wet flags of the tiles with wet cells, which
+// the caller cleared a grid barrier before (other warps hold rows of the same
+// tiles: a clear here would undo what they set).  One warp, the lanes and
+// columns of marchRows; two rows of loads in flight.
 template <uint32_t FIX, bool CLEAR, class On>
 __device__ __forceinline__ void updateRows(const Params& P, const StageConsts& C, int seg, int j0,
                                            int j1, On on, bool led, Led& L) {
@@ -114,8 +116,8 @@ __device__ __forceinline__ void updateRows(const Params& P, const StageConsts& C
     for (int j = j0; j < j1; j += 2) {
         const int by = (j - 2) / TH, by2 = (j - 1) / TH;
         const bool a0 = on(by, bx), a1 = j + 1 < j1 && (by2 == by ? a0 : on(by2, bx));
-        if (CLEAR && leader && a0 && by != byOld) clearTile(P, by * P.nBX + bx, euler);
-        if (CLEAR && leader && a1 && by2 != by) clearTile(P, by2 * P.nBX + bx, euler);
+        if (CLEAR && !euler && leader && a0 && by != byOld) clearTile(P, by * P.nBX + bx, false);
+        if (CLEAR && !euler && leader && a1 && by2 != by) clearTile(P, by2 * P.nBX + bx, false);
         const int src0 = a0 ? sourceTile(P, by * P.nBX + bx) : -1;
         const int src1 = a1 ? (by2 == by ? src0 : sourceTile(P, by2 * P.nBX + bx)) : -1;
         byOld = a1 ? by2 : by;
