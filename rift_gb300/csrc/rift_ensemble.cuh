@@ -7,8 +7,10 @@
 //   T  (members with gridded rain or surge) re-wet tracking of inactive tiles
 //   G  grow: the strips of all live members (chunked over the CTAs) append
 //      each member's lists; the stale speed maxima of the tiles that are not
-//      active.  Only on the first iteration and when an active set changed:
-//      otherwise S runs on the last sets and checks them, as k_flow does
+//      active.  Only on the first iteration, when an active set changed, and
+//      while a member in Euler mode is live: otherwise S runs on the last sets
+//      and checks them, as k_flow does.  (An Euler member's tile speeds are
+//      folded in S, into entries that the grow has read and cleared.)
 //   S  flux: the stage-1 divergence and the members' speed maxima; the start
 //      of each member's step (one warp per member); U* re-sync of the tiles
 //      that went inactive
@@ -305,7 +307,8 @@ __global__ void __launch_bounds__(ENS_T, 1) k_ensemble(EnsArgs E) {
             const int k = E.M[m].P.st->nInact;
             return k >= 0 ? k : E.M[m].P.gridSize - 1;
         }, Q.offs);
-        bool guess = step > 0 && Q.offs[n] == 0;  // the same total in every CTA
+        // (the same total and count in every CTA)
+        bool guess = step > 0 && Q.offs[n] == 0 && D->nEuler[cur] == 0;
         if (Q.offs[n] > 0) {
             for (int g = blockIdx.x; g < Q.offs[n]; g += gridDim.x) {
                 const int m = ensMember(Q.offs, n, g);

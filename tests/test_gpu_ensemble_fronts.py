@@ -70,3 +70,18 @@ def test_tile_sets_follow_the_fronts(engine_api):
             last[m] = now
     ens.close()
     assert (on[:3] >= 5).all() and (off[:3] >= 5).all(), (on, off)  # fronts advanced, tiles dried
+
+
+def test_tile_speeds_and_dt_match_a_run_alone(engine_api):
+    """dt is bounded by the last speeds of tiles that went inactive: a speed
+    left over from an earlier step shortens it.  The speeds agree as far as the
+    states do (the parity bars), t to the rounding of dt's speeds."""
+    alone, members, ens = _pair(engine_api)
+    for steps in CALLS:
+        t, _ = ens.run(max_steps=steps)
+        for m, (a, b) in enumerate(zip(members, alone)):
+            tb = b.run(steps)[0]
+            assert abs(t[m] - tb) <= 1e-6 * max(1.0, abs(tb)), (m, steps, t[m], tb)
+            for va, vb in zip(a.tile_speeds(), b.tile_speeds()):
+                assert np.allclose(va, vb, rtol=1e-3, atol=1e-4), (m, steps, np.abs(va - vb).max())
+    ens.close()
