@@ -283,6 +283,10 @@ int rift_ensemble_run(rift_ensemble* e, double t_stop, int32_t max_steps, double
  * not stepped by the persistent ensemble kernel: after it, each of them runs
  * on its own, smallest first, with the whole GPU.  Their results are those of a run of their own, as every member's. */
 int rift_ensemble_set_solo_cells(rift_ensemble* e, int64_t min_cells);
+/* Polls after which a grid barrier of the ensemble kernel gives up (-1, the
+ * default: 2^22; 0: the first barrier does).  The run then fails, and every
+ * member it had been stepping reports an error until its next rift_init. */
+int rift_ensemble_set_wait_polls(rift_ensemble* e, int32_t polls);
 /* Per member (n entries): the device time, in seconds, from the start of the
  * last rift_ensemble_run's kernel to the end of the member's last step in it
  * (the GPU's global timer, read when the member's final iteration ends; for

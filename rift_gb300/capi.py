@@ -106,6 +106,9 @@ def bind(lib, prefix: str, create_has_mode: bool = False):
         if hasattr(lib, p + "ensemble_set_solo_cells"):
             ns["ensemble_set_solo_cells"] = _sig(lib, p + "ensemble_set_solo_cells", C.c_int,
                                                  [_P, C.c_int64])
+        if hasattr(lib, p + "ensemble_set_wait_polls"):
+            ns["ensemble_set_wait_polls"] = _sig(lib, p + "ensemble_set_wait_polls", C.c_int,
+                                                 [_P, C.c_int32])
         if hasattr(lib, p + "ensemble_launch_count"):
             ns["ensemble_launch_count"] = _sig(lib, p + "ensemble_launch_count", C.c_int,
                                                [_P, C.POINTER(C.c_int64)])
@@ -454,6 +457,13 @@ class Ensemble:
         rc = self.f["ensemble_set_solo_cells"](self.h, int(min_cells))
         if rc != RIFT_OK:
             raise RiftError(f"ensemble_set_solo_cells failed: {ERRORS.get(rc, rc)}")
+        return self
+
+    def set_wait_polls(self, polls):
+        """Polls after which a grid barrier of the ensemble kernel gives up (-1: the default)."""
+        rc = self.f["ensemble_set_wait_polls"](self.h, int(polls))
+        if rc != RIFT_OK:
+            raise RiftError(f"ensemble_set_wait_polls failed: {ERRORS.get(rc, rc)}")
         return self
 
     def launch_count(self):

@@ -438,6 +438,7 @@ int buildGraph(rift_handle* h) {
 const char* deviceErrorText(int err) {
     if (err & ERR_TILE_TABLE) return "persistent loop: tile table and active set disagree";
     if (err & ERR_BARRIER_TIMEOUT) return "device wait timed out (grid barrier)";
+    if (!(err & ERR_TMA_TIMEOUT)) return "the member's ensemble run was given up (a device wait timed out)";
     return "device wait timed out (TMA barrier)";
 }
 
@@ -624,6 +625,8 @@ int uploadState(rift_handle* h, const float* H, const float* U, const float* V,
               (r = upField(h, h->A + 2 * pl, V))))
         return r;  // (H null: U^n is already on the device)
     CUDA_TRY(h, cudaMemcpyAsync(h->B, h->A, 3 * pl * 4, cudaMemcpyDeviceToDevice, h->stream));
+    // (a loop that gave up may have left pairs stamped as listed)
+    CUDA_TRY(h, cudaMemsetAsync(h->itemStamp, 0, (size_t)segCount(h->nx) * h->nBY * 4, h->stream));
     CUDA_TRY(h, cudaMemcpyAsync(h->wet, wet.data(), h->gridSize, cudaMemcpyHostToDevice, h->stream));
     CUDA_TRY(h, cudaMemcpyAsync(h->prevAct, activeFlags.data(), h->gridSize,
                                 cudaMemcpyHostToDevice, h->stream));
@@ -1251,6 +1254,8 @@ int rift_run(rift_handle* h, int32_t nsteps, double t_stop, double* t, double* d
              int32_t* steps_done) {
     if (!h || nsteps < 0) return RIFT_ERR_ARG;
     if (!h->inited) return fail(h, RIFT_ERR_STATE, "init first");
+    // a run that gave up left list counters as they were: no launch on them
+    if (h->hst->error) return fail(h, RIFT_ERR_CUDA, deviceErrorText(h->hst->error));
     // every entry point leaves the pinned mirror equal to the device state
     h->hst->t_stop = t_stop;
     h->hst->steps_done = 0;
@@ -1876,6 +1881,7 @@ struct rift_ensemble {
     EnsTimes* hT = nullptr;  // pinned: the members' end times
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int grid = 0;
+    int polls = BAR_POLLS;  // rift_ensemble_set_wait_polls
     long long steps = 0;
     std::string err;
 };
@@ -1938,6 +1944,10 @@ int rift_ensemble_run(rift_ensemble* e, double t_stop, int32_t max_steps, double
     const int n = (int)e->m.size();
     std::vector<int> live(n, 0);
     int nAlive = 0;
+    for (int k = 0; k < n; k++)
+        if (e->m[k]->hst->error)  // as in rift_run
+            return efail(e, RIFT_ERR_CUDA,
+                         "member " + std::to_string(k) + ": " + deviceErrorText(e->m[k]->hst->error));
     for (int k = 0; k < n; k++) {
         rift_handle* h = e->m[k];
         ENS_TRY(e, cudaStreamSynchronize(h->stream));
@@ -1958,7 +1968,7 @@ int rift_ensemble_run(rift_ensemble* e, double t_stop, int32_t max_steps, double
     ENS_TRY(e, cudaMemsetAsync(e->dE, 0, sizeof(EnsDev), e->stream));
     ENS_TRY(e, cudaMemcpyAsync(e->dM, e->hM, sizeof(EnsMember) * n, cudaMemcpyHostToDevice, e->stream));
     k_ens_begin<<<n, 128, 0, e->stream>>>(e->dM, e->dE);
-    EnsArgs A{e->dM, e->dE, n, max_steps};
+    EnsArgs A{e->dM, e->dE, n, max_steps, e->polls};
     void* args[] = {(void*)&A};
     ENS_TRY(e, cudaEventRecord(ev0, e->stream));
     if (nAlive > 0) {
@@ -1967,7 +1977,7 @@ int rift_ensemble_run(rift_ensemble* e, double t_stop, int32_t max_steps, double
         e->launches += 1;
     }
     ENS_TRY(e, cudaEventRecord(ev1, e->stream));
-    k_ens_end<<<n, 128, 0, e->stream>>>(e->dM);
+    k_ens_end<<<n, 128, 0, e->stream>>>(e->dM, e->dE);
     ENS_TRY(e, cudaGetLastError());
     ENS_TRY(e, cudaMemcpyAsync(e->hM, e->dM, sizeof(EnsMember) * n, cudaMemcpyDeviceToHost, e->stream));
     ENS_TRY(e, cudaMemcpyAsync(e->hT, &e->dE->times, sizeof(EnsTimes), cudaMemcpyDeviceToHost, e->stream));
@@ -2033,6 +2043,12 @@ int rift_ensemble_launch_count(rift_ensemble* e, int64_t* kernels) {
 int rift_ensemble_set_solo_cells(rift_ensemble* e, int64_t min_cells) {
     if (!e || min_cells < 0) return RIFT_ERR_ARG;
     e->soloCells = min_cells;
+    return RIFT_OK;
+}
+
+int rift_ensemble_set_wait_polls(rift_ensemble* e, int32_t polls) {
+    if (!e) return RIFT_ERR_ARG;
+    e->polls = polls >= 0 ? polls : BAR_POLLS;
     return RIFT_OK;
 }
 

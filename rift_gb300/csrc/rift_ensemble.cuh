@@ -60,7 +60,7 @@ struct EnsDev {
     unsigned stale[ENS_MAX][2];          // speed maxima of the inactive tiles (bits)
     unsigned long long cells[ENS_MAX];   // interior cells of the active tiles
     int changed[2];        // by step parity: an active set differs from the last step's
-    int fail;              // a TMA wait gave up: every CTA leaves
+    int fail;              // a wait gave up: every CTA leaves
     StageConsts consts[ENS_MAX][2];  // each member's stage constants of the step (phase D)
     EnsTimes times;
 };
@@ -85,6 +85,7 @@ struct EnsArgs {
     EnsDev* dev;
     int n;
     int maxSteps;
+    int polls;  // of a grid barrier, after which it gives up
 };
 
 // The members' device states from the block the host sent, and back: one
@@ -99,8 +100,12 @@ __global__ void k_ens_begin(const EnsMember* M, EnsDev* D) {
         if (m.live && (m.P.flags & F_EULER)) atomicAdd(&D->nEuler[0], 1);
     }
 }
-__global__ void k_ens_end(EnsMember* M) {
+// When a wait gave up, the kernel left every live member between two of its
+// steps: the error is each one's.
+__global__ void k_ens_end(EnsMember* M, const EnsDev* D) {
     EnsMember& m = M[blockIdx.x];
+    if (threadIdx.x == 0 && m.live && D->fail) m.P.st->error |= ERR_ENSEMBLE;
+    __syncthreads();
     copyState(&m.st, m.P.st);
 }
 
@@ -292,8 +297,11 @@ __global__ void __launch_bounds__(ENS_T, 1) k_ensemble(EnsArgs E) {
     const int nW = FLOW_WARPS * (int)gridDim.x, gw = warp * (int)gridDim.x + (int)blockIdx.x;
     DevState* st0 = E.M[0].P.st;  // barrier timeouts are recorded in member 0
     if (blockIdx.x == 0 && tid == 0) D->times.t0 = globalTimerNs();  // before any member can finish
-#define ENS_SYNC()                               \
-    if (!gridSync(&D->bar, barTarget, st0)) return; \
+#define ENS_SYNC()                                                         \
+    if (!gridSync(&D->bar, barTarget, st0, false, nullptr, E.polls)) {     \
+        if (tid == 0) D->fail = 1;                                         \
+        return;                                                            \
+    }                                                                      \
     (void)0
     for (int step = 0;; step++) {
         const int cur = step & 1;

@@ -74,6 +74,7 @@ __device__ __forceinline__ uint32_t cellFlags(uint32_t runFlags) {
 constexpr int ERR_TMA_TIMEOUT = 1;
 constexpr int ERR_BARRIER_TIMEOUT = 2;
 constexpr int ERR_TILE_TABLE = 4;  // persistent loop: tile table and scan disagree
+constexpr int ERR_ENSEMBLE = 8;    // the ensemble kernel gave up between two steps of the member
 
 // Device-resident scalars of the run (one per handle).
 struct DevState {

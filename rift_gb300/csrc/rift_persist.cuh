@@ -27,7 +27,7 @@
 // the per-step launches, whose march kernels suit a dense grid).
 //
 // Every wait is bounded: a grid barrier or a neighbour wait gives up after
-// 2^22 polls, records ERR_BARRIER_TIMEOUT and the kernel returns; no TMA
+// BAR_POLLS polls, records ERR_BARRIER_TIMEOUT and the kernel returns; no TMA
 // copy is in flight at a barrier (each tile loop consumes every load it
 // issues).
 #pragma once
@@ -92,6 +92,7 @@ __device__ __forceinline__ void red_add_release_gpu(unsigned* p, unsigned v) {
 // into `target`, so later barriers see none.
 constexpr size_t GRIDBAR_CLEAR = offsetof(GridBar, slotTile);  // bytes cleared before a launch
 static_assert(GRIDBAR_CLEAR % 4 == 0, "cleared in words");
+constexpr int BAR_POLLS = 1 << 22;
 constexpr unsigned BAR_EVENT = 1u << 16;  // > any grid (PERSIST_MAX_CTAS)
 static_assert(BAR_EVENT > (unsigned)PERSIST_MAX_CTAS, "event unit above the arrivals");
 
@@ -113,7 +114,7 @@ __global__ void k_loop_begin(const DevState* host, DevState* st, GridBar* gb) {
 __global__ void k_loop_end(DevState* host, const DevState* st) { copyState(host, st); }
 
 __device__ bool gridSync(GridBar* gb, unsigned& target, DevState* st, bool raise = false,
-                         int* events = nullptr) {
+                         int* events = nullptr, int polls = BAR_POLLS) {
     __shared__ int sEvents;
     __syncthreads();
     int ok = 1;
@@ -122,7 +123,7 @@ __device__ bool gridSync(GridBar* gb, unsigned& target, DevState* st, bool raise
         red_add_release_gpu(&gb->count[0], raise ? BAR_EVENT + 1u : 1u);
         ok = 0;
         unsigned v = 0u;
-        for (int it = 0; it < (1 << 22); ++it) {
+        for (int it = 0; it < polls; ++it) {
             v = ld_acquire_gpu(&gb->count[0]);
             if ((int)(v - target) >= 0) {
                 ok = 1;
@@ -158,7 +159,7 @@ __device__ bool gridWait(GridBar* gb, unsigned& target, DevState* st) {
     if (threadIdx.x == 0) {
         ok = 0;
         unsigned v = 0u;
-        for (int it = 0; it < (1 << 22); ++it) {
+        for (int it = 0; it < BAR_POLLS; ++it) {
             v = ld_acquire_gpu(&gb->count[0]);
             if ((int)(v - target) >= 0) {
                 ok = 1;
