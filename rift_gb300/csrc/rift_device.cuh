@@ -45,14 +45,16 @@ struct Face {
 // The wet/dry correction against the face elevations: wBar = 2w, so the face
 // depths add up to bar = 2h - eP - eM, and "if (hP < 0) hP = 0, hM = bar; if
 // (hM < 0) hM = 0, hP = bar" is min(max(hP, 0), bar) and max(min(hM, bar), 0).
+// A NaN depth gives NaN depths at the cell's faces (no comparison holds for it),
+// so it shows in the neighbours' momenta after one flux.
 template <class V>
 __device__ __forceinline__ void construct(V h0, V u0, V v0, V tw, V tu, V tv, V eM, V eP, Face<V>& P,
                                           Face<V>& M) {
     const V k = splat<V>(kSlope), nk = splat<V>(-kSlope), zero = splat<V>(0.f);
     const V hP = vsub(vfma(k, tw, h0), eP), hM = vsub(vfma(nk, tw, h0), eM);
     const V bar = vsub(vadd(h0, h0), vadd(eP, eM));
-    P.h = vmin(vmax(hP, zero), bar);
-    M.h = vmax(vmin(hM, bar), zero);
+    P.h = vminNan(vmaxNan(hP, zero), bar);
+    M.h = vmaxNan(vminNan(hM, bar), zero);
     P.u = vfma(k, tu, u0);
     M.u = vfma(nk, tu, u0);
     P.v = vfma(k, tv, v0);
@@ -100,7 +102,8 @@ __device__ __forceinline__ V velFactor(V h, float kappa) {
 
 // One side of a face: velocities (n normal, t tangential), the momenta formed
 // from them, the wave speeds n + c and c - n, and the flux F(U), zero where
-// the depth is not positive (formed from the depth clamped at 0).
+// the depth is not positive (formed from the depth clamped at 0; a NaN velocity
+// there makes it NaN instead).
 template <class V>
 struct Side {
     V t, qn, qt, sp, sm, f0, fn, ft;

@@ -78,6 +78,25 @@ __device__ __forceinline__ P2 vmax(P2 a, P2 b) { return pack2(fmaxf(lo(a), lo(b)
 __device__ __forceinline__ P2 vmin(P2 a, P2 b) { return pack2(fminf(lo(a), lo(b)), fminf(hi(a), hi(b))); }
 __device__ __forceinline__ P2 vmax(P2 a, float b) { return pack2(fmaxf(lo(a), b), fmaxf(hi(a), b)); }
 
+// maximum and minimum that are NaN when an argument is (the ones above leave a
+// NaN argument out)
+__device__ __forceinline__ float vmaxNan(float a, float b) {
+    float r;
+    asm("max.ftz.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float vminNan(float a, float b) {
+    float r;
+    asm("min.ftz.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ P2 vmaxNan(P2 a, P2 b) {
+    return pack2(vmaxNan(lo(a), lo(b)), vmaxNan(hi(a), hi(b)));
+}
+__device__ __forceinline__ P2 vminNan(P2 a, P2 b) {
+    return pack2(vminNan(lo(a), lo(b)), vminNan(hi(a), hi(b)));
+}
+
 // max(a, b, 0): a NaN argument is left out
 __device__ __forceinline__ float vmaxz(float a, float b) {
     float r;
