@@ -318,11 +318,13 @@ __global__ void __launch_bounds__(ENS_T, 1) k_ensemble(EnsArgs E) {
         // (the same total and count in every CTA)
         bool guess = step > 0 && Q.offs[n] == 0 && D->nEuler[cur] == 0;
         if (Q.offs[n] > 0) {
-            for (int g = blockIdx.x; g < Q.offs[n]; g += gridDim.x) {
+            int of = -1;  // member of the factors
+            float fac0 = 0.f, fac2 = 0.f;
+            for (int g = gw; g < Q.offs[n]; g += nW) {
                 const int m = ensMember(Q.offs, n, g);
                 const Params& P = E.M[m].P;
-                float fac0, fac2;
-                trackFactors(P, fac0, fac2);
+                if (m != of) trackFactors(P, fac0, fac2);
+                of = m;
                 const bool listed = P.st->nInact >= 0;
                 const int b = listed ? P.inact[g - Q.offs[m]] : g - Q.offs[m] + 1;
                 if (listed || !P.prevAct[b]) trackTile(P, b, fac0, fac2);

@@ -732,40 +732,64 @@ __device__ __forceinline__ void trackFactors(const Params& P, float& fac0, float
     if (s->map_timed[2]) fac2 = (float)((s->t - s->map_t0[2]) / (s->map_t1[2] - s->map_t0[2]));
 }
 
-// One inactive tile: re-wet it when a cell of the rows the reference checks
-// has gridded rain above epsilon or a positive surge depth.
+// One inactive tile, by one warp: re-wet it when a cell of the rows the
+// reference checks has gridded rain above epsilon or a positive surge depth.
+// Bound by the latency of the map loads: a lane's seven are in flight together,
+// and a tile takes a warp, not a CTA with a barrier.  (2000^2 rain maps, half of
+// the 18,144 tiles inactive, on 152 CTAs of 16 warps: 290 us a step with a CTA
+// per tile, 229 with a warp; 300^2, 418 tiles, on k_persist: 26.4, 24.7.)
 __device__ __forceinline__ void trackTile(const Params& P, int tile, float fac0, float fac2) {
-    if (P.wet[tile]) return;  // uniform across the block
-    const int bX = tile % P.nBX, bY = tile / P.nBX;
-    bool hit = false;
-    if (threadIdx.x < TW * TH) {
-        int tx = threadIdx.x % TW, ty = threadIdx.x / TW;
-        int i = bX * TW + tx + 2, j = bY * TW + ty + 2;
-        if (i >= 2 && j >= 2 && i <= P.nx - 3 && j <= P.ny - 3) {
-            size_t c = cidx(P, 0, j, i);
-            if (P.flags & F_RAIN_G) {
-                float v = mapValue(P, 0, c, fac0);
-                if (v > kEps) hit = true;
-            }
-            if (P.flags & F_SURGE) {
-                float v = mapValue(P, 2, c, fac2);
-                if (v != P.nodata && v > 0.f) hit = true;
-            }
+    if (P.wet[tile]) return;  // uniform across the warp
+    const int lane = threadIdx.x & 31;
+    constexpr int PER = TW * TH / 32;
+    static_assert(PER * 32 == TW * TH, "whole rows of lanes");
+    const int i0 = (tile % P.nBX) * TW + 2, j0 = (tile / P.nBX) * TW + 2;
+    if (i0 > P.nx - 3 || j0 > P.ny - 3) return;  // no cell to check
+    auto found = [&](int which, float fac, float floor, bool nodata) {
+        float x0[PER], x1[PER];
+        bool in[PER], hit = false;
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            const int i = i0 + (q * 32 + lane) % TW, j = j0 + (q * 32 + lane) / TW;
+            in[q] = i <= P.nx - 3 && j <= P.ny - 3;
+            const size_t c = in[q] ? cidx(P, 0, j, i) : 0;
+            x0[q] = P.mapMode[which] != 0 ? P.map0[which][c] : 0.f;
+            x1[q] = P.mapMode[which] == 2 ? P.map1[which][c] : 0.f;
         }
-    }
-    if (__syncthreads_or(hit) && threadIdx.x == 0) P.wet[tile] = 1;
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            const float v = mapFrom(P, which, x0[q], x1[q], fac);
+            hit |= in[q] && !(nodata && v == P.nodata) && v > floor;
+        }
+        return hit;
+    };
+    bool hit = (P.flags & F_RAIN_G) && found(0, fac0, kEps, false);
+    hit |= (P.flags & F_SURGE) && found(2, fac2, 0.f, true);
+    if (__any_sync(0xffffffffu, hit) && lane == 0) P.wet[tile] = 1;
 }
 
+// The inactive tiles, a warp each.  (All threads of the CTA; the factors' FP64
+// divisions by one warp of it.)
 __device__ __forceinline__ void trackTiles(const Params& P) {
-    const int n = P.st->nInact;
-    float fac0, fac2;
-    trackFactors(P, fac0, fac2);
+    __shared__ float fac[2];
+    const int n = P.st->nInact, warps = (int)(blockDim.x / 32) * (int)gridDim.x;
+    const int w = (int)(threadIdx.x / 32) * (int)gridDim.x + (int)blockIdx.x;
+    if (threadIdx.x < 32) {
+        float a, b;
+        trackFactors(P, a, b);
+        if (threadIdx.x == 0) {
+            fac[0] = a;
+            fac[1] = b;
+        }
+    }
+    __syncthreads();
+    const float fac0 = fac[0], fac2 = fac[1];
     if (n < 0) {  // no list (a step of the persistent loop's tile table): scan
-        for (int b = blockIdx.x + 1; b < P.gridSize; b += gridDim.x)
+        for (int b = w + 1; b < P.gridSize; b += warps)
             if (!P.prevAct[b]) trackTile(P, b, fac0, fac2);
         return;
     }
-    for (int k = blockIdx.x; k < n; k += gridDim.x) trackTile(P, P.inact[k], fac0, fac2);
+    for (int k = w; k < n; k += warps) trackTile(P, P.inact[k], fac0, fac2);
 }
 
 __global__ void __launch_bounds__(NT) k_track(Params P) {
