@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(FLOW_T, 1) k_flow(const __grid_constant__ CUte
     DevState* st = P.st;
     GridBar* const T = P.gbar;
     const uint32_t fl = P.flags;
-    const bool track = (fl & (F_RAIN_G | F_SURGE)) != 0;
+    const bool track = (cellFlags<FIX>(fl) & (F_RAIN_G | F_SURGE)) != 0;
     const bool spare = blockIdx.x == gridDim.x - 1;
     const bool led = (cellFlags<FIX>(fl) & F_CHECKVOL) != 0;
     Led L;

@@ -353,8 +353,8 @@ __global__ void __launch_bounds__(NT, 4) k_persist(const __grid_constant__ CUten
     GridBar* const T = P.gbar;
     const int tid = threadIdx.x;
     const uint32_t fl = P.flags;
-    const bool track = (fl & (F_RAIN_G | F_SURGE)) != 0;
-    const bool euler = (fl & F_EULER) != 0;
+    const bool track = (cellFlags<FIX>(fl) & (F_RAIN_G | F_SURGE)) != 0;
+    const bool euler = (cellFlags<FIX>(fl) & F_EULER) != 0;
     const bool tableOk = !track && !euler && P.owner != nullptr;
     const bool spare = blockIdx.x == gridDim.x - 1;
     const bool led = (cellFlags<FIX>(fl) & F_CHECKVOL) != 0;  // check_volume ledger
