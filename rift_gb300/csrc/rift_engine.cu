@@ -67,7 +67,8 @@ struct rift_handle {
     int marchMin = 0;  // active strips from which the march kernels run
     int gridGrow = 0;      // CTAs of the grow kernel of the graph path
     int gridPersist = 0;   // CTAs of the cooperative step kernel (0: unavailable)
-    int persistMax = 0;    // it runs while the active tiles are at most this many
+    int persistMax = 0;    // it runs while the active tiles are at most this many (see loopMax)
+    bool persistAuto = true;  // ... not set by the caller
     GridBar* gbar = nullptr;
     int* owner = nullptr;  // [gridSize] tile table of the persistent loop
     int *items = nullptr, *itemStamp = nullptr;  // [segments x tile rows] item list of k_flow
@@ -1042,6 +1043,7 @@ int rift_set_schedule(rift_handle* h, int32_t march_min_strips) {
 
 int rift_set_persistent(rift_handle* h, int32_t max_active_tiles) {
     if (!h) return RIFT_ERR_ARG;
+    h->persistAuto = max_active_tiles < 0;
     if (h->gridPersist == 0) {
         h->persistMax = 0;
         return max_active_tiles > 0 ? fail(h, RIFT_ERR_UNSUPPORTED, "no cooperative launch")
@@ -1093,12 +1095,42 @@ int persistGrid(const rift_handle* h) {
     return std::max(1, std::min(h->gridPersist, h->numSMs * perSM));
 }
 
+bool allActive(const rift_handle* h) {
+    return h->hst->nActive == ((h->nx - 4 + TW - 1) / TW) * ((h->ny - 4 + TH - 1) / TH);
+}
+
+// Options read at run time (no instantiation of their own) on a set with
+// inactive tiles: a few rows per warp whose loads wait for one another, the more
+// of them the more options.
+bool listedGeneric(const rift_handle* h) {
+    return h->flowOk && !h->has(RIFT_F_EULER) && marchFix(h) == 0u && !allActive(h);
+}
+
+// Active tiles up to which k_flow takes such a set.  Against the per-tile phases
+// of k_persist, us per step, channel floods with infiltration and maps of maxima
+// and arrivals: 651 tiles 42 -> 38, 962 tiles 43 -> 48, 1318 tiles 56 -> 64, 1927
+// tiles 68 -> 86 (with infiltration and a drain 42 -> 43 at 962, 65 -> 74 at
+// 1927).  Without infiltration k_flow is never behind where it runs (loopMax).
+int flowMax(const rift_handle* h) {
+    return listedGeneric(h) && h->has(RIFT_F_INFILTRATION) ? h->gridPersist * 5 / 4 : INT32_MAX;
+}
+
+// Active tiles up to which the step loops run the steps.  By default fewer of
+// such a set: rain maps, half of the tiles active, k_flow and the step graph, us
+// per step: 56 and 68 at 2,516 tiles, 118 and 107 at 4,614, 236 and 192 at 9,250.
+int loopMax(const rift_handle* h) {
+    return h->persistAuto && listedGeneric(h) && !h->has(RIFT_F_INFILTRATION)
+               ? std::min(h->persistMax, 4096) : h->persistMax;
+}
+
 // The active set does not fit one tile per CTA of k_persist: k_flow's warps
 // take it (RK2 only).  Against the per-tile phases of k_persist, us per step:
 // 400^2 rain and infiltration, 754 tiles, 38 -> 22; 512^2 rain, 1221 tiles,
 // 34 -> 24; a 2048^2 channel flood, 651 tiles, 34 -> 27; 1024^2 rain, 4810
 // tiles, 86 -> 49.
-bool aboveOnePerCta(const rift_handle* h) { return h->hst->nActive > h->gridPersist; }
+bool aboveOnePerCta(const rift_handle* h) {
+    return h->hst->nActive > h->gridPersist && h->hst->nActive <= flowMax(h);
+}
 
 // Under gridded rain k_persist cannot keep its tile table and grows and tracks
 // every step; while every tile is active k_flow needs neither.  Rain maps and
@@ -1106,8 +1138,7 @@ bool aboveOnePerCta(const rift_handle* h) { return h->hst->nActive > h->gridPers
 // 25.1 -> 19.1, 550 29.2 -> 20.3.  A call of one step costs more up to about 400
 // tiles (195 tiles 37 -> 42), hence the least number of steps.
 bool fullRainGrid(const rift_handle* h, int nsteps) {
-    const int all = ((h->nx - 4 + TW - 1) / TW) * ((h->ny - 4 + TH - 1) / TH);
-    return marchFix(h) == FIX_RAINMAP_DRAIN && nsteps >= 8 && h->hst->nActive == all && all > h->numSMs;
+    return marchFix(h) == FIX_RAINMAP_DRAIN && nsteps >= 8 && allActive(h) && h->hst->nActive > h->numSMs;
 }
 
 bool useFlow(const rift_handle* h, int nsteps) {
@@ -1120,7 +1151,9 @@ constexpr int kLoopKernels = 3;
 
 cudaError_t enqueueLoop(rift_handle* h, int nsteps) {
     Params P = makeParams(h);
+    P.persistMax = loopMax(h);
     if (useFlow(h, nsteps)) {
+        P.persistMax = std::min(P.persistMax, flowMax(h));
         int rows = marchItemRows(h->nx, h->ny, h->numSMs * FLOW_WARPS);
         // (hysteresis between the two loops; under fullRainGrid: every tile)
         int minTiles = aboveOnePerCta(h) ? h->gridPersist * 3 / 4 : h->hst->nActive;
@@ -1129,7 +1162,9 @@ cudaError_t enqueueLoop(rift_handle* h, int nsteps) {
         return cudaLaunchCooperativeKernel(flowKernel(h), dim3(h->numSMs), dim3(FLOW_T), args, FLOW_SMEM,
                                            h->stream);
     }
-    if (h->flowOk && !h->has(RIFT_F_EULER)) P.persistMax = std::min(P.persistMax, h->gridPersist);
+    // (k_flow's turn above one tile per CTA, unless the set is past that too)
+    if (h->flowOk && !h->has(RIFT_F_EULER) && h->hst->nActive <= h->gridPersist)
+        P.persistMax = std::min(P.persistMax, h->gridPersist);
     void* args[] = {(void*)&h->tmA, (void*)&h->tmB, (void*)&h->tmE, (void*)&P, (void*)&nsteps};
     return cudaLaunchCooperativeKernel(persistKernel(h), dim3(persistGrid(h)), dim3(NT), args, 0,
                                        h->stream);
@@ -1167,7 +1202,7 @@ int runSteps(rift_handle* h, int nsteps, bool* mirrorCurrent) {
     bool pushed = false;  // the device holds the state
     *mirrorCurrent = nsteps <= 0;
     while (left > 0) {
-        if (h->persistMax > 0 && h->hst->nActive <= h->persistMax) {
+        if (h->hst->nActive <= loopMax(h) && h->persistMax > 0) {
             const int before = h->hst->steps_done;
             if ((rc = runPersist(h, left))) return rc;
             pushed = *mirrorCurrent = true;
@@ -1175,7 +1210,7 @@ int runSteps(rift_handle* h, int nsteps, bool* mirrorCurrent) {
             h->persistSteps += ran;
             left -= ran;
             if (!h->hst->persistExit) break;  // all steps done, or t_stop reached
-            if (left > 0 && h->hst->nActive <= h->persistMax) continue;  // the other loop's turn
+            if (left > 0 && h->hst->nActive <= loopMax(h)) continue;  // the other loop's turn
         }
         if (left <= 0) break;
         const int chunk = std::min(left, kGraphChunk);
@@ -1261,7 +1296,7 @@ int rift_run(rift_handle* h, int32_t nsteps, double t_stop, double* t, double* d
     h->hst->steps_done = 0;
     int rc;
     bool current = false;
-    if (nsteps == 1 && h->persistMax > 0 && h->hst->nActive <= h->persistMax &&
+    if (nsteps == 1 && h->persistMax > 0 && h->hst->nActive <= loopMax(h) &&
         stepGraph(h, rc)) {
         if (rc) return rc;
         if (t) *t = h->hst->t;
@@ -1805,7 +1840,7 @@ int rift_autotune(rift_handle* h, int32_t probe_steps, int32_t* choice, double* 
         return RIFT_OK;
     };
     const int keepPersist = h->persistMax, keepMarch = h->marchMin, keepRows = h->marchRows;
-    const bool keepAuto = h->marchAuto;
+    const bool keepAuto = h->marchAuto, keepPersistAuto = h->persistAuto;
     // candidates: persistent loop; per-step graph with the tile kernels; with
     // the march kernels on work items of 2, 1 and 4 tile rows
     constexpr int NC = RIFT_AUTOTUNE_CANDIDATES;
@@ -1816,6 +1851,7 @@ int rift_autotune(rift_handle* h, int32_t probe_steps, int32_t* choice, double* 
     int pick = 1;
     double ms3[NC] = {NAN, NAN, NAN, NAN, NAN};
     cudaEvent_t e0 = nullptr, e1 = nullptr;
+    h->persistAuto = false;
     rc = copyAll(true);
     if (!rc && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess))
         rc = fail(h, RIFT_ERR_CUDA, "cudaEventCreate");
@@ -1852,6 +1888,7 @@ int rift_autotune(rift_handle* h, int32_t probe_steps, int32_t* choice, double* 
         if ((rc = copyAll(false)) == RIFT_OK) rc = pushState(h);
     }
     h->persistMax = rc ? keepPersist : (pick == 0 ? INT32_MAX : 0);
+    if (rc) h->persistAuto = keepPersistAuto;
     h->marchMin = rc ? keepMarch : marchOf[pick];
     h->marchRows = rc ? keepRows : rowsOf[pick];
     h->marchAuto = rc || pick < 2 ? keepAuto : pick == 2;
