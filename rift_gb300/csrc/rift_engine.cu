@@ -342,7 +342,8 @@ template <int STAGE>
 void launchMarch(const rift_handle* h, const CUtensorMap& tmIn, const Params& P, cudaStream_t s,
                  int grid) {
     const CUtensorMap& tmE = h->tmEm;
-    const int rows = h->marchAuto ? marchItemRows(h->nx, h->ny, grid * MW) : h->marchRows * TH, pf = h->marchPrefetch ? 1 : 0;
+    const int rows = h->marchAuto ? -marchItemRows(h->nx, h->ny, grid * MW) : h->marchRows * TH;
+    const int pf = h->marchPrefetch ? 1 : 0;
     if (STAGE == 1) {  // no cell update in stage 1: one instantiation
         k_march<1><<<grid, MT, 0, s>>>(tmIn, tmE, P, rows, pf);
         return;
