@@ -255,30 +255,25 @@ def run_ours(args, device=0, sync=None):
     clocks = ClockSampler().start()
     if sync:
         sync()
-    p0, g0 = sim.path_stats()
+    (p0, g0), f0 = sim.path_stats(), sim.flow_steps()
     ms, active_cells, done, stage_ms, stage_cells = device_timed_run(sim, args.steps)
-    p1, g1 = sim.path_stats()
+    (p1, g1), f1 = sim.path_stats(), sim.flow_steps()
     if sync:
         sync()
     clk = clocks.stop()
-    persist_steps, graph_steps = p1 - p0, g1 - g0
+    persist_steps, flow_steps, graph_steps = p1 - p0, f1 - f0, g1 - g0
     steps = int(done)
     value = interior * steps / (ms * 1e-3)
     active_rate = active_cells / (ms * 1e-3)
     peak, peak_kind = peaks()
     bytes_per = 4 * WORDS[cfg]
-    one_launch = persist_steps > 0 and graph_steps == 0
-    if one_launch:
-        # one cooperative launch ran every timed step: the kernel is the step
-        kernel = ("k_persist (whole step in one cooperative launch: grow, speeds + dt, "
-                  "RK stages 1+2)")
+    key, kernel = timed_kernel(persist_steps, flow_steps, graph_steps)
+    if key != "stages":
         achieved = active_cells * bytes_per / (ms * 1e-3) / 1e9
-        launches = 3  # the loop, and the kernels that bring its state and take it back
     else:
-        kernel = ("RK stages 1+2 (k_march<1>, k_update1, k_march<2> or k_stage<1>, k_stage<2>; one "
-                  "schedule runs, the other exits at entry)")
         achieved = stage_cells * bytes_per / (stage_ms * 1e-3) / 1e9 if stage_ms > 0 else None
-        launches = graph_steps * launches_per_step(case.flags) + (3 if persist_steps else 0)
+    # 3: the loop, and the kernels that bring its state and take it back
+    launches = graph_steps * launches_per_step(case.flags) + (3 if persist_steps else 0)
     # DRAM bytes (read + write) of the reported kernel per launch, from the
     # ncu capture summarised under profiles/ (per step there)
     traffic = None
@@ -286,8 +281,8 @@ def run_ours(args, device=0, sync=None):
     if os.path.exists(prof) and args.N is None:
         try:
             rec = json.load(open(prof))
-            if rec.get("kernel") == ("k_persist" if one_launch else "stages"):
-                traffic = rec["bytes_per_step"] * (steps if one_launch else 1)
+            if rec.get("kernel") == key:
+                traffic = rec["bytes_per_step"] * (1 if key == "stages" else steps)
         except Exception:
             traffic = None
     line = {
@@ -318,13 +313,29 @@ def run_ours(args, device=0, sync=None):
                      "kernel": kernel},
         "clocks": clk,
         "gpu_launches": launches,
-        "path": {"persistent_steps": persist_steps, "graph_steps": graph_steps,
+        "path": {"persistent_steps": persist_steps, "flow_steps": flow_steps, "graph_steps": graph_steps,
                  "autotune": tuned, "march_rows": sim.march_rows()},
     }
     if args.cpu_baseline:
         line["cpu_baseline"] = cpu_baseline(case, snap, args)
     sim.close()
     return line
+
+
+def timed_kernel(persist_steps, flow_steps, graph_steps):
+    """The kernel the roofline of a timed run is of, as a traffic record names
+    it and in words: a step loop when it ran every step (one cooperative
+    launch: the kernel is the step), else the stage kernels of the graph.
+    flow_steps: of the persistent steps, those of k_flow."""
+    if graph_steps or not persist_steps:
+        return "stages", ("RK stages 1+2 (k_march<1>, k_update1, k_march<2> or k_stage<1>, k_stage<2>; "
+                          "one schedule runs, the other exits at entry)")
+    whole = " (whole step in one cooperative launch: grow, speeds + dt, RK stages 1+2)"
+    if flow_steps == 0:
+        return "k_persist", "k_persist" + whole
+    if flow_steps == persist_steps:
+        return "k_flow", "k_flow" + whole
+    return "k_persist+k_flow", "k_persist and k_flow, one after the other" + whole
 
 
 def launches_per_step(flags):

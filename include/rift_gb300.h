@@ -302,9 +302,14 @@ void rift_ensemble_destroy(rift_ensemble* e);
 /* Steps run so far by the persistent launch and by the per-step graph. */
 int rift_get_path_stats(rift_handle* h, int64_t* persist_steps, int64_t* graph_steps);
 
+/* Of the persistent steps, those run by the loop on the march's items (sets
+ * above one tile per CTA).  No reference counterpart. */
+int rift_get_flow_steps(rift_handle* h, int64_t* flow_steps);
+
 /* Kernels launched so far by rift_run / rift_step on this handle: each
- * persistent launch counts one, each replay of the per-step graph the
- * kernels in it. */
+ * persistent launch counts three (the loop and the kernels that bring its
+ * state and take it back), each replay of the per-step graph the kernels in
+ * it. */
 int rift_get_launch_count(rift_handle* h, int64_t* kernels);
 
 /* Of the persistent steps, those run from the loop's tile table: one

@@ -120,6 +120,8 @@ def bind(lib, prefix: str, create_has_mode: bool = False):
                                     [_P, C.POINTER(C.c_int64), C.POINTER(C.c_int64)])
         ns["get_table_steps"] = _sig(lib, p + "get_table_steps", C.c_int,
                                      [_P, C.POINTER(C.c_int64)])
+        ns["get_flow_steps"] = _sig(lib, p + "get_flow_steps", C.c_int,
+                                    [_P, C.POINTER(C.c_int64)])
     if hasattr(lib, p + "get_launch_count"):
         ns["get_launch_count"] = _sig(lib, p + "get_launch_count", C.c_int, [_P, C.POINTER(C.c_int64)])
     if hasattr(lib, p + "set_host_access"):
@@ -315,6 +317,12 @@ class Sim:
         a, b = C.c_int64(), C.c_int64()
         self._check(self.f["get_path_stats"](self.h, C.byref(a), C.byref(b)), "get_path_stats")
         return a.value, b.value
+
+    def flow_steps(self):
+        """Persistent steps run by the loop on the march's items (rift_get_flow_steps)."""
+        a = C.c_int64()
+        self._check(self.f["get_flow_steps"](self.h, C.byref(a)), "get_flow_steps")
+        return a.value
 
     def table_steps(self):
         """Persistent steps run from the loop's tile table (no grow phase)."""

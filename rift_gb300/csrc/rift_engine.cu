@@ -75,6 +75,7 @@ struct rift_handle {
     bool flowOk = false;      // k_flow fits one CTA per SM
     int* tileFlag = nullptr;  // [gridSize] stage-1 completion of the persistent loop
     long long persistSteps = 0, graphSteps = 0;  // steps run by each path (diagnostics)
+    long long flowSteps = 0;  // of persistSteps, those run by k_flow
     long long launches = 0;  // kernels launched by the run paths (graph replays count their kernels)
     int graphKernels = 0;    // kernel nodes of the per-step graph
     int* strips = nullptr;
@@ -1205,10 +1206,12 @@ int runSteps(rift_handle* h, int nsteps, bool* mirrorCurrent) {
     while (left > 0) {
         if (h->hst->nActive <= loopMax(h) && h->persistMax > 0) {
             const int before = h->hst->steps_done;
+            const bool flow = useFlow(h, left);
             if ((rc = runPersist(h, left))) return rc;
             pushed = *mirrorCurrent = true;
             const int ran = h->hst->steps_done - before;
             h->persistSteps += ran;
+            if (flow) h->flowSteps += ran;
             left -= ran;
             if (!h->hst->persistExit) break;  // all steps done, or t_stop reached
             if (left > 0 && h->hst->nActive <= loopMax(h)) continue;  // the other loop's turn
@@ -1281,6 +1284,7 @@ bool stepGraph(rift_handle* h, int& rc) {
         return true;
     }
     h->persistSteps += h->hst->steps_done - before;
+    if (grid < 0) h->flowSteps += h->hst->steps_done - before;
     h->launches += kLoopKernels;
     return true;
 }
@@ -1788,6 +1792,12 @@ int rift_get_path_stats(rift_handle* h, int64_t* persist_steps, int64_t* graph_s
     if (!h) return RIFT_ERR_ARG;
     if (persist_steps) *persist_steps = h->persistSteps;
     if (graph_steps) *graph_steps = h->graphSteps;
+    return RIFT_OK;
+}
+
+int rift_get_flow_steps(rift_handle* h, int64_t* flow_steps) {
+    if (!h || !flow_steps) return RIFT_ERR_ARG;
+    *flow_steps = h->flowSteps;
     return RIFT_OK;
 }
 
