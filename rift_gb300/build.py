@@ -14,7 +14,8 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-std=c++17", "-use_fast_math", "-lineinfo", "-Xcompiler", "-fPIC", "-shared"]
 SOURCES = ["rift_engine.cu"]
 DEPS = ["rift_engine.cu", "rift_kernels.cuh", "rift_march.cuh", "rift_persist.cuh", "rift_grow.cuh",
-        "rift_device.cuh", "rift_ensemble.cuh", "rift_update1.cuh", "rift_pair.cuh", "rift_flow.cuh"]
+        "rift_device.cuh", "rift_ensemble.cuh", "rift_update1.cuh", "rift_pair.cuh", "rift_flow.cuh",
+        "rift_bar.cuh"]
 
 
 def _stale(out, deps):

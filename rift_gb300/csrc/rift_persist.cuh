@@ -31,6 +31,7 @@
 // copy is in flight at a barrier (each tile loop consumes every load it
 // issues).
 #pragma once
+#include "rift_bar.cuh"
 #include "rift_grow.cuh"
 #include "rift_kernels.cuh"
 
@@ -38,11 +39,11 @@ namespace rift {
 
 constexpr int PERSIST_MAX_CTAS = 4096;
 
-// Grid barrier state: one arrival counter on its own 128-byte line; then
+// Grid barrier state: its word (rift_bar.cuh) on its own 128-byte line; then
 // the tile table of the persistent loop (cleared with the counter before
 // every launch).
 struct GridBar {
-    unsigned count[32];
+    BarWord count[16];
     // step reductions of the fused steps, by step parity: a step's values
     // are cleared during the next step, when no CTA can still read them
     unsigned maxb[2][2];   // speed maxima of the scheduled tiles (bits)
@@ -71,8 +72,13 @@ __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void red_add_release_gpu(unsigned* p, unsigned v) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ BarWord ld_acquire_gpu(const BarWord* p) {
+    BarWord v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void red_add_release_gpu(BarWord* p, BarWord v) {
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 // Grid-wide barrier.  Every CTA adds 1 to a monotonic counter with release
@@ -83,18 +89,14 @@ __device__ __forceinline__ void red_add_release_gpu(unsigned* p, unsigned v) {
 // before it.  Measured on GB300: 1.2 us for 152 CTAs, 2.1 us for 608.  False
 // after the poll limit (error recorded).
 //
-// A CTA may raise an event at a barrier (`raise`): its arrival adds
-// BAR_EVENT + 1.  Every CTA leaves with the number of events raised there
-// (*events): no barrier passes before every arrival is counted, and the
-// arrivals at the next barrier that a slow poller may also see add less
-// than BAR_EVENT in all (they raise nothing: the caller raises events at
-// one barrier only, never at the one after it).  The event count then moves
-// into `target`, so later barriers see none.
+// A CTA may raise an event at a barrier (`raise`).  A CTA that asks (`ev`) leaves
+// with the number raised since it last asked: the word is read after the last
+// arrival, and the arrivals at the next barrier that a slow poller may also see
+// raise nothing (the caller raises events at one barrier only, never at the one
+// after it).
 constexpr size_t GRIDBAR_CLEAR = offsetof(GridBar, slotTile);  // bytes cleared before a launch
 static_assert(GRIDBAR_CLEAR % 4 == 0, "cleared in words");
 constexpr int BAR_POLLS = 1 << 22;
-constexpr unsigned BAR_EVENT = 1u << 16;  // > any grid (PERSIST_MAX_CTAS)
-static_assert(BAR_EVENT > (unsigned)PERSIST_MAX_CTAS, "event unit above the arrivals");
 
 // What goes with a launch of a step loop, one CTA each: the device state from
 // the host's pinned mirror with the barrier cleared, and the state back.
@@ -113,19 +115,22 @@ __global__ void k_loop_begin(const DevState* host, DevState* st, GridBar* gb) {
 }
 __global__ void k_loop_end(DevState* host, const DevState* st) { copyState(host, st); }
 
+struct BarCount {  // a CTA's count of events, in shared memory (zero at the start)
+    unsigned seen;
+    int raised;  // at the last barrier that asked
+};
 __device__ bool gridSync(GridBar* gb, unsigned& target, DevState* st, bool raise = false,
-                         int* events = nullptr, int polls = BAR_POLLS) {
-    __shared__ int sEvents;
+                         BarCount* ev = nullptr, int polls = BAR_POLLS) {
     __syncthreads();
     int ok = 1;
     if (threadIdx.x == 0) {
         target += gridDim.x;
-        red_add_release_gpu(&gb->count[0], raise ? BAR_EVENT + 1u : 1u);
+        red_add_release_gpu(&gb->count[0], barArrival(raise));
         ok = 0;
-        unsigned v = 0u;
+        BarWord v = 0u;
         for (int it = 0; it < polls; ++it) {
             v = ld_acquire_gpu(&gb->count[0]);
-            if ((int)(v - target) >= 0) {
+            if (barPassed(v, target)) {
                 ok = 1;
                 break;
             }
@@ -133,13 +138,12 @@ __device__ bool gridSync(GridBar* gb, unsigned& target, DevState* st, bool raise
         }
         fence_proxy_async_global();
         if (!ok) atomicOr(&st->error, ERR_BARRIER_TIMEOUT);
-        const unsigned k = ok ? (v - target) / BAR_EVENT : 0u;
-        target += k * BAR_EVENT;
-        sEvents = (int)k;
+        if (ev) {
+            ev->raised = (int)(barEvents(v) - ev->seen);
+            ev->seen = barEvents(v);
+        }
     }
-    ok = __syncthreads_and(ok);
-    if (events) *events = sEvents;
-    return ok != 0;
+    return __syncthreads_and(ok) != 0;
 }
 
 // The same barrier in two halves, so a CTA can work on its own data between
@@ -150,18 +154,17 @@ __device__ __forceinline__ void gridArrive(GridBar* gb, unsigned& target) {
     __syncthreads();
     if (threadIdx.x == 0) {
         target += gridDim.x;
-        red_add_release_gpu(&gb->count[0], 1u);
+        red_add_release_gpu(&gb->count[0], barArrival(false));
     }
 }
 
-__device__ bool gridWait(GridBar* gb, unsigned& target, DevState* st) {
+__device__ bool gridWait(GridBar* gb, unsigned target, DevState* st) {
     int ok = 1;
     if (threadIdx.x == 0) {
         ok = 0;
-        unsigned v = 0u;
         for (int it = 0; it < BAR_POLLS; ++it) {
-            v = ld_acquire_gpu(&gb->count[0]);
-            if ((int)(v - target) >= 0) {
+            const BarWord v = ld_acquire_gpu(&gb->count[0]);
+            if (barPassed(v, target)) {
                 ok = 1;
                 break;
             }
@@ -169,8 +172,6 @@ __device__ bool gridWait(GridBar* gb, unsigned& target, DevState* st) {
         }
         fence_proxy_async_global();
         if (!ok) atomicOr(&st->error, ERR_BARRIER_TIMEOUT);
-        const unsigned k = ok ? (v - target) / BAR_EVENT : 0u;  // no events here; keep the count
-        target += k * BAR_EVENT;
     }
     return __syncthreads_and(ok) != 0;
 }
@@ -346,6 +347,7 @@ __global__ void __launch_bounds__(NT, 4) k_persist(const __grid_constant__ CUten
     __shared__ int sFail;
     __shared__ int sSched;
     __shared__ int sOverflow;  // a claim of this CTA found no free CTA
+    __shared__ BarCount sVoided;  // claims that found none, of all CTAs
     __shared__ StepRates sRates;  // this step's source rates (every CTA computes them)
     __shared__ StageConsts sPre;  // stage-1 constants without the step's dt
     __shared__ CellSrc sSrc[NT];  // stage-1 sources of each thread's cell
@@ -365,6 +367,7 @@ __global__ void __launch_bounds__(NT, 4) k_persist(const __grid_constant__ CUten
         prefetch_tmap(&tmB);
         deCount = 0;
         sOverflow = 0;
+        sVoided.seen = 0u;
     }
     uint32_t ph[2] = {0u, 0u};
     unsigned barTarget = 0u;
@@ -630,10 +633,9 @@ __global__ void __launch_bounds__(NT, 4) k_persist(const __grid_constant__ CUten
                 }
             }
             if (led) flushLed(L, st->led);
-            int voided = 0;
-            if (!gridSync(P.gbar, barTarget, st, sOverflow != 0, &voided)) return;
+            if (!gridSync(P.gbar, barTarget, st, sOverflow != 0, &sVoided)) return;
             if (tid == 0) sOverflow = 0;
-            table = (table || built) && voided == 0;
+            table = (table || built) && sVoided.raised == 0;
             haveNext = true;
             continue;
         }
