@@ -1164,12 +1164,15 @@ cudaError_t enqueueLoop(rift_handle* h, int nsteps) {
         return cudaLaunchCooperativeKernel(flowKernel(h), dim3(h->numSMs), dim3(FLOW_T), args, FLOW_SMEM,
                                            h->stream);
     }
-    // (k_flow's turn above one tile per CTA, unless the set is past that too)
+    // (k_flow's turn above one tile per CTA, unless the set is past that too;
+    // below, the next launch has more CTAs: the 2048^2 channel flood grows from
+    // 151 tiles to 219, 26 us a step on 152 CTAs and 13 on 304)
+    const int grid = persistGrid(h);
     if (h->flowOk && !h->has(RIFT_F_EULER) && h->hst->nActive <= h->gridPersist)
         P.persistMax = std::min(P.persistMax, h->gridPersist);
+    if (grid < h->gridPersist) P.persistMax = std::min(P.persistMax, grid);
     void* args[] = {(void*)&h->tmA, (void*)&h->tmB, (void*)&h->tmE, (void*)&P, (void*)&nsteps};
-    return cudaLaunchCooperativeKernel(persistKernel(h), dim3(persistGrid(h)), dim3(NT), args, 0,
-                                       h->stream);
+    return cudaLaunchCooperativeKernel(persistKernel(h), dim3(grid), dim3(NT), args, 0, h->stream);
 }
 
 cudaError_t enqueuePersist(rift_handle* h, int nsteps) {
