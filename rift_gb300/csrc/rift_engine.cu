@@ -1112,7 +1112,7 @@ bool listedGeneric(const rift_handle* h) {
 // of k_persist, us per step, channel floods with infiltration and maps of maxima
 // and arrivals: 651 tiles 42 -> 38, 962 tiles 43 -> 48, 1318 tiles 56 -> 64, 1927
 // tiles 68 -> 86 (with infiltration and a drain 42 -> 43 at 962, 65 -> 74 at
-// 1927).  Without infiltration k_flow is never behind where it runs (loopMax).
+// 1927).  Without infiltration k_flow is behind in thin sets only (thinSet).
 int flowMax(const rift_handle* h) {
     return listedGeneric(h) && h->has(RIFT_F_INFILTRATION) ? h->gridPersist * 5 / 4 : INT32_MAX;
 }
@@ -1125,13 +1125,24 @@ int loopMax(const rift_handle* h) {
                ? std::min(h->persistMax, 4096) : h->persistMax;
 }
 
+// A long thin set that is not tracked: two tiles per CTA of k_persist, but so many
+// (segment, tile row) pairs, about 2.6 per strip, that a warp of k_flow has four
+// rows of one.  Channel floods, k_persist and k_flow, us per step: 962 tiles in 180
+// strips 40 and 39, 1,065 in 196 42 and 45 (with maxima and arrivals 43 and 49, with
+// infiltration 37 and 38), 1,169 in 211 42 and 45 (44 and 51, 38 and 39); a round
+// pond of 1,046 in 99 42 and 34; past two tiles per CTA, 1,291 in 238, 52 and 48.
+bool thinSet(const rift_handle* h) {
+    return !h->has(RIFT_F_RAIN_GRID) && !h->has(RIFT_F_SURGE_GRID) && !allActive(h) &&
+           h->hst->nActive <= 2 * h->gridPersist && 4 * h->hst->nStrips > 5 * h->numSMs;
+}
+
 // The active set does not fit one tile per CTA of k_persist: k_flow's warps
 // take it (RK2 only).  Against the per-tile phases of k_persist, us per step:
 // 400^2 rain and infiltration, 754 tiles, 38 -> 22; 512^2 rain, 1221 tiles,
 // 34 -> 24; a 2048^2 channel flood, 651 tiles, 34 -> 27; 1024^2 rain, 4810
 // tiles, 86 -> 49.
 bool aboveOnePerCta(const rift_handle* h) {
-    return h->hst->nActive > h->gridPersist && h->hst->nActive <= flowMax(h);
+    return h->hst->nActive > h->gridPersist && h->hst->nActive <= flowMax(h) && !thinSet(h);
 }
 
 // Under gridded rain k_persist cannot keep its tile table and grows and tracks
@@ -1171,6 +1182,8 @@ cudaError_t enqueueLoop(rift_handle* h, int nsteps) {
     if (h->flowOk && !h->has(RIFT_F_EULER) && h->hst->nActive <= h->gridPersist)
         P.persistMax = std::min(P.persistMax, h->gridPersist);
     if (grid < h->gridPersist) P.persistMax = std::min(P.persistMax, grid);
+    if (h->hst->nActive > h->gridPersist && thinSet(h))
+        P.persistMax = std::min(P.persistMax, 2 * h->gridPersist);
     void* args[] = {(void*)&h->tmA, (void*)&h->tmB, (void*)&h->tmE, (void*)&P, (void*)&nsteps};
     return cudaLaunchCooperativeKernel(persistKernel(h), dim3(grid), dim3(NT), args, 0, h->stream);
 }

@@ -64,3 +64,36 @@ def test_channel_flood_in_one_call(engine_api):
     assert np.array_equal(wa, wb) and np.array_equal(np.sort(aa), np.sort(ab))
     d = np.abs(a.field("W") - b.field("W"))[2:-2, 2:-2]
     assert np.quantile(d, 0.99) <= Q99 and d.max() <= MAX, d.max()
+
+
+@pytest.mark.parametrize("flags", [0, synth.SAVE_MAX | synth.SAVE_ARRIVAL, synth.INFILTRATION])
+def test_thin_set_past_one_tile_per_cta(engine_api, flags):
+    """Strands of water a tile apart: few tiles in many strips, which stay on the
+    tile loop up to two tiles per CTA of its largest grid, then on k_flow."""
+    nx, ny = 16 * 60 - 4, 14 * 46 - 4
+    rng = np.random.default_rng(1)
+    z = 10.0 + 0.02 * rng.standard_normal((ny + 1, nx + 1))
+    n = np.zeros((ny + 4, nx + 4))
+    n[2:-2, 2:-2] = 0.03
+    h0 = np.zeros_like(n)
+    for k in range(8):  # a column of tiles and one on either side: 1,104 active tiles in 207 strips
+        i = 2 + 16 * (7 * k + 6)
+        h0[2:-2, i + 7:i + 9] = 0.3
+    case = synth.Case(name="strands", B=z, cell=4.0, n=n, h0=h0, psi=0.11, dtheta=0.3,
+                      flags=synth.TILE_ACCEL | synth.H_INIT | flags)
+    if flags & synth.INFILTRATION:
+        case.K = np.where(n > 0, 1e-6, 0.0)
+    a = capi.Sim(case, api=engine_api).setup()
+    b = capi.Sim(case, api=engine_api).set_schedule(1 << 30).set_persistent(0).setup()
+    for chunk in (2, 1, 5, 60):
+        for sim in (a, b):
+            sim.run(chunk)
+        (wa, aa), (wb, ab) = a.tiles(), b.tiles()
+        assert np.array_equal(wa, wb) and np.array_equal(np.sort(aa), np.sort(ab))
+        if chunk == 2:
+            assert 608 < aa.size <= 1216 and len(set(zip(aa % 60 // 7, aa // 60 // 2))) > 190
+            first = a.flow_steps()
+        if chunk == 5:
+            assert a.flow_steps() == first
+    d = np.abs(a.field("W") - b.field("W"))[2:-2, 2:-2]
+    assert np.quantile(d, 0.99) <= Q99 and d.max() <= MAX, d.max()
