@@ -43,7 +43,7 @@ constexpr int PERSIST_MAX_CTAS = 4096;
 // the tile table of the persistent loop (cleared with the counter before
 // every launch).
 struct GridBar {
-    BarWord count[16];
+    unsigned count[32];
     // step reductions of the fused steps, by step parity: a step's values
     // are cleared during the next step, when no CTA can still read them
     unsigned maxb[2][2];   // speed maxima of the scheduled tiles (bits)
@@ -72,13 +72,8 @@ __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ BarWord ld_acquire_gpu(const BarWord* p) {
-    BarWord v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void red_add_release_gpu(BarWord* p, BarWord v) {
-    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+__device__ __forceinline__ void red_add_release_gpu(unsigned* p, unsigned v) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 // Grid-wide barrier.  Every CTA adds 1 to a monotonic counter with release
@@ -89,13 +84,13 @@ __device__ __forceinline__ void red_add_release_gpu(BarWord* p, BarWord v) {
 // before it.  Measured on GB300: 1.2 us for 152 CTAs, 2.1 us for 608.  False
 // after the poll limit (error recorded).
 //
-// A CTA may raise an event at a barrier (`raise`).  A CTA that asks (`ev`) leaves
-// with the number raised since it last asked: the word is read after the last
-// arrival, and the arrivals at the next barrier that a slow poller may also see
-// raise nothing (the caller raises events at one barrier only, never at the one
-// after it).
+// A CTA may raise an event at a barrier (`raise`).  Every CTA leaves with the
+// number raised there (*events): the word is read after the last arrival, and the
+// arrivals at the next barrier that a slow poller may also see raise nothing (the
+// caller raises events at one barrier only, never at the one after it).
 constexpr size_t GRIDBAR_CLEAR = offsetof(GridBar, slotTile);  // bytes cleared before a launch
 static_assert(GRIDBAR_CLEAR % 4 == 0, "cleared in words");
+static_assert(PERSIST_MAX_CTAS < 1 << 15, "arrivals in half a word");
 constexpr int BAR_POLLS = 1 << 22;
 
 // What goes with a launch of a step loop, one CTA each: the device state from
@@ -115,19 +110,16 @@ __global__ void k_loop_begin(const DevState* host, DevState* st, GridBar* gb) {
 }
 __global__ void k_loop_end(DevState* host, const DevState* st) { copyState(host, st); }
 
-struct BarCount {  // a CTA's count of events, in shared memory (zero at the start)
-    unsigned seen;
-    int raised;  // at the last barrier that asked
-};
 __device__ bool gridSync(GridBar* gb, unsigned& target, DevState* st, bool raise = false,
-                         BarCount* ev = nullptr, int polls = BAR_POLLS) {
+                         int* events = nullptr, int polls = BAR_POLLS) {
+    __shared__ int sEvents;
     __syncthreads();
     int ok = 1;
     if (threadIdx.x == 0) {
         target += gridDim.x;
         red_add_release_gpu(&gb->count[0], barArrival(raise));
         ok = 0;
-        BarWord v = 0u;
+        unsigned v = 0u;
         for (int it = 0; it < polls; ++it) {
             v = ld_acquire_gpu(&gb->count[0]);
             if (barPassed(v, target)) {
@@ -138,12 +130,15 @@ __device__ bool gridSync(GridBar* gb, unsigned& target, DevState* st, bool raise
         }
         fence_proxy_async_global();
         if (!ok) atomicOr(&st->error, ERR_BARRIER_TIMEOUT);
-        if (ev) {
-            ev->raised = (int)(barEvents(v) - ev->seen);
-            ev->seen = barEvents(v);
+        if (events) {
+            const unsigned k = ok ? barEvents(v, target) : 0u;
+            target = barSeen(target, k);
+            sEvents = (int)k;
         }
     }
-    return __syncthreads_and(ok) != 0;
+    ok = __syncthreads_and(ok);
+    if (events) *events = sEvents;
+    return ok != 0;
 }
 
 // The same barrier in two halves, so a CTA can work on its own data between
@@ -163,7 +158,7 @@ __device__ bool gridWait(GridBar* gb, unsigned target, DevState* st) {
     if (threadIdx.x == 0) {
         ok = 0;
         for (int it = 0; it < BAR_POLLS; ++it) {
-            const BarWord v = ld_acquire_gpu(&gb->count[0]);
+            const unsigned v = ld_acquire_gpu(&gb->count[0]);
             if (barPassed(v, target)) {
                 ok = 1;
                 break;
@@ -347,7 +342,6 @@ __global__ void __launch_bounds__(NT, 4) k_persist(const __grid_constant__ CUten
     __shared__ int sFail;
     __shared__ int sSched;
     __shared__ int sOverflow;  // a claim of this CTA found no free CTA
-    __shared__ BarCount sVoided;  // claims that found none, of all CTAs
     __shared__ StepRates sRates;  // this step's source rates (every CTA computes them)
     __shared__ StageConsts sPre;  // stage-1 constants without the step's dt
     __shared__ CellSrc sSrc[NT];  // stage-1 sources of each thread's cell
@@ -367,7 +361,6 @@ __global__ void __launch_bounds__(NT, 4) k_persist(const __grid_constant__ CUten
         prefetch_tmap(&tmB);
         deCount = 0;
         sOverflow = 0;
-        sVoided.seen = 0u;
     }
     uint32_t ph[2] = {0u, 0u};
     unsigned barTarget = 0u;
@@ -633,9 +626,10 @@ __global__ void __launch_bounds__(NT, 4) k_persist(const __grid_constant__ CUten
                 }
             }
             if (led) flushLed(L, st->led);
-            if (!gridSync(P.gbar, barTarget, st, sOverflow != 0, &sVoided)) return;
+            int voided = 0;
+            if (!gridSync(P.gbar, barTarget, st, sOverflow != 0, &voided)) return;
             if (tid == 0) sOverflow = 0;
-            table = (table || built) && sVoided.raised == 0;
+            table = (table || built) && voided == 0;
             haveNext = true;
             continue;
         }

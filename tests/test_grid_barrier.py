@@ -16,8 +16,8 @@ using namespace rift;
 // (the counter's wrap).
 int play(int n, int raisers, unsigned start, unsigned seed) {
     std::mt19937 g(seed);
-    BarWord word = (BarWord)start << 32;
-    std::vector<unsigned> target(n, start), seen(n, 0u);
+    unsigned word = start;
+    std::vector<unsigned> target(n, start);
     std::vector<int> at(n, 0), in(n, 0);  // barriers passed; arrived at the next one
     std::vector<int> arrived(9, 0), raisedAt(9, 0);
     for (int b = 0; b < 8; b += 2) raisedAt[b] = (int)(g() % (raisers + 1));
@@ -36,8 +36,9 @@ int play(int n, int raisers, unsigned start, unsigned seed) {
         } else if (barPassed(word, target[c])) {
             if (arrived[b] != n) return printf("left early: barrier %d, %d of %d\n", b, arrived[b], n), 1;
             if (b % 2 == 0) {
-                if ((int)(barEvents(word) - seen[c]) != raised[b]) return printf("events\n"), 1;
-                seen[c] = barEvents(word);
+                const unsigned k = barEvents(word, target[c]);
+                if ((int)k != raised[b]) return printf("events\n"), 1;
+                target[c] = barSeen(target[c], k);
             }
             in[c] = 0;
             if (++at[c] == 8) done++;
@@ -49,7 +50,7 @@ int main() {
     for (unsigned seed = 0; seed < 300; seed++)
         for (int n : {1, 2, 7, 40})
             for (int r : {0, 1, n})
-                for (unsigned start : {0u, 0xffffffffu - 3u * n, 0x7fffffffu - n})
+                for (unsigned start : {0u, 0xffffffffu - 3u * n, 0x7fffffffu - n, 0xffffu - 3u * n})
                     if (play(n, r, start, seed)) return 1;
     return 0;
 }
