@@ -1149,7 +1149,10 @@ bool aboveOnePerCta(const rift_handle* h) {
 // every step; while every tile is active k_flow needs neither.  Rain maps and
 // drain, us per step of a run: 110 tiles 18.8 -> 17.4, 195 21.4 -> 18.0, 418
 // 25.1 -> 19.1, 550 29.2 -> 20.3.  A call of one step costs more up to about 400
-// tiles (195 tiles 37 -> 42), hence the least number of steps.
+// tiles (195 tiles 37 -> 42), hence the least number of steps.  Other options under
+// gridded rain have the generic update there and gain nothing: rain maps alone,
+// 224 tiles 20.9 -> 26.5, 360 24.7 -> 26.8, 504 27.9 -> 27.8; with a surge 21.6 ->
+// 26.5, 22.0 -> 27.2, 26.9 -> 27.7.
 bool fullRainGrid(const rift_handle* h, int nsteps) {
     return marchFix(h) == FIX_RAINMAP_DRAIN && nsteps >= 8 && allActive(h) && h->hst->nActive > h->numSMs;
 }
@@ -1848,6 +1851,7 @@ std::vector<std::pair<void*, size_t>> stepRegions(rift_handle* h) {
 int rift_autotune(rift_handle* h, int32_t probe_steps, int32_t* choice, double* ms_per_step) {
     if (!h || probe_steps < 1) return RIFT_ERR_ARG;
     if (!h->inited) return fail(h, RIFT_ERR_STATE, "init first");
+    if (h->hst->error) return fail(h, RIFT_ERR_CUDA, deviceErrorText(h->hst->error));  // as rift_run
     int rc;
     auto regions = stepRegions(h);
     size_t total = 0;

@@ -49,3 +49,16 @@ def test_members_of_a_failed_run_stop_and_start_again(engine_api):
         assert all(np.array_equal(m.field(f), fresh.field(f)) for f in ("W", "HU", "HV"))
     ens.run(max_steps=5)
     ens.close()
+
+
+def test_autotune_refuses_a_failed_member(engine_api):
+    member = _member(engine_api, 0)
+    ens = capi.Ensemble([member])
+    ens.set_wait_polls(0)
+    with pytest.raises(capi.RiftError, match="timed out"):
+        ens.run(max_steps=3)
+    with pytest.raises(capi.RiftError, match="timed out"):
+        member.autotune(2)
+    member.init()
+    member.autotune(2)
+    ens.close()
