@@ -212,7 +212,8 @@ def run_ours(args, device=0, sync=None):
     # ---- e2e through the C ABI with host buffers ----------------------------
     t0 = time.perf_counter()
     sim = capi.Sim(case, device=device).set_schedule(args.schedule).set_persistent(args.persistent)
-    sim.set_march_rows(args.march_rows)
+    if args.march_rows:
+        sim.set_march_rows(args.march_rows)
     sim.setup()
     t_setup = time.perf_counter() - t0
     spin_up(sim, spin)
@@ -314,12 +315,21 @@ def run_ours(args, device=0, sync=None):
         "clocks": clk,
         "gpu_launches": launches,
         "path": {"persistent_steps": persist_steps, "flow_steps": flow_steps, "graph_steps": graph_steps,
-                 "autotune": tuned, "march_rows": sim.march_rows()},
+                 "autotune": tuned, "march_rows": march_rows(sim, args.march_rows, tuned)},
     }
     if args.cpu_baseline:
         line["cpu_baseline"] = cpu_baseline(case, snap, args)
     sim.close()
     return line
+
+
+def march_rows(sim, given, tuned):
+    """Height of the march's items in the timed run: tile rows where the command
+    line or the autotune set it (its candidates after the third), else the default."""
+    candidates = capi.Sim.AUTOTUNE_CANDIDATES
+    if tuned and candidates.index(tuned["choice"]) == 2:  # sets the default height
+        return "fitted"
+    return sim.march_rows() if given or (tuned and candidates.index(tuned["choice"]) > 2) else "fitted"
 
 
 def timed_kernel(persist_steps, flow_steps, graph_steps):
@@ -760,8 +770,9 @@ def main():
     ap.add_argument("--autotune", type=int, default=0,
                     help="before the timed region, time each schedule for this many steps "
                          "from the spun-up state and keep the fastest (0: off)")
-    ap.add_argument("--march-rows", type=int, default=2, choices=(1, 2, 4),
-                    help="column march work items of this many 16 x 14 tile rows")
+    ap.add_argument("--march-rows", type=int, default=0, choices=(0, 1, 2, 4),
+                    help="column march work items of this many 16 x 14 tile rows "
+                         "(0: the engine's default, fitted to the grid)")
     ap.add_argument("--persistent", type=int, default=-1,
                     help="persistent step loop while at most this many tiles are active "
                          "(-1: engine default, 0: off)")
