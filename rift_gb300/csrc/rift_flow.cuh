@@ -29,9 +29,10 @@
 // bit.  They are formed only for faces near the maximum and above 15/16 of the
 // last step's (1117 x 1531 rain: 94 us a step, 96 without that seed).
 //
-// What bounds it (us per step, GB300).  512^2 rain, 1221 tiles: 24.2 (34 with
-// the per-tile phases) = flux 5, dt 1.0, update 3.1, stage 2 7 and three
-// barriers of 1.3 to 1.8 with the wait for the slowest CTA on top: latency.
+// What bounds it (us per step, GB300).  512^2 rain, 1221 tiles: 22.7 (34 with
+// the per-tile phases; 24.2 with tracking code in it, of which flux 5, dt 1.0,
+// update 3.1, stage 2 7 and three barriers of 1.3 to 1.8 with the wait for the
+// slowest CTA on top): latency.
 // 1024^2 rain: 50 (86) = 12 + 1.0 + 8.7 + 17 + barriers and waits 10: issue in
 // the flux passes, L2 in the update (52 bytes per cell).
 #pragma once
